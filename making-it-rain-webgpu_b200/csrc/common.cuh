@@ -27,7 +27,6 @@ constexpr int kPmeOrder = 5;
 constexpr int kMaxClusterAtoms = 8;
 constexpr int kMaxClusterConstraints = 8;
 constexpr int kMaxShakeIterations = 150;  // src/reference/constraints.ts:34
-constexpr int kMaxRadices = 12;
 
 // Per-system energy accumulators, int64 at the 2^32 fixed-point scale.
 enum EnergySlot : int {
@@ -113,8 +112,7 @@ struct SysDev {
   long long cgrid_off;  // complex half spectrum
   int mod_off;          // moduli: x at mod_off, y at +Kx, z at +Kx+Ky
   int tw_off[3];        // twiddle tables per axis
-  int radices[3][kMaxRadices];
-  int nradix[3];
+  unsigned plan[3];     // radices of each axis' transform, four bits a stage (plan_radices)
   long long umat[6];  // K o M, 2^32 fixed: u_a = x m0 + y m1 + z m2, u_b = y m3 + z m4, u_c = z m5
   float umat_f[9];    // K o M as f32, [v*3+u]
   float pme_pref;     // ONE_4PI_EPS0 * 2 pi / V

@@ -47,10 +47,9 @@ struct Dev {
 
   // slots, sorted order
   int* order;     // global atom or -1
-  // the order as the last integrator step saw it, kept only when the PME
-  // spread goes by slot (spread_sorted): the spread reads this copy
+  // the order as the last integrator step saw it: the PME spread reads this
+  // copy while the list kernels may be rewriting the order
   int* spread_atom;
-  int spread_sorted;
   int* tmp_order;
   int4* pc;
   float4* prm;
@@ -138,6 +137,7 @@ struct Dev {
   const FftWork* fft_x; int n_fft_x;
   const FftWork* fft_p; int n_fft_p;  // whole x-planes (sys, x): the fused z+y passes, when they fit
   int fft_planes;                     // 1: the plane kernels replace the separate z and y passes
+  int smem_p, smem_z, smem_y, smem_x; // shared-memory bytes of the passes' largest work items
   float* influence;                   // per x-pass work item: its elements' influence function (k_influence)
   int influence_stride;               // floats per work item: kFftTile x the largest Kx
 
@@ -202,7 +202,10 @@ void launch_inner_prune(const Dev& d, cudaStream_t s);      // the inner list, w
 void launch_nonbonded(const Dev& d, bool energy, cudaStream_t s);
 void launch_listed(const Dev& d, bool energy, cudaStream_t s);
 void launch_pme(const Dev& d, bool energy, cudaStream_t s);
-bool spread_by_slot(int n_slots);  // whether an engine of n_slots slots spreads PME charges by slot
+int allow_pme_smem(int bytes);  // raise the transform kernels' shared-memory limit; nonzero: refused
+int plane_smem(int Ky, int Kz);       // bytes of a whole x-plane,
+int z_smem(int lines, int Kz);        // of `lines` z lines,
+int strip_smem(int lines, int n);     // of `lines` lines of n points in a y or x pass
 void launch_pme_spread(const Dev& d, cudaStream_t s);
 void launch_pme_fft(const Dev& d, bool energy, cudaStream_t s);
 void launch_pme_gather(const Dev& d, cudaStream_t s);

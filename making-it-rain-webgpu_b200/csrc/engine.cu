@@ -34,10 +34,6 @@
 #include "mlp.h"
 #include "prep.h"
 
-namespace mdb {
-void set_pme_smem(int z, int y, int x, int plane);
-}
-
 using namespace mdb;
 
 namespace {
@@ -53,7 +49,8 @@ int row_cap_for(int cluster) { return cluster == 8 ? 384 : 192; }
 // the exact stage switches the screening network off once its running RMS
 // error exceeds this many kT (the plain barostat takes over)
 constexpr double kSurrogateMaxRmsKT = 1.5;
-constexpr int kPlaneSmemLimit = 200 * 1024;  // bytes: two complex Ky x Kz planes per CTA
+constexpr int kPlanePoints = 25600;       // 2 Ky Kz + Ky + Kz up to which one CTA transforms a whole x-plane
+constexpr int kPmeSmemLimit = 200 * 1024;  // bytes of shared memory a transform kernel may ask for
 
 struct Allocation {
   std::string label;
@@ -510,7 +507,7 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   std::vector<int> iblk_sys, iblk_unit0, iblk_nunit, iblk_atom0, iblk_natom, iatom;
   int atoms = 0, slots = 0, blocks = 0, cells = 0, tiles = 0, units_n = 0, iblk = 0;
   long long grid_pts = 0, cgrid_pts = 0;
-  int smem_z = 0, smem_y = 0, smem_x = 0, smem_p = 0;
+  int smem_z = 0, smem_y = 0, smem_x = 0, smem_p = 0, plane_points = 0;
   std::vector<FftWork> wp;
   const float sq = float(std::sqrt(kOne4PiEps0));
   for (int s = 0; s < n; ++s) {
@@ -562,7 +559,7 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
     for (int k = 0; k < 3; ++k)
       for (double m : bspline_moduli(h.grid[k])) moduli.push_back(float(m));
     for (int k = 0; k < 3; ++k) {
-      plan_radices(h.grid[k], S.radices[k], &S.nradix[k]);
+      plan_radices(h.grid[k], &S.plan[k]);
       S.tw_off[k] = int(twiddles.size());
       for (int j = 0; j < h.grid[k]; ++j) {
         const double a = -2 * 3.14159265358979323846 * j / h.grid[k];
@@ -573,20 +570,23 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
     const int Kx = h.grid[0], Ky = h.grid[1], Kz = h.grid[2];
     // lines per z-pass CTA: at most 2048 points in shared memory, and enough
     // CTAs (about two per SM) that a small mesh still fills the device
-    const int lines = std::max(1, std::min(2048 / Kz, (Kx * Ky + 295) / 296));
-    for (int l = 0; l < Kx * Ky; l += lines) wz.push_back({s, l, 0, std::min(lines, Kx * Ky - l)});
-    smem_z = std::max(smem_z, 2 * lines * Kz * int(sizeof(float2)));
+    // (an even number, within a plane: the z passes take lines two at a time)
+    const int lines = std::max(2, std::min(2048 / Kz, (Kx * Ky + 295) / 296) & ~1);
+    for (int x = 0; x < Kx; ++x)
+      for (int y = 0; y < Ky; y += lines) wz.push_back({s, x * Ky + y, 0, std::min(lines, Ky - y)});
+    smem_z = std::max(smem_z, z_smem(lines, Kz));
     for (int x = 0; x < Kx; ++x)
       for (int k = 0; k < S.kzh; k += kFftTile) wy.push_back({s, x, k, std::min(kFftTile, S.kzh - k)});
-    smem_y = std::max(smem_y, 2 * kFftTile * Ky * int(sizeof(float2)));
+    smem_y = std::max(smem_y, strip_smem(kFftTile, Ky));
     for (int y = 0; y < Ky; ++y)
       for (int k = 0; k < S.kzh; k += kFftTile) {
         wx.push_back({s, y, k, std::min(kFftTile, S.kzh - k)});
         e->fft_x_sys.push_back(s);
       }
-    smem_x = std::max(smem_x, (2 * kFftTile + 1) * Kx * int(sizeof(float2)));  // two tiles of lines, twiddles
+    smem_x = std::max(smem_x, strip_smem(kFftTile, Kx));
     for (int x = 0; x < Kx; ++x) wp.push_back({s, x, 0, 1});
-    smem_p = std::max(smem_p, (2 * Ky * Kz + Ky + Kz) * int(sizeof(float2)));  // two planes, twiddles
+    smem_p = std::max(smem_p, plane_smem(Ky, Kz));
+    plane_points = std::max(plane_points, 2 * Ky * Kz + Ky + Kz);
 
     // atoms
     const double* pos = states[s].positions;
@@ -767,8 +767,7 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   TRY(upload(e, "pair parameters by atom", prm_atom_dev, prm_atom));
   d.prm_atom = prm_atom_dev;
   TRY(alloc(e, "order", d.order, slots));
-  d.spread_sorted = spread_by_slot(int(slots)) ? 1 : 0;
-  TRY(alloc(e, "spread order", d.spread_atom, d.spread_sorted ? slots : 1));
+  TRY(alloc(e, "spread order", d.spread_atom, slots));
   TRY(alloc(e, "scatter order", d.tmp_order, slots));
   TRY(alloc(e, "pair coordinates", d.pc, slots));
   TRY(alloc(e, "pair parameters", d.prm, slots));
@@ -876,8 +875,12 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   TRY(alloc(e, "pme influence function", d.influence, wx.size() * size_t(d.influence_stride)));
   TRY(upload(e, "fft plane work", w_dev, wp));
   d.fft_p = w_dev; d.n_fft_p = int(wp.size());
-  // a whole x-plane in shared memory, twice, when every system's fits
-  d.fft_planes = smem_p <= kPlaneSmemLimit ? 1 : 0;
+  // whole x-planes by one CTA each, when every system's are small enough
+  d.fft_planes = plane_points <= kPlanePoints ? 1 : 0;
+  d.smem_p = smem_p;
+  d.smem_z = smem_z;
+  d.smem_y = smem_y;
+  d.smem_x = smem_x;
   e->n_mesh_items = int(wx.size());
   TRY(alloc(e, "energies", d.energy, size_t(n) * kECount));
   {
@@ -931,7 +934,7 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   TRY(alloc(e, "constraint failures", d.shake_failures, n));
 #undef TRY
   e->step = states[0].step;
-  set_pme_smem(smem_z, smem_y, smem_x, d.fft_planes ? smem_p : 0);
+  if (allow_pme_smem(kPmeSmemLimit)) return fail(e, MDB_ERR_DEVICE, "the transforms' shared memory was refused");
 
   // PME and the listed terms run beside the pair kernel at the highest
   // priority: their small, latency-bound grids take SMs as pair blocks
@@ -968,7 +971,7 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
     if (const int st = grow_tile_list(e)) return st;
   }
   // the slot-ordered spread's copy of the order, until the first step writes it
-  if (e->d.spread_sorted)
+  if (e->d.n_slots)
     CUDA_TRY(e, cudaMemcpyAsync(e->d.spread_atom, e->d.order, sizeof(int) * size_t(e->d.n_slots),
                                 cudaMemcpyDeviceToDevice, e->s0));
   launch_momentum(e->d, e->s0);
@@ -1027,6 +1030,8 @@ int evaluate_many(mdb_engine* e, const std::vector<int>& systems, double* forces
     CUDA_TRY(e, cudaStreamSynchronize(e->s0));  // `on` is pageable host memory
     dv.active = e->active;
   }
+  // the spread goes by the list's order at these positions (they may be the caller's)
+  CUDA_TRY(e, cudaMemcpyAsync(d.spread_atom, d.order, sizeof(int) * size_t(d.n_slots), cudaMemcpyDeviceToDevice, e->s0));
   launch_pme(dv, true, e->s0);
   launch_listed(dv, true, e->s0);
   launch_nonbonded(dv, true, e->s0);

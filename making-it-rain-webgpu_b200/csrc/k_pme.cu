@@ -16,7 +16,7 @@
 //   * the charge grid is int64 fixed point filled with atomics, so the spread
 //     is order independent and runs are bit-identical;
 //   * the transform is three passes, each CTA running a Stockham mixed-radix
-//     (2, 3, 4, 5, 7) FFT over whole lines in shared memory: one CTA per
+//     (2 to 10) FFT over whole lines in shared memory: one CTA per
 //     x-plane does z (int64 -> complex, real-to-complex, clearing the grid it
 //     read) and y; the x pass does x forward + convolution + x inverse; one
 //     CTA per x-plane does y inverse and z complex-to-real.  Meshes whose
@@ -27,6 +27,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "device_state.h"
 #include "prep.h"
@@ -36,98 +37,135 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// ------------------------------------------------------------ transforms --
+// Discrete transforms of R values in registers, R = 2 .. 10, so that a mesh
+// axis of up to 100 points takes two passes through shared memory.  SIGN is
+// the exponent's (-1 forward, +1 inverse).  Products that feed a sum are
+// written as fused steps, so every kernel that runs a line gives the same bits.
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y)); }
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
+template <int SIGN>
+__device__ __forceinline__ float2 times_i(float2 a) {
+  return SIGN < 0 ? make_float2(a.y, -a.x) : make_float2(-a.y, a.x);
+}
+// a + c b and a + SIGN i c b
+__device__ __forceinline__ float2 axpy(float c, float2 b, float2 a) { return make_float2(fmaf(c, b.x, a.x), fmaf(c, b.y, a.y)); }
+
+template <int SIGN>
+__device__ __forceinline__ void dft2(float2& a, float2& b) {
+  const float2 s = cadd(a, b);
+  b = csub(a, b);
+  a = s;
+}
+template <int SIGN>
+__device__ __forceinline__ void dft3(float2& a, float2& b, float2& c) {
+  const float2 t = cadd(b, c), u = axpy(-0.5f, t, a);
+  const float2 w = times_i<SIGN>(make_float2(__fmul_rn(0.866025404f, b.x - c.x), __fmul_rn(0.866025404f, b.y - c.y)));
+  a = cadd(a, t);
+  b = cadd(u, w);
+  c = csub(u, w);
+}
+template <int SIGN>
+__device__ __forceinline__ void dft4(float2& a, float2& b, float2& c, float2& d) {
+  const float2 p = cadd(a, c), q = csub(a, c), r = cadd(b, d), s = times_i<SIGN>(csub(b, d));
+  a = cadd(p, r);
+  c = csub(p, r);
+  b = cadd(q, s);
+  d = csub(q, s);
+}
+template <int SIGN>
+__device__ __forceinline__ void dft5(float2& a, float2& b, float2& c, float2& d, float2& e) {
+  const float c1 = 0.309016994f, c2 = -0.809016994f, s1 = 0.951056516f, s2 = 0.587785252f;
+  const float2 t1 = cadd(b, e), t2 = cadd(c, d), t3 = csub(b, e), t4 = csub(c, d);
+  const float2 m1 = axpy(c2, t2, axpy(c1, t1, a)), m2 = axpy(c1, t2, axpy(c2, t1, a));
+  const float2 n1 = times_i<SIGN>(axpy(s2, t4, make_float2(__fmul_rn(s1, t3.x), __fmul_rn(s1, t3.y))));
+  const float2 n2 = times_i<SIGN>(axpy(-s1, t4, make_float2(__fmul_rn(s2, t3.x), __fmul_rn(s2, t3.y))));
+  a = cadd(a, cadd(t1, t2));
+  b = cadd(m1, n1);
+  e = csub(m1, n1);
+  c = cadd(m2, n2);
+  d = csub(m2, n2);
 }
 
-// exp(-2 pi i t / R) for the small DFTs.
-__constant__ float2 kRoot3[3] = {{1.f, 0.f}, {-0.500000000f, -0.866025404f}, {-0.500000000f, 0.866025404f}};
-__constant__ float2 kRoot5[5] = {{1.f, 0.f},
-                                 {0.309016994f, -0.951056516f},
-                                 {-0.809016994f, -0.587785252f},
-                                 {-0.809016994f, 0.587785252f},
-                                 {0.309016994f, 0.951056516f}};
-__constant__ float2 kRoot7[7] = {{1.f, 0.f},
-                                 {0.623489802f, -0.781831482f},
-                                 {-0.222520934f, -0.974927912f},
-                                 {-0.900968868f, -0.433883739f},
-                                 {-0.900968868f, 0.433883739f},
-                                 {-0.222520934f, 0.974927912f},
-                                 {0.623489802f, 0.781831482f}};
-
-template <int R>
-__device__ __forceinline__ float2 root(int t, int sign) {
-  float2 w;
-  if (R == 3) w = kRoot3[t];
-  else if (R == 5) w = kRoot5[t];
-  else w = kRoot7[t];
-  if (sign > 0) w.y = -w.y;
-  return w;
-}
-
-template <int R>
-__device__ __forceinline__ void small_dft(float2* v, int sign) {
-  if (R == 2) {
-    const float2 a = v[0], b = v[1];
-    v[0] = make_float2(a.x + b.x, a.y + b.y);
-    v[1] = make_float2(a.x - b.x, a.y - b.y);
-  } else if (R == 4) {
-    const float2 a0 = make_float2(v[0].x + v[2].x, v[0].y + v[2].y);
-    const float2 a1 = make_float2(v[0].x - v[2].x, v[0].y - v[2].y);
-    const float2 b0 = make_float2(v[1].x + v[3].x, v[1].y + v[3].y);
-    float2 b1 = make_float2(v[1].x - v[3].x, v[1].y - v[3].y);
-    // multiply by -i (forward) or +i (inverse)
-    b1 = sign < 0 ? make_float2(b1.y, -b1.x) : make_float2(-b1.y, b1.x);
-    v[0] = make_float2(a0.x + b0.x, a0.y + b0.y);
-    v[2] = make_float2(a0.x - b0.x, a0.y - b0.y);
-    v[1] = make_float2(a1.x + b1.x, a1.y + b1.y);
-    v[3] = make_float2(a1.x - b1.x, a1.y - b1.y);
+template <int R, int SIGN>
+__device__ __forceinline__ void dft(float2* v) {
+  if constexpr (R == 2) dft2<SIGN>(v[0], v[1]);
+  else if constexpr (R == 3) dft3<SIGN>(v[0], v[1], v[2]);
+  else if constexpr (R == 4) dft4<SIGN>(v[0], v[1], v[2], v[3]);
+  else if constexpr (R == 5) dft5<SIGN>(v[0], v[1], v[2], v[3], v[4]);
+  else if constexpr (R == 7) {
+    const float c1 = 0.623489802f, c2 = -0.222520934f, c3 = -0.900968868f;
+    const float s1 = 0.781831482f, s2 = 0.974927912f, s3 = 0.433883739f;
+    const float2 p1 = cadd(v[1], v[6]), p2 = cadd(v[2], v[5]), p3 = cadd(v[3], v[4]);
+    const float2 q1 = csub(v[1], v[6]), q2 = csub(v[2], v[5]), q3 = csub(v[3], v[4]);
+    auto even = [&](float a, float b, float c) { return axpy(c, p3, axpy(b, p2, axpy(a, p1, v[0]))); };
+    auto odd = [&](float a, float b, float c) {
+      return times_i<SIGN>(axpy(c, q3, axpy(b, q2, make_float2(__fmul_rn(a, q1.x), __fmul_rn(a, q1.y)))));
+    };
+    const float2 e1 = even(c1, c2, c3), e2 = even(c2, c3, c1), e3 = even(c3, c1, c2);
+    const float2 o1 = odd(s1, s2, s3), o2 = odd(s2, -s3, -s1), o3 = odd(s3, -s1, s2);
+    v[0] = cadd(v[0], cadd(p1, cadd(p2, p3)));
+    v[1] = cadd(e1, o1);
+    v[6] = csub(e1, o1);
+    v[2] = cadd(e2, o2);
+    v[5] = csub(e2, o2);
+    v[3] = cadd(e3, o3);
+    v[4] = csub(e3, o3);
+  } else if constexpr (R == 8) {
+    dft4<SIGN>(v[0], v[2], v[4], v[6]);
+    dft4<SIGN>(v[1], v[3], v[5], v[7]);
+    const float h = 0.707106781f;
+    const float2 w1 = make_float2(h, SIGN * h), w3 = make_float2(-h, SIGN * h);
+    const float2 o1 = cmul(v[3], w1), o2 = times_i<SIGN>(v[5]), o3 = cmul(v[7], w3);
+    const float2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
+    v[0] = cadd(e0, o0); v[4] = csub(e0, o0);
+    v[1] = cadd(e1, o1); v[5] = csub(e1, o1);
+    v[2] = cadd(e2, o2); v[6] = csub(e2, o2);
+    v[3] = cadd(e3, o3); v[7] = csub(e3, o3);
+  } else if constexpr (R == 9) {
+#pragma unroll
+    for (int n = 0; n < 3; ++n) dft3<SIGN>(v[n], v[n + 3], v[n + 6]);  // v[n + 3 k] holds component k of column n
+    const float2 w1 = make_float2(0.766044443f, SIGN * 0.642787610f), w2 = make_float2(0.173648178f, SIGN * 0.984807753f),
+                 w4 = make_float2(-0.939692621f, SIGN * 0.342020143f);
+    v[4] = cmul(v[4], w1);
+    v[5] = cmul(v[5], w2);
+    v[7] = cmul(v[7], w2);
+    v[8] = cmul(v[8], w4);
+    // component k2 of the columns gives outputs k2, k2 + 3, k2 + 6
+#pragma unroll
+    for (int k = 0; k < 3; ++k) dft3<SIGN>(v[3 * k], v[3 * k + 1], v[3 * k + 2]);
+    const float2 t[9] = {v[0], v[3], v[6], v[1], v[4], v[7], v[2], v[5], v[8]};
+#pragma unroll
+    for (int k = 0; k < 9; ++k) v[k] = t[k];
   } else {
-    float2 out[R];
+    // R = 2 N, N odd: the prime-factor form (Good 1958), no twiddles between
+    static_assert(R == 6 || R == 10, "radix");
+    constexpr int N = R / 2;
+    float2 t[2][N];
 #pragma unroll
-    for (int m = 0; m < R; ++m) {
-      float2 s = v[0];
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int q = 1; q < R; ++q) {
-        const float2 w = root<R>((m * q) % R, sign);
-        s.x += v[q].x * w.x - v[q].y * w.y;
-        s.y += v[q].x * w.y + v[q].y * w.x;
-      }
-      out[m] = s;
+      for (int b = 0; b < N; ++b) t[a][b] = v[(N * a + 2 * b) % R];
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      if constexpr (N == 3) dft3<SIGN>(t[a][0], t[a][1], t[a][2]);
+      else dft5<SIGN>(t[a][0], t[a][1], t[a][2], t[a][3], t[a][4]);
     }
 #pragma unroll
-    for (int m = 0; m < R; ++m) v[m] = out[m];
+    for (int b = 0; b < N; ++b) dft2<SIGN>(t[0][b], t[1][b]);
+#pragma unroll
+    for (int k = 0; k < R; ++k) v[k] = t[k % 2][k % N];
   }
 }
 
-// Quotient by a per-stage divisor d > 1 without a division: magic = 2^32 / d
+// Quotient by a divisor d > 1 without a division: magic = 2^32 / d
 // rounded up is exact for numerator x divisor < 2^32 (all FFT indices here
 // are below 2^16).  d = 1 (magic 0) means the numerator itself.
 __device__ __forceinline__ unsigned quotient(unsigned x, unsigned magic) { return magic ? __umulhi(x, magic) : x; }
 __host__ __device__ __forceinline__ unsigned magic_for(unsigned d) { return d > 1 ? 0xFFFFFFFFu / d + 1u : 0u; }
-
-template <int R>
-__device__ __forceinline__ void stage_butterfly(const float2* src, float2* dst, int n, int j, int ns,
-                                                unsigned ns_magic, int step, const float2* tw, int sign) {
-  const int bf = n / R;
-  const int jq = int(quotient(unsigned(j), ns_magic));
-  const int k = j - jq * ns;
-  float2 v[R];
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    float2 x = src[j + q * bf];
-    if (q > 0 && k > 0) {
-      float2 w = tw[k * q * step];  // k q step < ns R step = n
-      if (sign > 0) w.y = -w.y;
-      x = cmul(x, w);
-    }
-    v[q] = x;
-  }
-  small_dft<R>(v, sign);
-  const int dest = jq * ns * R + k;
-#pragma unroll
-  for (int q = 0; q < R; ++q) dst[dest + q * ns] = v[q];
-}
 
 // A transform's twiddle table (n entries) into shared memory, where the
 // butterflies read it: a global read in every butterfly stage otherwise.
@@ -135,36 +173,102 @@ __device__ __forceinline__ void stage_twiddles(float2* dst, const float2* src, i
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(&src[i]);
 }
 
-// Stockham autosort over `nl` lines of length n in shared memory
-// (src/reference/fft.ts:128 is the f64 restatement of the same recursion).
-// Returns the buffer holding the result.
-__device__ float2* fft_lines(float2* a, float2* b, int n, int nl, const int* radices, int nrad,
-                             const float2* tw, int sign) {
-  int ns = 1;
-  for (int st = 0; st < nrad; ++st) {
-    const int r = radices[st];
-    const int bf = n / r;
-    const int step = n / (ns * r);
-    const unsigned bf_magic = magic_for(unsigned(bf)), ns_magic = magic_for(unsigned(ns));
-    for (int idx = threadIdx.x; idx < nl * bf; idx += blockDim.x) {
-      const int line = int(quotient(unsigned(idx), bf_magic)), j = idx - line * bf;
-      const float2* src = a + line * n;
-      float2* dst = b + line * n;
-      switch (r) {
-        case 2: stage_butterfly<2>(src, dst, n, j, ns, ns_magic, step, tw, sign); break;
-        case 3: stage_butterfly<3>(src, dst, n, j, ns, ns_magic, step, tw, sign); break;
-        case 4: stage_butterfly<4>(src, dst, n, j, ns, ns_magic, step, tw, sign); break;
-        case 5: stage_butterfly<5>(src, dst, n, j, ns, ns_magic, step, tw, sign); break;
-        default: stage_butterfly<7>(src, dst, n, j, ns, ns_magic, step, tw, sign); break;
+// One axis' transform plan: the length and its radices, four bits each from
+// the first stage up (plan_radices).
+struct Axis {
+  int n;
+  unsigned plan;
+};
+__device__ __forceinline__ int radix_at(Axis ax, int stage) { return (ax.plan >> (4 * stage)) & 15; }
+__device__ __forceinline__ int stages_of(Axis ax) { return (35 - __clz(ax.plan)) >> 2; }
+
+// One Stockham stage of radix R over `nl` lines of length ax.n (ns = the
+// product of the radices before it): butterfly (j, l) takes elements
+// j + q n/R of line l from `load` and gives elements to `store`.  Lines vary
+// fastest over the threads, so with line-fastest layouts every access is
+// contiguous.
+template <int R, int SIGN, class Load, class Store>
+__device__ __forceinline__ void stage_of(int n, int ns, int nl, unsigned nl_magic, const float2* tw, Load load,
+                                         Store store) {
+  const int bf = n / R, step = bf / ns;
+  const unsigned ns_magic = magic_for(unsigned(ns));
+  for (int idx = threadIdx.x; idx < nl * bf; idx += blockDim.x) {
+    const int j = int(quotient(unsigned(idx), nl_magic)), l = idx - j * nl;
+    const int jq = ns == 1 ? j : (step == 1 ? 0 : int(quotient(unsigned(j), ns_magic)));
+    const int k = j - jq * ns;
+    float2 v[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = load(j + q * bf, l);
+    if (ns > 1) {
+#pragma unroll
+      for (int q = 1; q < R; ++q) {
+        float2 w = tw[k * q * step];  // k q step < ns R step = n
+        if (SIGN > 0) w.y = -w.y;
+        v[q] = cmul(v[q], w);
       }
     }
+    dft<R, SIGN>(v);
+    const int dest = jq * ns * R + k;
+#pragma unroll
+    for (int q = 0; q < R; ++q) store(dest + q * ns, l, v[q]);
+  }
+}
+
+#define MDB_RADIX_SWITCH(r, CALL) \
+  switch (r) {                    \
+    case 2: CALL(2); break;       \
+    case 3: CALL(3); break;       \
+    case 4: CALL(4); break;       \
+    case 5: CALL(5); break;       \
+    case 6: CALL(6); break;       \
+    case 7: CALL(7); break;       \
+    case 8: CALL(8); break;       \
+    case 9: CALL(9); break;       \
+    default: CALL(10); break;     \
+  }
+
+// All stages of `nl` lines: the first loads through `load`, the last stores
+// through `store` (each given (t, l)), those between go through the two
+// buffers, element (t, l) at t * pitch + l.  Ends with a barrier.  Each kind of
+// stage is compiled on its own: a block runs few instructions more than once,
+// so the fewer it has to fetch the better.
+template <int SIGN, class Load, class Store>
+__device__ __forceinline__ void transform(Axis ax, int nl, int pitch, const float2* tw, float2* a, float2* b, Load load,
+                                          Store store) {
+  const int count = stages_of(ax);
+  const unsigned nl_magic = magic_for(unsigned(nl));
+  const int n = ax.n;
+  int ns = radix_at(ax, 0);
+  auto from = [&](const float2* p) { return [p, pitch](int t, int l) { return p[t * pitch + l]; }; };
+  auto to = [&](float2* p) { return [p, pitch](int t, int l, float2 v) { p[t * pitch + l] = v; }; };
+  if (count == 1) {
+#define MDB_STAGE(R) stage_of<R, SIGN>(n, 1, nl, nl_magic, tw, load, store)
+    MDB_RADIX_SWITCH(ns, MDB_STAGE)
+#undef MDB_STAGE
     __syncthreads();
-    float2* t = a;
-    a = b;
-    b = t;
+    return;
+  }
+#define MDB_STAGE(R) stage_of<R, SIGN>(n, 1, nl, nl_magic, tw, load, to(b))
+  MDB_RADIX_SWITCH(ns, MDB_STAGE)
+#undef MDB_STAGE
+  __syncthreads();
+  float2 *cur = b, *next = a;
+  for (int st = 1; st < count - 1; ++st) {
+    const int r = radix_at(ax, st);
+#define MDB_STAGE(R) stage_of<R, SIGN>(n, ns, nl, nl_magic, tw, from(cur), to(next))
+    MDB_RADIX_SWITCH(r, MDB_STAGE)
+#undef MDB_STAGE
+    __syncthreads();
+    float2* t = cur;
+    cur = next;
+    next = t;
     ns *= r;
   }
-  return a;
+  const int r = radix_at(ax, count - 1);
+#define MDB_STAGE(R) stage_of<R, SIGN>(n, ns, nl, nl_magic, tw, from(cur), store)
+  MDB_RADIX_SWITCH(r, MDB_STAGE)
+#undef MDB_STAGE
+  __syncthreads();
 }
 
 // ------------------------------------------------------------- splines ----
@@ -199,131 +303,77 @@ __device__ __forceinline__ void bspline5(float w, float* th, float* dth) {
   th[0] = dv * (1.f - w) * th[0];
 }
 
-struct Spline {
-  int base[3];
-  float th[3][5], dth[3][5];
-};
-
-__device__ __forceinline__ void spline_for(const SysDev& S, long long x, long long y, long long z,
-                                           Spline& sp, bool derivatives) {
-  const long long u[3] = {fixed_mul(x, S.umat[0]) + fixed_mul(y, S.umat[1]) + fixed_mul(z, S.umat[2]),
-                          fixed_mul(y, S.umat[3]) + fixed_mul(z, S.umat[4]), fixed_mul(z, S.umat[5])};
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const long long cell = u[k] >> 32;
-    const float w = static_cast<float>(static_cast<unsigned int>(u[k] & 0xffffffffll)) * 2.3283064365386963e-10f;
-    long long b = (cell - (kPmeOrder - 1)) % S.grid[k];
-    if (b < 0) b += S.grid[k];
-    sp.base[k] = static_cast<int>(b);
-    bspline5(w, sp.th[k], derivatives ? sp.dth[k] : nullptr);
-  }
+// One axis of an atom's spline from its position: the base mesh index and the
+// weights (and derivatives) of its five points.
+__device__ __forceinline__ int spline_axis(const SysDev& S, int axis, long long x, long long y, long long z, float* th,
+                                           float* dth) {
+  const long long u = axis == 0   ? fixed_mul(x, S.umat[0]) + fixed_mul(y, S.umat[1]) + fixed_mul(z, S.umat[2])
+                      : axis == 1 ? fixed_mul(y, S.umat[3]) + fixed_mul(z, S.umat[4])
+                                  : fixed_mul(z, S.umat[5]);
+  const float w = static_cast<float>(static_cast<unsigned int>(u & 0xffffffffll)) * 2.3283064365386963e-10f;
+  const int K = S.grid[axis];
+  // an atom within a few cells of its box needs a few subtractions, not a
+  // 64-bit remainder
+  long long b = (u >> 32) - (kPmeOrder - 1);
+  if (b < -2ll * K || b >= 3ll * K) b %= K;
+  while (b < 0) b += K;
+  while (b >= K) b -= K;
+  bspline5(w, th, dth);
+  return static_cast<int>(b);
 }
 
 // ---------------------------------------------------------------- spread --
-// Both spreads read nothing the list kernels write, so they run on their own
-// stream while the list kernels sort and rebuild.
-//
-// By atom (engines under one block of slots per SM): a block takes up to
-// kSplineAtoms atoms: their splines are computed once each into shared memory,
-// then all its threads share the 25 (ix, iy) rows of 5 z points per atom, so
-// no thread makes more than a few atomics in a row (one thread per atom making
-// all 125 left the kernel latency-bound at any size).  Consecutive atoms are
-// neighbours in space (molecules, solvent laid down in order), so block b
-// takes atoms b, b + B, b + 2B, ... (B blocks): atoms spread at once sit far
-// apart on the mesh.  The grid is int64 fixed point: the order of the atomics
-// does not change the sums.
-constexpr int kSplineAtoms = 128;  // at most; 32, 64 and 256 measured slower
-static_assert(kSplineAtoms <= kThreads, "one thread per atom computes the splines");
+// The spread reads nothing the list kernels write, so it runs on its own
+// stream while the list kernels sort and rebuild: it goes by the slots of a
+// snapshot of the list's sorted order that the integrator writes at the end of
+// every step (`spread_atom`), never by the order the list kernels are
+// rewriting.  A block takes P consecutive slots -- P / 32 super-clusters along
+// the space-filling curve, a compact piece of space -- adds their charges into
+// a patch of the mesh in shared memory, and adds the patch's nonzero points to
+// the grid: an eighth to a quarter of the global atomics of spreading each
+// atom's 125 points directly.  The patch holds the block's spline bases
+// (unwrapped around its first atom) plus the 5-point stencil; a block whose
+// patch would not fit (a cluster torn across a jump of the curve) or whose
+// slots reach into the next system spreads directly.  The grid is int64 fixed
+// point and every contribution the same value either way, so the grid is the
+// same to the bit whatever the order and the route.  What bounds it is a
+// block's chain of loads, splines, shared atomics and grid atomics; hence
+// short blocks for small engines.  Measured against 128 slots a block from
+// 148 blocks up and atomics straight to the grid below: 12k-atom peptide (32
+// slots) 13.6 -> 9.2 us, 27k-atom octahedron (64) 24.2 -> 14.4 us, 100k atoms
+// (128) 45.6 -> 40.7 us, 64-system ensemble (128) 248 -> 229 us; the
+// octahedron at 128 slots took 26.2 us.
+constexpr int kPatchPoints = 4096;  // 32 KB in two 32-bit halves
 
-struct SplineTable {
-  int base[kSplineAtoms][3];
-  float th[kSplineAtoms][3][5];
-  float q[kSplineAtoms];
-  int sys[kSplineAtoms];
-};
-
-__global__ void __launch_bounds__(kThreads) k_spread(Dev d, int per) {
-  wait_for_predecessor();
-  __shared__ SplineTable t;
-  const int nblocks = gridDim.x;
-  for (int first = blockIdx.x; first < d.n_atoms; first += nblocks * per) {
-    // atom k (< per <= kSplineAtoms) of this round is first + k * nblocks
-    if (threadIdx.x < per) {
-      const int k = threadIdx.x, a = first + k * nblocks;
-      float q = 0.f;
-      if (a < d.n_atoms && sys_active(d, d.atom_sys[a])) q = d.prm_atom[a].w;
-      t.q[k] = q;
-      if (q != 0.f) {
-        const int s = d.atom_sys[a];
-        Spline sp;
-        spline_for(d.sys[s], d.px[a], d.py[a], d.pz[a], sp, false);
-        t.sys[k] = s;
-        for (int ax = 0; ax < 3; ++ax) {
-          t.base[k][ax] = sp.base[ax];
-          for (int i = 0; i < kPmeOrder; ++i) t.th[k][ax][i] = sp.th[ax][i];
-        }
-      }
-    }
-    __syncthreads();
-    for (int w = threadIdx.x; w < per * kPmeOrder * kPmeOrder; w += blockDim.x) {
-      const int k = w / (kPmeOrder * kPmeOrder), r = w - k * kPmeOrder * kPmeOrder;
-      const float q = t.q[k];
-      if (q == 0.f) continue;
-      const SysDev& S = d.sys[t.sys[k]];
-      const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2];
-      const int ix = r / kPmeOrder, iy = r - ix * kPmeOrder;
-      int gx = t.base[k][0] + ix;
-      if (gx >= Kx) gx -= Kx;
-      int gy = t.base[k][1] + iy;
-      if (gy >= Ky) gy -= Ky;
-      const float wxy = q * t.th[k][0][ix] * t.th[k][1][iy];
-      unsigned long long* row = d.qgrid + S.grid_off + (static_cast<long long>(gx) * Ky + gy) * Kz;
-#pragma unroll
-      for (int iz = 0; iz < kPmeOrder; ++iz) {
-        int gz = t.base[k][2] + iz;
-        if (gz >= Kz) gz -= Kz;
-        add_fixed(&row[gz], wxy * t.th[k][2][iz]);
-      }
-    }
-    __syncthreads();
-  }
+// x 2^32 rounded to an integer, as hi 2^20 + lo, for |x| < 1024: both
+// roundings are f32 additions of 1.5 2^23 (whose low bits then hold the
+// integer), in place of a float-to-int64 conversion at a sixteenth of the f32
+// rate.  hi takes the multiple of 2^-12 nearest x, what is left is exact, and
+// its rounding to 2^-32 is the whole value's (2^20 is even: ties agree).
+__device__ __forceinline__ void split_fixed(float x, int& hi, int& lo) {
+  constexpr float kMagic = 12582912.f;  // 1.5 2^23
+  const float t = fmaf(x, 4096.f, kMagic);
+  const float rest = fmaf(x, 4096.f, -__fsub_rn(t, kMagic));
+  hi = __float_as_int(t) - 0x4B400000;
+  lo = __float_as_int(fmaf(rest, 1048576.f, kMagic)) - 0x4B400000;
 }
 
-// By slot (larger engines): the slots of a snapshot of the list's sorted
-// order that the integrator writes at the end of every step (`spread_atom`),
-// so the order the list kernels are rewriting is never read.  A block takes
-// 128 consecutive slots -- four super-clusters along the space-filling curve,
-// a compact piece of space -- adds their charges into a patch of the mesh in
-// shared memory, and adds the patch's nonzero points to the grid: about a
-// fifth of the global atomics of spreading each atom's 125 points directly.
-// The patch holds the block's spline bases (unwrapped around its first atom)
-// plus the 5-point stencil; a block whose patch would not fit (a cluster torn
-// across a jump of the curve) or whose slots reach into the next system
-// spreads directly.  Every contribution is the same fixed-point value as in
-// the by-atom spread, so the grid is the same to the bit.  The shared-memory
-// phases make a block's chain longer: below one block per SM (the 12k-atom
-// peptide) the by-atom kernel finishes first; above it this one takes less
-// time (the 27k-atom octahedron 7% less, a 64-system ensemble of 627k atoms
-// 45% less).
-constexpr int kPatchSlots = 128;
-constexpr int kPatchPoints = 4096;  // 32 KB of int64
-
-__global__ void __launch_bounds__(kThreads) k_spread_sorted(Dev d) {
+template <int P>
+__global__ void __launch_bounds__(kThreads) k_spread(Dev d) {
   wait_for_predecessor();
-  // the patch's fixed-point sums in two 32-bit halves (hi = v >> 20 signed,
-  // lo = the low 20 bits), so the adds are 32-bit shared atomics: at most 128
-  // atoms add to a point, which keeps both halves far from overflow
-  __shared__ int patch_hi[kPatchPoints];
-  __shared__ unsigned int patch_lo[kPatchPoints];
-  __shared__ int base[kPatchSlots][3];
-  __shared__ float th[kPatchSlots][3][5];
-  __shared__ float qs[kPatchSlots];
-  __shared__ int sysk[kPatchSlots];
-  __shared__ int lo_part[kPatchSlots / 32][3], hi_part[kPatchSlots / 32][3];
-  __shared__ int lo[3], ext[3], use_patch;
-  const int first = blockIdx.x * kPatchSlots;
+  // the patch's sums in two 32-bit halves (hi 2^20 + lo), so the adds are
+  // 32-bit shared atomics: at most P atoms add to a point, which keeps both
+  // halves far from overflow
+  __shared__ int patch_hi[kPatchPoints], patch_lo[kPatchPoints];
+  __shared__ int base[P][3];
+  __shared__ float th[P][3][5];
+  __shared__ float qs[P];
+  __shared__ int sysk[P];
+  __shared__ int lo[3], hi[3];
+  const int t = threadIdx.x;
+  const int first = blockIdx.x * P;
   if (first >= d.n_slots) return;
-  const int last = min(d.n_slots, first + kPatchSlots) - 1;
+  const int last = min(d.n_slots, first + P) - 1;
   // a block may hold the end of one system and the start of the next: then
   // every atom spreads directly into its own system's grid
   const int s = d.slot_sys[first];
@@ -331,110 +381,106 @@ __global__ void __launch_bounds__(kThreads) k_spread_sorted(Dev d) {
   const int a0 = d.spread_atom[first];
   if (one_system && (a0 < 0 || !sys_active(d, s))) return;  // padding only, or a skipped system
   const SysDev& S = d.sys[s];
-  const int K[3] = {S.grid[0], S.grid[1], S.grid[2]};
-  // splines; in a one-system block the bases unwrapped around the first slot's atom
-  const int t = threadIdx.x;
-  int ub[3] = {0, 0, 0};
-  bool live = false;
-  if (t < kPatchSlots) {
-    const int gs = first + t;
-    float q = 0.f;
-    int st = s;
-    if (gs <= last) {
-      st = d.slot_sys[gs];
-      const int a = d.spread_atom[gs];
-      if (a >= 0 && sys_active(d, st)) q = d.prm_atom[a].w;
-      if (q != 0.f) {
-        const SysDev& Sa = d.sys[st];
-        Spline sp;
-        spline_for(Sa, d.px[a], d.py[a], d.pz[a], sp, false);
-        Spline sp0;
-        if (one_system) spline_for(S, d.px[a0], d.py[a0], d.pz[a0], sp0, false);
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-          int b = sp.base[ax];
-          if (one_system) {
-            const int r = sp0.base[ax];
-            if (b - r > K[ax] / 2) b -= K[ax];
-            if (r - b > K[ax] / 2) b += K[ax];
-          }
-          ub[ax] = b;
-          base[t][ax] = b;
-          for (int i = 0; i < kPmeOrder; ++i) th[t][ax][i] = sp.th[ax][i];
-        }
-        live = true;
-      }
-    }
-    qs[t] = q;
-    sysk[t] = st;
+  if (t < 3) {
+    lo[t] = 1 << 30;
+    hi[t] = -(1 << 30);
   }
-  // the bases' range: warp reductions, then the block's
-  if (t < kPatchSlots) {
-    const int big = 1 << 30;
+  __syncthreads();
+  // splines, a thread per atom and axis (a warp's lanes share the axis)
+  for (int w = t; w < 3 * P; w += blockDim.x) {
+    const int axis = w / P, k = w - axis * P, gs = first + k;
+    const int a = gs <= last ? d.spread_atom[gs] : -1;
+    const int st = gs <= last && !one_system ? d.slot_sys[gs] : s;
+    const bool live = a >= 0 && sys_active(d, st);
+    if (axis == 0) {
+      qs[k] = live ? d.prm_atom[a].w : 0.f;
+      sysk[k] = st;
+    }
+    if (live) {
+      float weights[5];
+      base[k][axis] = spline_axis(d.sys[st], axis, d.px[a], d.py[a], d.pz[a], weights, nullptr);
 #pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-      const int mn = __reduce_min_sync(0xffffffffu, live ? ub[ax] : big);
-      const int mx = __reduce_max_sync(0xffffffffu, live ? ub[ax] : -big);
+      for (int i = 0; i < kPmeOrder; ++i) th[k][axis][i] = weights[i];
+    }
+  }
+  __syncthreads();
+  if (one_system) {
+    // the bases unwrapped around the first atom's, and their range
+    for (int w = t; w < 3 * P; w += blockDim.x) {
+      const int axis = w / P, k = w - axis * P, K = S.grid[axis];
+      const bool live = qs[k] != 0.f;
+      int b = 0;
+      if (live) {
+        const int r = base[0][axis];
+        b = base[k][axis];
+        if (b - r > K / 2) b -= K;
+        if (r - b > K / 2) b += K;
+      }
+      const int mn = __reduce_min_sync(0xffffffffu, live ? b : 1 << 30);
+      const int mx = __reduce_max_sync(0xffffffffu, live ? b : -(1 << 30));
       if ((t & 31) == 0) {
-        lo_part[t >> 5][ax] = mn;
-        hi_part[t >> 5][ax] = mx;
+        atomicMin(&lo[axis], mn);
+        atomicMax(&hi[axis], mx);
       }
-    }
-  }
-  __syncthreads();
-  if (t == 0) {
-    int points = 1;
-    bool fits = one_system;
-    for (int ax = 0; ax < 3; ++ax) {
-      int mn = lo_part[0][ax], mx = hi_part[0][ax];
-      for (int w = 1; w < kPatchSlots / 32; ++w) {
-        mn = min(mn, lo_part[w][ax]);
-        mx = max(mx, hi_part[w][ax]);
-      }
-      lo[ax] = mn;
-      ext[ax] = mx - mn + kPmeOrder;
-      fits = fits && mx >= mn && ext[ax] <= K[ax];
-      points *= max(ext[ax], 1);
-    }
-    use_patch = fits && points <= kPatchPoints;
-  }
-  __syncthreads();
-  if (use_patch) {
-    const int ex = ext[0], ey = ext[1], ez = ext[2], np = ex * ey * ez;
-    for (int i = t; i < np; i += blockDim.x) {
-      patch_hi[i] = 0;
-      patch_lo[i] = 0u;
+      if (live && k > 0) base[k][axis] = b;
     }
     __syncthreads();
-    for (int w = t; w < kPatchSlots * kPmeOrder * kPmeOrder; w += blockDim.x) {
+  }
+  bool patch = one_system;
+  int points = 1, ext[3];
+#pragma unroll
+  for (int ax = 0; ax < 3; ++ax) {
+    ext[ax] = hi[ax] - lo[ax] + kPmeOrder;
+    patch = patch && hi[ax] >= lo[ax] && ext[ax] <= S.grid[ax];
+    if (patch) points *= ext[ax];
+    patch = patch && points <= kPatchPoints;
+  }
+  if (patch) {
+    const int ey = ext[1], ez = ext[2], lx = lo[0], ly = lo[1], lz = lo[2];
+    for (int i = t; i < points; i += blockDim.x) patch_hi[i] = patch_lo[i] = 0;
+    __syncthreads();
+    for (int w = t; w < P * kPmeOrder * kPmeOrder; w += blockDim.x) {
       const int k = w / (kPmeOrder * kPmeOrder), r = w - k * kPmeOrder * kPmeOrder;
       const float q = qs[k];
       if (q == 0.f) continue;
       const int ix = r / kPmeOrder, iy = r - ix * kPmeOrder;
       const float wxy = q * th[k][0][ix] * th[k][1][iy];
-      const int row = ((base[k][0] - lo[0] + ix) * ey + (base[k][1] - lo[1] + iy)) * ez + (base[k][2] - lo[2]);
+      const int row = ((base[k][0] - lx + ix) * ey + (base[k][1] - ly + iy)) * ez + (base[k][2] - lz);
+      const bool small = fabsf(wxy) < 1000.f;  // any charge there is; the weights are below 1
 #pragma unroll
       for (int iz = 0; iz < kPmeOrder; ++iz) {
-        const long long v = to_fixed(wxy * th[k][2][iz]);
-        atomicAdd(&patch_hi[row + iz], static_cast<int>(v >> 20));
-        atomicAdd(&patch_lo[row + iz], static_cast<unsigned int>(v & 0xFFFFF));
+        const float x = wxy * th[k][2][iz];
+        int h, l;
+        if (small) {
+          split_fixed(x, h, l);
+        } else {
+          const long long v = to_fixed(x);
+          h = static_cast<int>(v >> 20);
+          l = static_cast<int>(v & 0xFFFFF);
+        }
+        atomicAdd(&patch_hi[row + iz], h);
+        atomicAdd(&patch_lo[row + iz], l);
       }
     }
     __syncthreads();
-    for (int i = t; i < np; i += blockDim.x) {
-      const unsigned long long v = static_cast<unsigned long long>(
-          (static_cast<long long>(patch_hi[i]) << 20) + static_cast<long long>(patch_lo[i]));
+    const unsigned plane_magic = magic_for(unsigned(ey * ez)), row_magic = magic_for(unsigned(ez));
+    const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2];
+    unsigned long long* grid = d.qgrid + S.grid_off;
+    for (int i = t; i < points; i += blockDim.x) {
+      const long long v = static_cast<long long>(patch_hi[i]) * (1ll << 20) + patch_lo[i];
       if (!v) continue;
-      const int px = i / (ey * ez), rem = i - px * ey * ez, py = rem / ez, pz = rem - py * ez;
-      int gx = (lo[0] + px) % K[0], gy = (lo[1] + py) % K[1], gz = (lo[2] + pz) % K[2];
-      if (gx < 0) gx += K[0];
-      if (gy < 0) gy += K[1];
-      if (gz < 0) gz += K[2];
-      atomicAdd(d.qgrid + S.grid_off + (static_cast<long long>(gx) * K[1] + gy) * K[2] + gz, v);
+      const int px = int(quotient(unsigned(i), plane_magic)), rem = i - px * ey * ez;
+      const int py = int(quotient(unsigned(rem), row_magic)), pz = rem - py * ez;
+      // unwrapped bases lie within half a mesh of one in it: one turn at most
+      int gx = lx + px, gy = ly + py, gz = lz + pz;
+      gx += gx < 0 ? Kx : (gx >= Kx ? -Kx : 0);
+      gy += gy < 0 ? Ky : (gy >= Ky ? -Ky : 0);
+      gz += gz < 0 ? Kz : (gz >= Kz ? -Kz : 0);
+      add_fixed64(grid + (static_cast<long long>(gx) * Ky + gy) * Kz + gz, v);
     }
   } else {
     // the direct spread of each atom's 125 points, into its own system's grid
-    for (int w = t; w < kPatchSlots * kPmeOrder * kPmeOrder; w += blockDim.x) {
+    for (int w = t; w < P * kPmeOrder * kPmeOrder; w += blockDim.x) {
       const int k = w / (kPmeOrder * kPmeOrder), r = w - k * kPmeOrder * kPmeOrder;
       const float q = qs[k];
       if (q == 0.f) continue;
@@ -456,56 +502,298 @@ __global__ void __launch_bounds__(kThreads) k_spread_sorted(Dev d) {
   }
 }
 
-// --------------------------------------------------------------- z pass ---
-// int64 charge grid -> complex half spectrum along z, clearing the grid.
-__global__ void __launch_bounds__(kThreads) k_fft_z_forward(Dev d) {
-  wait_for_predecessor();
-  extern __shared__ float2 smem[];
-  const FftWork w = d.fft_z[blockIdx.x];
-  if (!sys_active(d, w.sys)) return;  // the whole block: before any barrier
-  const SysDev& S = d.sys[w.sys];
-  const int Kz = S.grid[2], kzh = S.kzh;
-  float2* A = smem;
-  float2* B = smem + w.n * Kz;
-  unsigned long long* grid = d.qgrid + S.grid_off + static_cast<long long>(w.a) * Kz;
-  for (int i = threadIdx.x; i < w.n * Kz; i += blockDim.x) {
-    const long long v = static_cast<long long>(grid[i]);
-    A[i] = make_float2(from_fixed(v), 0.f);
-    grid[i] = 0ull;
+// ---------------------------------------------------------------- passes --
+// A mesh as the passes see it: the engine's tables of one system, or the
+// allocation-free path's.
+struct Mesh {
+  Axis x, y, z;
+  int kzh;  // Kz / 2 + 1
+  unsigned long long* charge;  // [Kx][Ky][Kz], 2^32 fixed point; cleared as it is read
+  float2* spectrum;            // [Kx][Ky][kzh]
+  float* potential;            // [Kx][Ky][Kz]
+  const float2 *twx, *twy, *twz;
+};
+
+__device__ __forceinline__ Mesh mesh_of(const Dev& d, const SysDev& S) {
+  Mesh m;
+  m.x = {S.grid[0], S.plan[0]};
+  m.y = {S.grid[1], S.plan[1]};
+  m.z = {S.grid[2], S.plan[2]};
+  m.kzh = S.kzh;
+  m.charge = d.qgrid + S.grid_off;
+  m.spectrum = d.cgrid + S.cgrid_off;
+  m.potential = d.phi + S.grid_off;
+  m.twx = d.twiddles + S.tw_off[0];
+  m.twy = d.twiddles + S.tw_off[1];
+  m.twz = d.twiddles + S.tw_off[2];
+  return m;
+}
+
+// The z transforms take real lines two at a time: lines y = 2p and 2p + 1 of
+// an x-plane are the real and the imaginary part of one complex line, whose
+// transform Z gives both: (Z_k + conj Z_-k) / 2 and (Z_k - conj Z_-k) / 2i.
+// The pairs are counted inside the plane (an odd Ky leaves the last line
+// alone), whichever kernel runs them, so all give the same bits.
+__device__ __forceinline__ float2 line_of_pair(float2 a, float2 b, bool odd) {  // a = Z_k, b = Z_-k
+  return odd ? make_float2(0.5f * __fadd_rn(a.y, b.y), 0.5f * __fsub_rn(b.x, a.x))
+             : make_float2(0.5f * __fadd_rn(a.x, b.x), 0.5f * __fsub_rn(a.y, b.y));
+}
+// The inverse: element t of the complex line of two half spectra.  Elements
+// 0 and Kz/2 of a real line's spectrum are real; what rounding left in their
+// imaginary parts would run into the other line.
+template <class Half>
+__device__ __forceinline__ float2 pair_of_lines(int Kz, int t, bool second, Half half) {
+  const int k = 2 * t <= Kz ? t : Kz - t;
+  float2 a = half(0, k), b = second ? half(1, k) : make_float2(0.f, 0.f);
+  if (t == 0 || 2 * t == Kz) a.y = b.y = 0.f;
+  if (k != t) {
+    a.y = -a.y;
+    b.y = -b.y;
   }
-  __syncthreads();
-  const float2* R = fft_lines(A, B, Kz, w.n, S.radices[2], S.nradix[2], d.twiddles + S.tw_off[2], -1);
-  float2* out = d.cgrid + S.cgrid_off + static_cast<long long>(w.a) * kzh;
-  for (int i = threadIdx.x; i < w.n * kzh; i += blockDim.x) {
-    const int line = i / kzh, k = i - line * kzh;
-    out[i] = R[line * Kz + k];
+  return make_float2(__fsub_rn(a.x, b.y), __fadd_rn(a.y, b.x));
+}
+
+// Pitches and sizes of the plane passes' two shared buffers: z lines
+// [Kz][pairs] (an odd pitch keeps the charge loads' bank conflicts at two), y
+// lines [Ky][kzh].
+__host__ __device__ __forceinline__ int pair_pitch(int lines) { return ((lines + 1) / 2) | 1; }
+__host__ __device__ __forceinline__ int plane_buffer(int Ky, int Kz) {
+  const int z = Kz * pair_pitch(Ky), y = Ky * (Kz / 2 + 1);
+  return z > y ? z : y;
+}
+
+// Charges of `lines` consecutive z lines (from an even one of the plane) into
+// paired complex lines, clearing the grid ("consumer clears": the next spread
+// starts from zero).
+__device__ __forceinline__ void load_charges(unsigned long long* grid, int lines, int Kz, int pitch, float2* a) {
+  const unsigned kz_magic = magic_for(unsigned(Kz));
+  float* flat = reinterpret_cast<float*>(a);
+  const int total = lines * Kz;
+  // four loads in flight per thread before any is used
+  for (int i0 = threadIdx.x; i0 < total; i0 += 4 * blockDim.x) {
+    long long v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * blockDim.x;
+      v[u] = i < total ? static_cast<long long>(__ldcg(&grid[i])) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * blockDim.x;
+      if (i < total) {
+        const int y = int(quotient(unsigned(i), kz_magic)), z = i - y * Kz;
+        flat[(z * pitch + (y >> 1)) * 2 + (y & 1)] = from_fixed(v[u]);
+        grid[i] = 0ull;
+      }
+    }
+  }
+  if (lines & 1)
+    for (int z = threadIdx.x; z < Kz; z += blockDim.x) a[z * pitch + (lines >> 1)].y = 0.f;
+}
+
+// Real lines out of paired complex lines.
+__device__ __forceinline__ void store_potential(float* out, int lines, int Kz, int pitch, const float2* a) {
+  const unsigned kz_magic = magic_for(unsigned(Kz));
+  const float* flat = reinterpret_cast<const float*>(a);
+  for (int i = threadIdx.x; i < lines * Kz; i += blockDim.x) {
+    const int y = int(quotient(unsigned(i), kz_magic)), z = i - y * Kz;
+    out[i] = flat[(z * pitch + (y >> 1)) * 2 + (y & 1)];
   }
 }
 
-// --------------------------------------------------------------- y pass ---
-__global__ void __launch_bounds__(kThreads) k_fft_y(Dev d, int sign) {
-  wait_for_predecessor();
-  extern __shared__ float2 smem[];
-  const FftWork w = d.fft_y[blockIdx.x];
-  if (!sys_active(d, w.sys)) return;  // the whole block: before any barrier
-  const SysDev& S = d.sys[w.sys];
-  const int Ky = S.grid[1], kzh = S.kzh;
-  float2* A = smem;
-  float2* B = smem + w.n * Ky;
-  float2* base = d.cgrid + S.cgrid_off + static_cast<long long>(w.a) * Ky * kzh + w.b;
-  for (int i = threadIdx.x; i < w.n * Ky; i += blockDim.x) {
-    const int y = i / w.n, l = i - y * w.n;
-    A[l * Ky + y] = base[static_cast<long long>(y) * kzh + l];
-  }
+// Whole x-planes: z and y of one plane by one CTA, so a transform in one
+// direction is two launches (with the x pass) and each has a plane of work.
+// What bounds them is the chain of one CTA (a load, four stages, four
+// barriers, a store), not bandwidth: 50^3 moves 2 MB.  Two real lines to a
+// complex one halve the z stages; radices up to 10 make an axis two stages;
+// the y transform's first stage separates the pairs as it loads and its last
+// stores to global memory, so nothing is copied between.  Measured with the x
+// pass against radices up to 5, lines one at a time and copies between the
+// axes: 50^3 27.7 -> 21.2 us, 60 x 54 x 48 30.6 -> 21.4 us, 81^3 54 -> 29 us,
+// the 64-system ensemble's meshes 274 -> 92 us.
+__device__ __forceinline__ void plane_forward(const Mesh& m, int x, float2* smem) {
+  const int Ky = m.y.n, Kz = m.z.n, kzh = m.kzh, pitch = pair_pitch(Ky), size = plane_buffer(Ky, Kz);
+  float2 *a = smem, *b = smem + size, *twz = smem + 2 * size, *twy = twz + Kz;
+  stage_twiddles(twz, m.twz, Kz);
+  stage_twiddles(twy, m.twy, Ky);
+  load_charges(m.charge + static_cast<long long>(x) * Ky * Kz, Ky, Kz, pitch, a);
   __syncthreads();
-  const float2* R = fft_lines(A, B, Ky, w.n, S.radices[1], S.nradix[1], d.twiddles + S.tw_off[1], sign);
-  for (int i = threadIdx.x; i < w.n * Ky; i += blockDim.x) {
-    const int y = i / w.n, l = i - y * w.n;
-    base[static_cast<long long>(y) * kzh + l] = R[l * Ky + y];
+  // an even number of stages comes back to the first buffer
+  const bool swapped = stages_of(m.z) & 1;
+  transform<-1>(m.z, (Ky + 1) / 2, pitch, twz, a, b, [&](int t, int l) { return a[t * pitch + l]; },
+                [&](int t, int l, float2 v) { (swapped ? b : a)[t * pitch + l] = v; });
+  const float2* Z = swapped ? b : a;
+  float2 *free0 = swapped ? a : b, *free1 = swapped ? b : a;
+  float2* out = m.spectrum + static_cast<long long>(x) * Ky * kzh;
+  transform<-1>(m.y, kzh, kzh, twy, free1, free0,
+                [&](int y, int k) {
+                  const int p = y >> 1;
+                  return line_of_pair(Z[k * pitch + p], Z[(k ? Kz - k : 0) * pitch + p], y & 1);
+                },
+                [&](int y, int k, float2 v) { out[y * kzh + k] = v; });
+}
+
+__device__ __forceinline__ void plane_inverse(const Mesh& m, int x, float2* smem) {
+  const int Ky = m.y.n, Kz = m.z.n, kzh = m.kzh, pitch = pair_pitch(Ky), size = plane_buffer(Ky, Kz);
+  float2 *a = smem, *b = smem + size, *twz = smem + 2 * size, *twy = twz + Kz;
+  stage_twiddles(twz, m.twz, Kz);
+  stage_twiddles(twy, m.twy, Ky);
+  const float2* in = m.spectrum + static_cast<long long>(x) * Ky * kzh;
+  __syncthreads();
+  const bool swapped = stages_of(m.y) & 1;
+  transform<+1>(m.y, kzh, kzh, twy, a, b, [&](int y, int k) { return __ldcg(&in[y * kzh + k]); },
+                [&](int y, int k, float2 v) { (swapped ? b : a)[y * kzh + k] = v; });
+  const float2* Y = swapped ? b : a;
+  float2 *free0 = swapped ? a : b, *free1 = swapped ? b : a;
+  float2* R = stages_of(m.z) & 1 ? free0 : free1;
+  transform<+1>(m.z, (Ky + 1) / 2, pitch, twz, free1, free0,
+                [&](int t, int p) {
+                  return pair_of_lines(Kz, t, 2 * p + 1 < Ky, [&](int h, int k) { return Y[(2 * p + h) * kzh + k]; });
+                },
+                [&](int t, int p, float2 v) { R[t * pitch + p] = v; });
+  store_potential(m.potential + static_cast<long long>(x) * Ky * Kz, Ky, Kz, pitch, R);
+}
+
+// z and y passes of their own, for planes that do not fit shared memory: lines
+// [line0, line0 + lines) of the mesh, an even number from an even line of
+// one plane (or the rest of it); a strip of `nk` kz columns of an x-plane.
+__device__ __forceinline__ void z_forward(const Mesh& m, int line0, int lines, float2* smem) {
+  const int Kz = m.z.n, kzh = m.kzh, pitch = pair_pitch(lines);
+  float2 *a = smem, *b = smem + Kz * pitch, *tw = smem + 2 * Kz * pitch;
+  stage_twiddles(tw, m.twz, Kz);
+  load_charges(m.charge + static_cast<long long>(line0) * Kz, lines, Kz, pitch, a);
+  __syncthreads();
+  const bool swapped = stages_of(m.z) & 1;
+  transform<-1>(m.z, (lines + 1) / 2, pitch, tw, a, b, [&](int t, int l) { return a[t * pitch + l]; },
+                [&](int t, int l, float2 v) { (swapped ? b : a)[t * pitch + l] = v; });
+  const float2* Z = swapped ? b : a;
+  float2* out = m.spectrum + static_cast<long long>(line0) * kzh;
+  for (int i = threadIdx.x; i < lines * kzh; i += blockDim.x) {
+    const int y = i / kzh, k = i - y * kzh, p = y >> 1;
+    out[i] = line_of_pair(Z[k * pitch + p], Z[(k ? Kz - k : 0) * pitch + p], y & 1);
   }
 }
 
-// ------------------------------------------- x pass with the convolution ---
+__device__ __forceinline__ void z_inverse(const Mesh& m, int line0, int lines, float2* smem) {
+  const int Kz = m.z.n, kzh = m.kzh, pitch = pair_pitch(lines);
+  float2 *a = smem, *b = smem + Kz * pitch, *tw = smem + 2 * Kz * pitch;
+  stage_twiddles(tw, m.twz, Kz);
+  const float2* in = m.spectrum + static_cast<long long>(line0) * kzh;
+  __syncthreads();
+  float2* R = stages_of(m.z) & 1 ? b : a;
+  transform<+1>(m.z, (lines + 1) / 2, pitch, tw, a, b,
+                [&](int t, int p) {
+                  return pair_of_lines(Kz, t, 2 * p + 1 < lines,
+                                       [&](int h, int k) { return __ldcg(&in[(2 * p + h) * kzh + k]); });
+                },
+                [&](int t, int p, float2 v) { R[t * pitch + p] = v; });
+  store_potential(m.potential + static_cast<long long>(line0) * Kz, lines, Kz, pitch, R);
+}
+
+template <int SIGN>
+__device__ __forceinline__ void y_pass(const Mesh& m, int x, int kz0, int nk, float2* smem) {
+  const int Ky = m.y.n, kzh = m.kzh;
+  float2 *a = smem, *b = smem + nk * Ky, *tw = smem + 2 * nk * Ky;
+  stage_twiddles(tw, m.twy, Ky);
+  float2* base = m.spectrum + static_cast<long long>(x) * Ky * kzh + kz0;
+  __syncthreads();
+  transform<SIGN>(m.y, nk, nk, tw, a, b, [&](int y, int l) { return base[static_cast<long long>(y) * kzh + l]; },
+                  [&](int y, int l, float2 v) { base[static_cast<long long>(y) * kzh + l] = v; });
+}
+
+// The x pass: `nk` lines at (y, kz0 ..), forward, each element through
+// `factor(mx, l, v)`, inverse.  The inverse runs the radices backwards, so its
+// first butterflies take exactly the elements the forward transform's last
+// ones give: those two stages and the factor happen in registers, and a
+// two-stage axis makes three passes with two barriers in all, loading and
+// storing global memory directly.
+template <class Factor>
+__device__ __forceinline__ void x_pass(const Mesh& m, int y, int kz0, int nk, float2* smem, Factor factor) {
+  const int Kx = m.x.n, count = stages_of(m.x);
+  float2 *a = smem, *b = smem + nk * Kx, *tw = smem + 2 * nk * Kx;
+  stage_twiddles(tw, m.twx, Kx);
+  const long long stride = static_cast<long long>(m.y.n) * m.kzh;
+  float2* base = m.spectrum + static_cast<long long>(y) * m.kzh + kz0;
+  const unsigned nk_magic = magic_for(unsigned(nk));
+  __syncthreads();
+  auto load = [&](int t, int l) { return __ldcg(&base[t * stride + l]); };
+  auto save = [&](int t, int l, float2 v) { base[t * stride + l] = v; };
+  auto from = [&](const float2* p) { return [p, nk](int t, int l) { return p[t * nk + l]; }; };
+  auto to = [&](float2* p) { return [p, nk](int t, int l, float2 v) { p[t * nk + l] = v; }; };
+  auto swap = [&]() {
+    float2* t = a;
+    a = b;
+    b = t;
+  };
+  // forward, up to the last stage: from global memory into b, then a to b
+  int ns = 1;
+  for (int st = 0; st < count - 1; ++st) {
+    const int r = radix_at(m.x, st);
+    if (st == 0) {
+#define MDB_STAGE(R) stage_of<R, -1>(Kx, 1, nk, nk_magic, tw, load, to(b))
+      MDB_RADIX_SWITCH(r, MDB_STAGE)
+#undef MDB_STAGE
+    } else {
+#define MDB_STAGE(R) stage_of<R, -1>(Kx, ns, nk, nk_magic, tw, from(a), to(b))
+      MDB_RADIX_SWITCH(r, MDB_STAGE)
+#undef MDB_STAGE
+    }
+    __syncthreads();
+    swap();
+    ns *= r;
+  }
+  // the forward transform's last butterflies, the factor, the inverse's first
+  const int turn = radix_at(m.x, count - 1);
+  auto middle = [&](auto radix, auto in, auto out) {
+    constexpr int R = decltype(radix)::value;
+    const int bf = Kx / R;
+    for (int idx = threadIdx.x; idx < nk * bf; idx += blockDim.x) {
+      const int k = int(quotient(unsigned(idx), nk_magic)), l = idx - k * nk;
+      float2 v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = in(k + q * bf, l);
+      if (bf > 1) {
+#pragma unroll
+        for (int q = 1; q < R; ++q) v[q] = cmul(v[q], tw[k * q]);
+      }
+      dft<R, -1>(v);
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = factor(k + q * bf, l, v[q]);
+      dft<R, +1>(v);
+#pragma unroll
+      for (int q = 0; q < R; ++q) out(k * R + q, l, v[q]);
+    }
+  };
+  if (count == 1) {
+#define MDB_TURN(R) middle(std::integral_constant<int, R>{}, load, save)
+    MDB_RADIX_SWITCH(turn, MDB_TURN)
+#undef MDB_TURN
+    __syncthreads();
+    return;
+  }
+#define MDB_TURN(R) middle(std::integral_constant<int, R>{}, from(a), to(b))
+  MDB_RADIX_SWITCH(turn, MDB_TURN)
+#undef MDB_TURN
+  __syncthreads();
+  ns = turn;
+  for (int st = count - 2; st >= 0; --st) {
+    swap();
+    const int r = radix_at(m.x, st);
+    if (st == 0) {
+#define MDB_STAGE(R) stage_of<R, +1>(Kx, ns, nk, nk_magic, tw, from(a), save)
+      MDB_RADIX_SWITCH(r, MDB_STAGE)
+#undef MDB_STAGE
+    } else {
+#define MDB_STAGE(R) stage_of<R, +1>(Kx, ns, nk, nk_magic, tw, from(a), to(b))
+      MDB_RADIX_SWITCH(r, MDB_STAGE)
+#undef MDB_STAGE
+    }
+    __syncthreads();
+    ns *= r;
+  }
+}
+
+// ------------------------------------------------ the Ewald convolution ---
 // The Ewald influence function (pme-convolve.wgsl:34; pme.ts:160-209) at
 // mesh index (mx, my, kz) of the half spectrum, mb the signed y index; the
 // wave vector and its square come back for the virial.  0 at the origin.
@@ -528,8 +816,8 @@ __device__ __forceinline__ float influence(const SysDev& S, const float* modx, c
 }
 
 // The influence function of every x-pass work item of system `s` (all
-// systems: s < 0), in the order the x pass visits its elements.  Run after
-// every change of a box.
+// systems: s < 0), element (mx, l) at mx * lines + l as the x pass reads it.
+// Run after every change of a box.
 __global__ void __launch_bounds__(kThreads) k_influence(Dev d, int s) {
   const FftWork w = d.fft_x[blockIdx.x];
   if (s >= 0 && w.sys != s) return;
@@ -541,346 +829,284 @@ __global__ void __launch_bounds__(kThreads) k_influence(Dev d, int s) {
   const int my = w.a, mb = my <= Ky / 2 ? my : my - Ky;
   float* table = d.influence + static_cast<long long>(blockIdx.x) * d.influence_stride;
   for (int i = threadIdx.x; i < w.n * Kx; i += blockDim.x) {
-    const int l = i / Kx, mx = i - l * Kx;
+    const int mx = i / w.n, l = i - mx * w.n;
     float kx, ky, kzv, k2;
     table[i] = influence(S, modx, mody, modz, Kx, mx, mb, my, w.b + l, kx, ky, kzv, k2);
   }
 }
 
+constexpr int kXThreads = 128;  // eight lines of 50 points are 80 or 40 butterflies a stage
+
+// The block's sums of `val`, in a fixed order in FP64 (deterministic), to out(c, total).
+template <int N, class Out>
+__device__ __forceinline__ void block_sums(double* val, Out out) {
+  __shared__ double partial[N][kXThreads / 32];
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) val[c] += __shfl_xor_sync(0xffffffffu, val[c], o);
+    if ((threadIdx.x & 31) == 0) partial[c][threadIdx.x >> 5] = val[c];
+  }
+  __syncthreads();
+  if (threadIdx.x < N) {
+    double total = 0.0;
+    for (int k = 0; k < int(blockDim.x >> 5); ++k) total += partial[threadIdx.x][k];
+    out(int(threadIdx.x), total);
+  }
+}
+
 template <bool ENERGY>
-__global__ void __launch_bounds__(kThreads) k_fft_x_convolve(Dev d) {
+__global__ void __launch_bounds__(kXThreads) k_fft_x_convolve(Dev d) {
   wait_for_predecessor();
   extern __shared__ float2 smem[];
-  __shared__ double partial[7][kThreads / 32];
   const FftWork w = d.fft_x[blockIdx.x];
   if (!sys_active(d, w.sys)) return;  // the whole block: before any barrier
   const SysDev& S = d.sys[w.sys];
-  const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2], kzh = S.kzh;
-  float2* A = smem;
-  float2* B = smem + w.n * Kx;
-  float2* twx = smem + 2 * kFftTile * Kx;  // the twiddles, after the two tiles of lines
-  stage_twiddles(twx, d.twiddles + S.tw_off[0], Kx);
-  const long long stride = static_cast<long long>(Ky) * kzh;
-  float2* base = d.cgrid + S.cgrid_off + static_cast<long long>(w.a) * kzh + w.b;
-  const unsigned n_magic = magic_for(unsigned(w.n)), kx_magic = magic_for(unsigned(Kx));
-  for (int i0 = threadIdx.x; i0 < w.n * Kx; i0 += 2 * blockDim.x) {
-    float2 v[2];
-    int x[2], l[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int i = i0 + u * blockDim.x;
-      x[u] = int(quotient(unsigned(i), n_magic));
-      l[u] = i - x[u] * w.n;
-      v[u] = i < w.n * Kx ? __ldcg(&base[x[u] * stride + l[u]]) : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-      if (i0 + u * int(blockDim.x) < w.n * Kx) A[l[u] * Kx + x[u]] = v[u];
-  }
-  __syncthreads();
-  float2* R = fft_lines(A, B, Kx, w.n, S.radices[0], S.nradix[0], twx, -1);
-  float2* other = R == A ? B : A;
-  // Convolution (pme-convolve.wgsl:34; pme.ts:160-209) on the half spectrum.
-  double energy = 0.0;
-  double vir[6] = {0, 0, 0, 0, 0, 0};  // xx yy zz xy xz yz
-  const int my = w.a;
-  const int mb = my <= Ky / 2 ? my : my - Ky;
-  const float* modx = d.moduli + S.mod_off;
-  const float* mody = modx + Kx;
-  const float* modz = mody + Ky;
+  const Mesh m = mesh_of(d, S);
+  const int my = w.a, nk = w.n;
   // the force variant (every MD step) reads the influence function from the
   // table k_influence fills at every box change; the energy variant needs the
   // wave vectors for the virial and evaluates it here, the same function
   const float* table = d.influence + static_cast<long long>(blockIdx.x) * d.influence_stride;
-  for (int i = threadIdx.x; i < w.n * Kx; i += blockDim.x) {
-    const int l = int(quotient(unsigned(i), kx_magic)), mx = i - l * Kx;
-    const int kz = w.b + l;
-    float2 v = R[i];
-    float factor, kx = 0.f, ky = 0.f, kzv = 0.f, k2 = 1.f;
-    if (ENERGY) factor = influence(S, modx, mody, modz, Kx, mx, mb, my, kz, kx, ky, kzv, k2);
-    else factor = __ldg(&table[i]);
+  double sums[7] = {0, 0, 0, 0, 0, 0, 0};  // energy, virial xx yy zz xy xz yz
+  x_pass(m, my, w.b, nk, smem, [&](int mx, int l, float2 v) {
+    float f;
     if (ENERGY) {
+      const int Kx = m.x.n, Ky = m.y.n, Kz = m.z.n, kz = w.b + l, mb = my <= Ky / 2 ? my : my - Ky;
+      const float* modx = d.moduli + S.mod_off;
+      float kx = 0.f, ky = 0.f, kzv = 0.f, k2 = 1.f;
+      f = influence(S, modx, modx + Kx, modx + Kx + Ky, Kx, mx, mb, my, kz, kx, ky, kzv, k2);
       const double weight = (kz == 0 || (2 * kz == Kz)) ? 1.0 : 2.0;
       const double ek =
-          weight * static_cast<double>(factor) * (static_cast<double>(v.x) * v.x + static_cast<double>(v.y) * v.y);
-      energy += ek;
+          weight * static_cast<double>(f) * (static_cast<double>(v.x) * v.x + static_cast<double>(v.y) * v.y);
       // -dE_k/d eps_ab = E_k (delta_ab - 2 k_a k_b (1/k^2 + 1/(4 alpha^2)))
       const double c = 2.0 * (1.0 / static_cast<double>(k2) - static_cast<double>(S.exp_scale));
       const double ka = kx, kb = ky, kc = kzv;
-      vir[0] += ek * (1.0 - c * ka * ka);
-      vir[1] += ek * (1.0 - c * kb * kb);
-      vir[2] += ek * (1.0 - c * kc * kc);
-      vir[3] -= ek * c * ka * kb;
-      vir[4] -= ek * c * ka * kc;
-      vir[5] -= ek * c * kb * kc;
+      sums[0] += ek;
+      sums[1] += ek * (1.0 - c * ka * ka);
+      sums[2] += ek * (1.0 - c * kb * kb);
+      sums[3] += ek * (1.0 - c * kc * kc);
+      sums[4] -= ek * c * ka * kb;
+      sums[5] -= ek * c * ka * kc;
+      sums[6] -= ek * c * kb * kc;
+    } else {
+      f = __ldg(&table[mx * nk + l]);
     }
-    v.x *= 2.f * factor;
-    v.y *= 2.f * factor;
-    R[i] = v;
-  }
-  __syncthreads();
-  const float2* Q = fft_lines(R, other, Kx, w.n, S.radices[0], S.nradix[0], twx, +1);
-  for (int i = threadIdx.x; i < w.n * Kx; i += blockDim.x) {
-    const int x = int(quotient(unsigned(i), n_magic)), l = i - x * w.n;
-    base[x * stride + l] = Q[l * Kx + x];
-  }
+    const float g = 2.f * f;
+    return make_float2(__fmul_rn(v.x, g), __fmul_rn(v.y, g));
+  });
   if (ENERGY) {
-    // fixed-order block reduction in FP64: deterministic
-    double val[7] = {energy, vir[0], vir[1], vir[2], vir[3], vir[4], vir[5]};
-#pragma unroll
-    for (int c = 0; c < 7; ++c) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) val[c] += __shfl_xor_sync(0xffffffffu, val[c], o);
-      if ((threadIdx.x & 31) == 0) partial[c][threadIdx.x >> 5] = val[c];
-    }
-    __syncthreads();
-    if (threadIdx.x < 7) {
-      double total = 0.0;
-      for (int k = 0; k < (blockDim.x >> 5); ++k) total += partial[threadIdx.x][k];
-      if (threadIdx.x == 0) d.mesh_partial[blockIdx.x] = total;
-      else d.mesh_virial[blockIdx.x * 6 + threadIdx.x - 1] = total;
-    }
+    block_sums<7>(sums, [&](int c, double total) {
+      if (c == 0) d.mesh_partial[blockIdx.x] = total;
+      else d.mesh_virial[blockIdx.x * 6 + c - 1] = total;
+    });
   }
 }
 
-// ------------------------------------------------- whole x-plane passes ---
-// With the plane in shared memory one CTA does both the z and the y
-// transforms of an x-plane (Ky x Kz grid points; 2 x 16 Ky Kz bytes), so a
-// forward or inverse transform is three launches instead of five and the
-// launches that remain have a plane of work each.
-constexpr int kPlaneThreads = 512;
+constexpr int kPlaneThreads = 256;
 
 __global__ void __launch_bounds__(kPlaneThreads) k_fft_zy_forward(Dev d) {
   wait_for_predecessor();
   extern __shared__ float2 smem[];
   const FftWork w = d.fft_p[blockIdx.x];
   if (!sys_active(d, w.sys)) return;  // the whole block: before any barrier
-  const SysDev& S = d.sys[w.sys];
-  const int Ky = S.grid[1], Kz = S.grid[2], kzh = S.kzh;
-  const unsigned ky_magic = magic_for(unsigned(Ky)), kzh_magic = magic_for(unsigned(kzh)),
-                 rest_magic = magic_for(unsigned(Kz - kzh));
-  float2* A = smem;
-  float2* B = smem + Ky * Kz;
-  float2* twz = smem + 2 * Ky * Kz;  // the twiddles, after the two planes
-  float2* twy = twz + Kz;
-  stage_twiddles(twz, d.twiddles + S.tw_off[2], Kz);
-  stage_twiddles(twy, d.twiddles + S.tw_off[1], Ky);
-  unsigned long long* grid = d.qgrid + S.grid_off + static_cast<long long>(w.a) * Ky * Kz;
-  // four loads in flight per thread before any is used
-  for (int i0 = threadIdx.x; i0 < Ky * Kz; i0 += 4 * blockDim.x) {
-    long long v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u * blockDim.x;
-      v[u] = i < Ky * Kz ? static_cast<long long>(__ldcg(&grid[i])) : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u * blockDim.x;
-      if (i < Ky * Kz) {
-        A[i] = make_float2(from_fixed(v[u]), 0.f);
-        grid[i] = 0ull;  // consumer clears: the next spread starts from zero
-      }
-    }
-  }
-  __syncthreads();
-  float2* R = fft_lines(A, B, Kz, Ky, S.radices[2], S.nradix[2], twz, -1);
-  float2* T = R == A ? B : A;
-  // the half spectrum's kz columns become y-lines
-  for (int i = threadIdx.x; i < kzh * Ky; i += blockDim.x) {
-    const int k = int(quotient(unsigned(i), ky_magic)), y = i - k * Ky;
-    T[k * Ky + y] = R[y * Kz + k];
-  }
-  __syncthreads();
-  const float2* Y = fft_lines(T, R, Ky, kzh, S.radices[1], S.nradix[1], twy, -1);
-  float2* out = d.cgrid + S.cgrid_off + static_cast<long long>(w.a) * Ky * kzh;
-  for (int i = threadIdx.x; i < Ky * kzh; i += blockDim.x) {
-    const int y = int(quotient(unsigned(i), kzh_magic)), k = i - y * kzh;
-    out[i] = Y[k * Ky + y];
-  }
+  plane_forward(mesh_of(d, d.sys[w.sys]), w.a, smem);
 }
 
 __global__ void __launch_bounds__(kPlaneThreads) k_fft_yz_inverse(Dev d) {
   wait_for_predecessor();
   extern __shared__ float2 smem[];
   const FftWork w = d.fft_p[blockIdx.x];
-  if (!sys_active(d, w.sys)) return;  // the whole block: before any barrier
-  const SysDev& S = d.sys[w.sys];
-  const int Ky = S.grid[1], Kz = S.grid[2], kzh = S.kzh;
-  const unsigned ky_magic = magic_for(unsigned(Ky)), kzh_magic = magic_for(unsigned(kzh)),
-                 rest_magic = magic_for(unsigned(Kz - kzh));
-  float2* A = smem;
-  float2* B = smem + Ky * Kz;
-  float2* twz = smem + 2 * Ky * Kz;  // the twiddles, after the two planes
-  float2* twy = twz + Kz;
-  stage_twiddles(twz, d.twiddles + S.tw_off[2], Kz);
-  stage_twiddles(twy, d.twiddles + S.tw_off[1], Ky);
-  const float2* in = d.cgrid + S.cgrid_off + static_cast<long long>(w.a) * Ky * kzh;
-  for (int i0 = threadIdx.x; i0 < Ky * kzh; i0 += 4 * blockDim.x) {
-    float2 v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u * blockDim.x;
-      v[u] = i < Ky * kzh ? __ldcg(&in[i]) : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = i0 + u * blockDim.x;
-      if (i < Ky * kzh) {
-        const int y = int(quotient(unsigned(i), kzh_magic)), k = i - y * kzh;
-        A[k * Ky + y] = v[u];
-      }
-    }
-  }
-  __syncthreads();
-  float2* Y = fft_lines(A, B, Ky, kzh, S.radices[1], S.nradix[1], twy, +1);
-  float2* Z = Y == A ? B : A;
-  for (int i = threadIdx.x; i < Ky * kzh; i += blockDim.x) {
-    const int y = int(quotient(unsigned(i), kzh_magic)), k = i - y * kzh;
-    Z[y * Kz + k] = Y[k * Ky + y];
-  }
-  __syncthreads();
-  // the rest of each z-line from Hermitian symmetry (the result is real)
-  for (int i = threadIdx.x; i < Ky * (Kz - kzh); i += blockDim.x) {
-    const int y = int(quotient(unsigned(i), rest_magic)), k = kzh + (i - y * (Kz - kzh));
-    const float2 c = Z[y * Kz + (Kz - k)];
-    Z[y * Kz + k] = make_float2(c.x, -c.y);
-  }
-  __syncthreads();
-  const float2* R = fft_lines(Z, Y, Kz, Ky, S.radices[2], S.nradix[2], twz, +1);
-  float* out = d.phi + S.grid_off + static_cast<long long>(w.a) * Ky * Kz;
-  for (int i = threadIdx.x; i < Ky * Kz; i += blockDim.x) out[i] = R[i].x;
+  if (!sys_active(d, w.sys)) return;
+  plane_inverse(mesh_of(d, d.sys[w.sys]), w.a, smem);
 }
 
-// ---------------------------------------------------------- z inverse ----
-// complex half spectrum -> real potential grid along z.
+__global__ void __launch_bounds__(kThreads) k_fft_z_forward(Dev d) {
+  wait_for_predecessor();
+  extern __shared__ float2 smem[];
+  const FftWork w = d.fft_z[blockIdx.x];
+  if (!sys_active(d, w.sys)) return;
+  z_forward(mesh_of(d, d.sys[w.sys]), w.a, w.n, smem);
+}
+
+template <int SIGN>
+__global__ void __launch_bounds__(kThreads) k_fft_y(Dev d) {
+  wait_for_predecessor();
+  extern __shared__ float2 smem[];
+  const FftWork w = d.fft_y[blockIdx.x];
+  if (!sys_active(d, w.sys)) return;
+  y_pass<SIGN>(mesh_of(d, d.sys[w.sys]), w.a, w.b, w.n, smem);
+}
+
 __global__ void __launch_bounds__(kThreads) k_fft_z_inverse(Dev d) {
   wait_for_predecessor();
   extern __shared__ float2 smem[];
   const FftWork w = d.fft_z[blockIdx.x];
-  if (!sys_active(d, w.sys)) return;  // the whole block: before any barrier
-  const SysDev& S = d.sys[w.sys];
-  const int Kz = S.grid[2], kzh = S.kzh;
-  float2* A = smem;
-  float2* B = smem + w.n * Kz;
-  const float2* in = d.cgrid + S.cgrid_off + static_cast<long long>(w.a) * kzh;
-  for (int i = threadIdx.x; i < w.n * kzh; i += blockDim.x) {
-    const int line = i / kzh, k = i - line * kzh;
-    A[line * Kz + k] = in[i];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < w.n * (Kz - kzh); i += blockDim.x) {
-    const int line = i / (Kz - kzh), k = kzh + (i - line * (Kz - kzh));
-    const float2 c = A[line * Kz + (Kz - k)];
-    A[line * Kz + k] = make_float2(c.x, -c.y);
-  }
-  __syncthreads();
-  const float2* R = fft_lines(A, B, Kz, w.n, S.radices[2], S.nradix[2], d.twiddles + S.tw_off[2], +1);
-  float* out = d.phi + S.grid_off + static_cast<long long>(w.a) * Kz;
-  for (int i = threadIdx.x; i < w.n * Kz; i += blockDim.x) out[i] = R[i].x;
+  if (!sys_active(d, w.sys)) return;
+  z_inverse(mesh_of(d, d.sys[w.sys]), w.a, w.n, smem);
 }
 
 // ---------------------------------------------------------------- gather --
-__global__ void __launch_bounds__(kThreads) k_gather(Dev d) {
-  wait_for_predecessor();
-  for (int gs = blockIdx.x * blockDim.x + threadIdx.x; gs < d.n_slots; gs += gridDim.x * blockDim.x) {
-    const int a = d.order[gs];
-    if (a < 0) continue;
-    const float q = d.prm[gs].w;
-    if (q == 0.f || !sys_active(d, d.slot_sys[gs])) continue;
-    const SysDev& S = d.sys[d.slot_sys[gs]];
-    Spline sp;
-    spline_for(S, d.px[a], d.py[a], d.pz[a], sp, true);
-    const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2];
-    const float* grid = d.phi + S.grid_off;
-    float ga = 0.f, gb = 0.f, gc = 0.f;
-    for (int ix = 0; ix < kPmeOrder; ++ix) {
-      int gx = sp.base[0] + ix;
-      if (gx >= Kx) gx -= Kx;
-      for (int iy = 0; iy < kPmeOrder; ++iy) {
-        int gy = sp.base[1] + iy;
-        if (gy >= Ky) gy -= Ky;
-        const float* row = grid + (static_cast<long long>(gx) * Ky + gy) * Kz;
-        const float wxy = sp.th[0][ix] * sp.th[1][iy];
-        const float dxy = sp.dth[0][ix] * sp.th[1][iy];
-        const float xdy = sp.th[0][ix] * sp.dth[1][iy];
+// A block of 32 atoms: their splines first, a warp to an axis; then a warp to
+// each of the five x planes of the stencil, lanes atoms, with the plane's 25
+// loads in flight together; then the five partial sums in a fixed order.  A
+// thread per atom walking its 125 points left the kernel waiting on loads with
+// few warps to hide them (12k-atom peptide 6.5 -> 5.2 us, 100k atoms 21.6 ->
+// 18.9 us).
+constexpr int kGatherAtoms = 32;
+constexpr int kGatherThreads = 32 * kPmeOrder;
+
+struct GatherTable {
+  int base[3][kGatherAtoms];
+  float th[3][5][kGatherAtoms], dth[3][5][kGatherAtoms];
+  float part[kPmeOrder][3][kGatherAtoms];
+};
+
+// `live`: whether this lane's atom (the same in every warp) has a charge; x,
+// y, z its position.  Returns true in warp 0 for the live atoms, with the
+// gradient of the potential along the mesh axes.
+__device__ __forceinline__ bool gather_block(GatherTable& t, bool live, const SysDev& S, const float* grid, long long x,
+                                             long long y, long long z, float& ga, float& gb, float& gc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (live && warp < 3) {
+    float th[5], dth[5];
+    t.base[warp][lane] = spline_axis(S, warp, x, y, z, th, dth);
 #pragma unroll
-        for (int iz = 0; iz < kPmeOrder; ++iz) {
-          int gz = sp.base[2] + iz;
-          if (gz >= Kz) gz -= Kz;
-          const float p = row[gz];
-          ga = fmaf(p * dxy, sp.th[2][iz], ga);
-          gb = fmaf(p * xdy, sp.th[2][iz], gb);
-          gc = fmaf(p * wxy, sp.dth[2][iz], gc);
-        }
-      }
+    for (int i = 0; i < kPmeOrder; ++i) {
+      t.th[warp][i][lane] = th[i];
+      t.dth[warp][i][lane] = dth[i];
     }
-    // F_v = -q sum_u (dE/du_u) K_u M[v][u]  (pme.ts:252-259)
-    const float* U = S.umat_f;
-    const float fx = -q * (ga * U[0] + gb * U[1] + gc * U[2]);
-    const float fy = -q * (ga * U[3] + gb * U[4] + gc * U[5]);
-    const float fz = -q * (ga * U[6] + gb * U[7] + gc * U[8]);
-    add_fixed(&d.fx[gs], fx);
-    add_fixed(&d.fy[gs], fy);
-    add_fixed(&d.fz[gs], fz);
   }
+  __syncthreads();
+  ga = gb = gc = 0.f;
+  if (live) {
+    const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2];
+    int gx = t.base[0][lane] + warp;
+    if (gx >= Kx) gx -= Kx;
+    const int by = t.base[1][lane], bz = t.base[2][lane];
+    int gz[5];
+#pragma unroll
+    for (int iz = 0; iz < kPmeOrder; ++iz) {
+      gz[iz] = bz + iz;
+      if (gz[iz] >= Kz) gz[iz] -= Kz;
+    }
+    float p[5][5];
+#pragma unroll
+    for (int iy = 0; iy < kPmeOrder; ++iy) {
+      int gy = by + iy;
+      if (gy >= Ky) gy -= Ky;
+      const float* row = grid + (static_cast<long long>(gx) * Ky + gy) * Kz;
+#pragma unroll
+      for (int iz = 0; iz < kPmeOrder; ++iz) p[iy][iz] = row[gz[iz]];
+    }
+    const float wx = t.th[0][warp][lane], dx = t.dth[0][warp][lane];
+#pragma unroll
+    for (int iy = 0; iy < kPmeOrder; ++iy) {
+      float along = 0.f, slope = 0.f;
+#pragma unroll
+      for (int iz = 0; iz < kPmeOrder; ++iz) {
+        along = fmaf(p[iy][iz], t.th[2][iz][lane], along);
+        slope = fmaf(p[iy][iz], t.dth[2][iz][lane], slope);
+      }
+      const float wy = t.th[1][iy][lane], dy = t.dth[1][iy][lane];
+      ga = fmaf(along, __fmul_rn(dx, wy), ga);
+      gb = fmaf(along, __fmul_rn(wx, dy), gb);
+      gc = fmaf(slope, __fmul_rn(wx, wy), gc);
+    }
+    if (warp > 0) {
+      t.part[warp][0][lane] = ga;
+      t.part[warp][1][lane] = gb;
+      t.part[warp][2][lane] = gc;
+    }
+  }
+  __syncthreads();
+  if (!live || warp > 0) return false;
+#pragma unroll
+  for (int w = 1; w < kPmeOrder; ++w) {
+    ga = __fadd_rn(ga, t.part[w][0][lane]);
+    gb = __fadd_rn(gb, t.part[w][1][lane]);
+    gc = __fadd_rn(gc, t.part[w][2][lane]);
+  }
+  return true;
 }
 
-int grid_blocks(int n) {
-  int b = (n + kThreads - 1) / kThreads;
-  if (b > 148 * 16) b = 148 * 16;
-  return b < 1 ? 1 : b;
+// F_v = -q sum_u (dE/du_u) K_u M[v][u]  (pme.ts:252-259)
+__device__ __forceinline__ float3 mesh_force(const SysDev& S, float q, float ga, float gb, float gc) {
+  const float* U = S.umat_f;
+  return make_float3(__fmul_rn(-q, fmaf(gc, U[2], fmaf(gb, U[1], __fmul_rn(ga, U[0])))),
+                     __fmul_rn(-q, fmaf(gc, U[5], fmaf(gb, U[4], __fmul_rn(ga, U[3])))),
+                     __fmul_rn(-q, fmaf(gc, U[8], fmaf(gb, U[7], __fmul_rn(ga, U[6])))));
+}
+
+__global__ void __launch_bounds__(kGatherThreads) k_gather(Dev d) {
+  wait_for_predecessor();
+  __shared__ GatherTable table;
+  const int gs = blockIdx.x * kGatherAtoms + (threadIdx.x & 31);  // n_slots is a multiple of 32
+  const int a = d.order[gs], s = d.slot_sys[gs];
+  const float q = a >= 0 ? d.prm[gs].w : 0.f;
+  const bool live = q != 0.f && sys_active(d, s);
+  const SysDev& S = d.sys[s];
+  float ga, gb, gc;
+  if (!gather_block(table, live, S, d.phi + S.grid_off, live ? d.px[a] : 0, live ? d.py[a] : 0, live ? d.pz[a] : 0, ga,
+                    gb, gc))
+    return;
+  const float3 f = mesh_force(S, q, ga, gb, gc);
+  add_fixed(&d.fx[gs], f.x);
+  add_fixed(&d.fy[gs], f.y);
+  add_fixed(&d.fz[gs], f.z);
 }
 
 }  // namespace
 
-// Shared-memory bytes for the largest work item of each pass, set by the host.
-struct PmeSmem { int z, y, x, p; };
-static PmeSmem g_smem{0, 0, 0, 0};
-void set_pme_smem(int z, int y, int x, int plane) {
-  g_smem = {z, y, x, plane};
-  if (plane > 0) {
-    cudaFuncSetAttribute(k_fft_zy_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, plane);
-    cudaFuncSetAttribute(k_fft_yz_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, plane);
-  }
-  cudaFuncSetAttribute(k_fft_z_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, z);
-  cudaFuncSetAttribute(k_fft_z_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, z);
-  cudaFuncSetAttribute(k_fft_y, cudaFuncAttributeMaxDynamicSharedMemorySize, y);
-  cudaFuncSetAttribute(k_fft_x_convolve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, x);
-  cudaFuncSetAttribute(k_fft_x_convolve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, x);
-}
+// Shared-memory bytes of one work item of each transform pass.
+int plane_smem(int Ky, int Kz) { return (2 * plane_buffer(Ky, Kz) + Ky + Kz) * int(sizeof(float2)); }
+int z_smem(int lines, int Kz) { return (2 * pair_pitch(lines) + 1) * Kz * int(sizeof(float2)); }
+int strip_smem(int lines, int n) { return (2 * lines + 1) * n * int(sizeof(float2)); }
 
-// Engines with at least one block of 128 slots per SM spread by slot: the
-// 27k-atom octahedron (205 blocks) spreads in 25.5 us by slot against 27.5 us
-// by atom, the 12k-atom peptide (96 blocks) in 15.5 us against 13.7 us.
-bool spread_by_slot(int n_slots) { return (n_slots + kPatchSlots - 1) / kPatchSlots >= 148; }
+// Every transform kernel may use up to `bytes` of dynamic shared memory (the
+// launches ask for their own engine's size): called once per engine with the
+// device's limit, so engines of different meshes do not disturb one another.
+int allow_pme_smem(int bytes) {
+  cudaError_t err = cudaSuccess;
+  auto allow = [&](auto kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) err = e;
+  };
+  allow(k_fft_zy_forward);
+  allow(k_fft_yz_inverse);
+  allow(k_fft_z_forward);
+  allow(k_fft_z_inverse);
+  allow(k_fft_x_convolve<true>);
+  allow(k_fft_x_convolve<false>);
+  allow(k_fft_y<-1>);
+  allow(k_fft_y<+1>);
+  return err == cudaSuccess ? 0 : 1;
+}
 
 void launch_pme_spread(const Dev& d, cudaStream_t st) {
   if (d.n_fft_z == 0) return;
-  if (d.spread_sorted) {
-    launch_chained(k_spread_sorted, (d.n_slots + kPatchSlots - 1) / kPatchSlots, kThreads, 0, st, d);
-    return;
-  }
-  // about one block per two SMs, up to kSplineAtoms atoms each: small systems
-  // get short blocks (latency), large ones full ones (fewer SMs taken from the
-  // pair kernel running beside)
-  const int per = std::max(16, std::min(kSplineAtoms, (d.n_atoms + 73) / 74));
-  launch_chained(k_spread, std::max(1, std::min((d.n_atoms + per - 1) / per, 148 * 8)), kThreads, 0, st, d, per);
+  // the most slots per block that still give every SM two blocks: compact
+  // patches share more points, short blocks have short chains
+  const int n = d.n_slots;
+  auto blocks = [n](int p) { return (n + p - 1) / p; };
+  if (blocks(128) >= 2 * 148) launch_chained(k_spread<128>, blocks(128), kThreads, 0, st, d);
+  else if (blocks(64) >= 2 * 148) launch_chained(k_spread<64>, blocks(64), kThreads, 0, st, d);
+  else launch_chained(k_spread<32>, blocks(32), kThreads, 0, st, d);
 }
 
 void launch_pme_fft(const Dev& d, bool energy, cudaStream_t st) {
   if (d.n_fft_z == 0) return;
-  if (d.fft_planes) launch_chained(k_fft_zy_forward, d.n_fft_p, kPlaneThreads, g_smem.p, st, d);
+  if (d.fft_planes) launch_chained(k_fft_zy_forward, d.n_fft_p, kPlaneThreads, d.smem_p, st, d);
   else {
-    launch_chained(k_fft_z_forward, d.n_fft_z, kThreads, g_smem.z, st, d);
-    launch_chained(k_fft_y, d.n_fft_y, kThreads, g_smem.y, st, d, -1);
+    launch_chained(k_fft_z_forward, d.n_fft_z, kThreads, d.smem_z, st, d);
+    launch_chained(k_fft_y<-1>, d.n_fft_y, kThreads, d.smem_y, st, d);
   }
-  if (energy) launch_chained(k_fft_x_convolve<true>, d.n_fft_x, kThreads, g_smem.x, st, d);
-  else launch_chained(k_fft_x_convolve<false>, d.n_fft_x, kThreads, g_smem.x, st, d);
-  if (d.fft_planes) launch_chained(k_fft_yz_inverse, d.n_fft_p, kPlaneThreads, g_smem.p, st, d);
+  if (energy) launch_chained(k_fft_x_convolve<true>, d.n_fft_x, kXThreads, d.smem_x, st, d);
+  else launch_chained(k_fft_x_convolve<false>, d.n_fft_x, kXThreads, d.smem_x, st, d);
+  if (d.fft_planes) launch_chained(k_fft_yz_inverse, d.n_fft_p, kPlaneThreads, d.smem_p, st, d);
   else {
-    launch_chained(k_fft_y, d.n_fft_y, kThreads, g_smem.y, st, d, +1);
-    launch_chained(k_fft_z_inverse, d.n_fft_z, kThreads, g_smem.z, st, d);
+    launch_chained(k_fft_y<+1>, d.n_fft_y, kThreads, d.smem_y, st, d);
+    launch_chained(k_fft_z_inverse, d.n_fft_z, kThreads, d.smem_z, st, d);
   }
 }
 
@@ -891,8 +1117,7 @@ void launch_influence(const Dev& d, int s, cudaStream_t st) {
 
 void launch_pme_gather(const Dev& d, cudaStream_t st) {
   if (d.n_fft_z == 0) return;
-  // a thread per slot; blocks of 64 so that even 10k atoms spread over every SM
-  launch_chained(k_gather, std::max(1, std::min((d.n_slots + 63) / 64, 148 * 16)), 64, 0, st, d);
+  launch_chained(k_gather, d.n_slots / kGatherAtoms, kGatherThreads, 0, st, d);
 }
 
 void launch_pme(const Dev& d, bool energy, cudaStream_t st) {
@@ -926,7 +1151,10 @@ namespace {
 
 constexpr long long kNoAllocMaxMeshPoints = 64ll * 64 * 64;
 constexpr int kNoAllocMaxAxis = 128;
-constexpr int kNoAllocMaxPartials = kNoAllocMaxAxis * ((kNoAllocMaxAxis / 2 + 1 + 15) / 16);
+// planes up to this size are transformed whole: what a block may use without
+// asking for more (64 x 64 needs 35 KB)
+constexpr int kNoAllocPlaneSmem = 48 * 1024;
+constexpr int kNoAllocMaxPartials = kNoAllocMaxAxis * ((kNoAllocMaxAxis / 2 + 1 + kFftTile - 1) / kFftTile);
 
 // Byte offsets of the pieces inside the scratch array.
 constexpr size_t kNaGrid = 0;                                           // int64 x K
@@ -948,236 +1176,186 @@ struct NaPtrs {
   double* partials;
 };
 
-// Moduli |b(m)|^2 of the order-5 spline (bspline.ts:102) and the twiddles
-// exp(-2 pi i j / K) of each axis, computed on the device in FP64; and the
-// charge grid cleared, because the array keeps the previous call's contents.
-__global__ void k_na_setup(SysDev S, NaPtrs p) {
+// Twiddles exp(-2 pi i j / K) and moduli |b(m)|^2 of the order-5 spline
+// (bspline.ts:102) of each axis, computed on the device in FP64 by the first
+// three blocks, one sine and cosine a point; and the charge grid cleared,
+// because the array keeps the previous call's contents.
+__global__ void __launch_bounds__(kThreads) k_na_setup(SysDev S, NaPtrs p) {
   const long long K = static_cast<long long>(S.grid[0]) * S.grid[1] * S.grid[2];
   for (long long i = blockIdx.x * blockDim.x + threadIdx.x; i < K; i += gridDim.x * blockDim.x) p.grid[i] = 0ull;
-  if (blockIdx.x != 0) return;
-  const double knots[4] = {1.0 / 24, 11.0 / 24, 11.0 / 24, 1.0 / 24};
-  for (int axis = 0; axis < 3; ++axis) {
+  __shared__ double co[kNoAllocMaxAxis], si[kNoAllocMaxAxis];
+  __shared__ float mod[kNoAllocMaxAxis];
+  for (int axis = blockIdx.x; axis < 3; axis += gridDim.x) {
     const int n = S.grid[axis];
-    float* mod = p.moduli + axis * kNoAllocMaxAxis;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+      sincospi(2.0 * j / n, &si[j], &co[j]);
+      p.twiddles[axis * kNoAllocMaxAxis + j] = make_float2(float(co[j]), float(-si[j]));
+    }
+    __syncthreads();
+    const double knots[4] = {1.0 / 24, 11.0 / 24, 11.0 / 24, 1.0 / 24};
     for (int m = threadIdx.x; m < n; m += blockDim.x) {
       double re = 0, im = 0;
-      for (int k = 0; k < 4 && k < n; ++k) {
-        double s, c;
-        sincospi(2.0 * double((static_cast<long long>(m) * k) % n) / n, &s, &c);
-        re += knots[k] * c;
-        im += knots[k] * s;
+      for (int k = 0; k < 4; ++k) {  // an axis has at least five points
+        re += knots[k] * co[(m * k) % n];
+        im += knots[k] * si[(m * k) % n];
       }
       mod[m] = float(re * re + im * im);
-      double s, c;
-      sincospi(-2.0 * m / n, &s, &c);
-      p.twiddles[axis * kNoAllocMaxAxis + m] = make_float2(float(c), float(s));
     }
-  }
-  __syncthreads();
-  // bspline.ts:126 -- replace a vanishing modulus by its neighbours' mean
-  for (int axis = 0; axis < 3; ++axis) {
-    const int n = S.grid[axis];
-    float* mod = p.moduli + axis * kNoAllocMaxAxis;
-    if (threadIdx.x == 0)
-      for (int m = 0; m < n; ++m)
-        if (mod[m] < 1e-7f) mod[m] = 0.5f * (mod[(m - 1 + n) % n] + mod[(m + 1) % n]);
+    __syncthreads();
+    // bspline.ts:126 -- replace a vanishing modulus by its neighbours' mean,
+    // from the first point up (a replaced neighbour counts as replaced)
+    for (int m = threadIdx.x; m < n; m += blockDim.x) {
+      float* out = p.moduli + axis * kNoAllocMaxAxis;
+      const float before = mod[(m - 1 + n) % n], after = mod[(m + 1) % n];
+      out[m] = mod[m] < 1e-7f ? 0.5f * (before + after) : mod[m];
+    }
+    __syncthreads();
   }
 }
 
 __device__ __forceinline__ long long fixed_from_double(double x) { return __double2ll_rn(x * 4294967296.0); }
 
-__global__ void k_na_spread(SysDev S, NaPtrs p, int n, const double* pos, const double* charge) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float q = float(charge[i]);
+// By atom: the caller's order says nothing about where the atoms are.  A
+// block computes its atoms' splines once (a thread per atom and axis), then
+// shares the 25 rows of 5 z points per atom over its threads.
+constexpr int kNaAtoms = 32;
+
+__global__ void __launch_bounds__(kThreads) k_na_spread(SysDev S, NaPtrs p, int n, const double* pos,
+                                                        const double* charge) {
+  wait_for_predecessor();
+  __shared__ int base[kNaAtoms][3];
+  __shared__ float th[kNaAtoms][3][5], qs[kNaAtoms];
+  const int first = blockIdx.x * kNaAtoms;
+  for (int w = threadIdx.x; w < 3 * kNaAtoms; w += blockDim.x) {
+    const int axis = w / kNaAtoms, k = w - axis * kNaAtoms, i = first + k;
+    const float q = i < n ? float(charge[i]) : 0.f;
+    if (axis == 0) qs[k] = q;
     if (q == 0.f) continue;
-    Spline sp;
-    spline_for(S, fixed_from_double(pos[3 * i]), fixed_from_double(pos[3 * i + 1]),
-               fixed_from_double(pos[3 * i + 2]), sp, false);
-    const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2];
-    for (int ix = 0; ix < kPmeOrder; ++ix) {
-      int gx = sp.base[0] + ix;
-      if (gx >= Kx) gx -= Kx;
-      const float wx = q * sp.th[0][ix];
-      for (int iy = 0; iy < kPmeOrder; ++iy) {
-        int gy = sp.base[1] + iy;
-        if (gy >= Ky) gy -= Ky;
-        const float wxy = wx * sp.th[1][iy];
-        unsigned long long* row = p.grid + (static_cast<long long>(gx) * Ky + gy) * Kz;
-        for (int iz = 0; iz < kPmeOrder; ++iz) {
-          int gz = sp.base[2] + iz;
-          if (gz >= Kz) gz -= Kz;
-          add_fixed(&row[gz], wxy * sp.th[2][iz]);
-        }
-      }
-    }
-  }
-}
-
-__global__ void k_na_z_forward(SysDev S, NaPtrs p, int lines_per_block) {
-  extern __shared__ float2 smem[];
-  const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2], kzh = S.kzh;
-  const int line0 = blockIdx.x * lines_per_block;
-  const int nl = min(lines_per_block, Kx * Ky - line0);
-  if (nl <= 0) return;
-  float2* A = smem;
-  float2* B = smem + nl * Kz;
-  unsigned long long* grid = p.grid + static_cast<long long>(line0) * Kz;
-  for (int i = threadIdx.x; i < nl * Kz; i += blockDim.x) {
-    A[i] = make_float2(from_fixed(static_cast<long long>(grid[i])), 0.f);
-    grid[i] = 0ull;
-  }
-  __syncthreads();
-  const float2* R = fft_lines(A, B, Kz, nl, S.radices[2], S.nradix[2], p.twiddles + 2 * kNoAllocMaxAxis, -1);
-  float2* out = p.spectrum + static_cast<long long>(line0) * kzh;
-  for (int i = threadIdx.x; i < nl * kzh; i += blockDim.x) {
-    const int line = i / kzh, k = i - line * kzh;
-    out[i] = R[line * Kz + k];
-  }
-}
-
-__global__ void k_na_y(SysDev S, NaPtrs p, int sign) {
-  extern __shared__ float2 smem[];
-  const int Ky = S.grid[1], kzh = S.kzh;
-  const int tiles = (kzh + 15) / 16;
-  const int x = blockIdx.x / tiles, kz0 = (blockIdx.x % tiles) * 16;
-  const int nk = min(16, kzh - kz0);
-  float2* A = smem;
-  float2* B = smem + nk * Ky;
-  float2* base = p.spectrum + static_cast<long long>(x) * Ky * kzh + kz0;
-  for (int i = threadIdx.x; i < nk * Ky; i += blockDim.x) {
-    const int y = i / nk, l = i - y * nk;
-    A[l * Ky + y] = base[static_cast<long long>(y) * kzh + l];
-  }
-  __syncthreads();
-  const float2* R = fft_lines(A, B, Ky, nk, S.radices[1], S.nradix[1], p.twiddles + kNoAllocMaxAxis, sign);
-  for (int i = threadIdx.x; i < nk * Ky; i += blockDim.x) {
-    const int y = i / nk, l = i - y * nk;
-    base[static_cast<long long>(y) * kzh + l] = R[l * Ky + y];
-  }
-}
-
-__global__ void k_na_x_convolve(SysDev S, NaPtrs p) {
-  extern __shared__ float2 smem[];
-  __shared__ double partial[kThreads / 32];
-  const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2], kzh = S.kzh;
-  const int tiles = (kzh + 15) / 16;
-  const int my = blockIdx.x / tiles, kz0 = (blockIdx.x % tiles) * 16;
-  const int nk = min(16, kzh - kz0);
-  float2* A = smem;
-  float2* B = smem + nk * Kx;
-  const long long stride = static_cast<long long>(Ky) * kzh;
-  float2* base = p.spectrum + static_cast<long long>(my) * kzh + kz0;
-  for (int i = threadIdx.x; i < nk * Kx; i += blockDim.x) {
-    const int x = i / nk, l = i - x * nk;
-    A[l * Kx + x] = base[x * stride + l];
-  }
-  __syncthreads();
-  float2* R = fft_lines(A, B, Kx, nk, S.radices[0], S.nradix[0], p.twiddles, -1);
-  float2* other = R == A ? B : A;
-  const int mb = my <= Ky / 2 ? my : my - Ky;
-  const float* modx = p.moduli;
-  const float* mody = p.moduli + kNoAllocMaxAxis;
-  const float* modz = p.moduli + 2 * kNoAllocMaxAxis;
-  double energy = 0.0;
-  for (int i = threadIdx.x; i < nk * Kx; i += blockDim.x) {
-    const int l = i / Kx, mx = i - l * Kx;
-    const int kz = kz0 + l;
-    float2 v = R[i];
-    float kx, ky, kzv, k2;
-    const float factor = influence(S, modx, mody, modz, Kx, mx, mb, my, kz, kx, ky, kzv, k2);
-    const double weight = (kz == 0 || (2 * kz == Kz)) ? 1.0 : 2.0;
-    energy += weight * double(factor) * (double(v.x) * v.x + double(v.y) * v.y);
-    v.x *= 2.f * factor;
-    v.y *= 2.f * factor;
-    R[i] = v;
-  }
-  __syncthreads();
-  const float2* Q = fft_lines(R, other, Kx, nk, S.radices[0], S.nradix[0], p.twiddles, +1);
-  for (int i = threadIdx.x; i < nk * Kx; i += blockDim.x) {
-    const int x = i / nk, l = i - x * nk;
-    base[x * stride + l] = Q[l * Kx + x];
-  }
+    float weights[5];
+    base[k][axis] = spline_axis(S, axis, fixed_from_double(pos[3 * i]), fixed_from_double(pos[3 * i + 1]),
+                                fixed_from_double(pos[3 * i + 2]), weights, nullptr);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) energy += __shfl_xor_sync(0xffffffffu, energy, o);
-  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = energy;
+    for (int j = 0; j < kPmeOrder; ++j) th[k][axis][j] = weights[j];
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double total = 0.0;
-    for (int k = 0; k < (blockDim.x >> 5); ++k) total += partial[k];
-    p.partials[blockIdx.x] = total;
+  const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2];
+  for (int w = threadIdx.x; w < kNaAtoms * kPmeOrder * kPmeOrder; w += blockDim.x) {
+    const int k = w / (kPmeOrder * kPmeOrder), r = w - k * kPmeOrder * kPmeOrder;
+    const float q = qs[k];
+    if (q == 0.f) continue;
+    const int ix = r / kPmeOrder, iy = r - ix * kPmeOrder;
+    int gx = base[k][0] + ix, gy = base[k][1] + iy;
+    if (gx >= Kx) gx -= Kx;
+    if (gy >= Ky) gy -= Ky;
+    const float wxy = q * th[k][0][ix] * th[k][1][iy];
+    unsigned long long* row = p.grid + (static_cast<long long>(gx) * Ky + gy) * Kz;
+#pragma unroll
+    for (int iz = 0; iz < kPmeOrder; ++iz) {
+      int gz = base[k][2] + iz;
+      if (gz >= Kz) gz -= Kz;
+      add_fixed(&row[gz], wxy * th[k][2][iz]);
+    }
   }
 }
 
-__global__ void k_na_z_inverse(SysDev S, NaPtrs p, int lines_per_block) {
+__device__ __forceinline__ Mesh mesh_of(const SysDev& S, const NaPtrs& p) {
+  Mesh m;
+  m.x = {S.grid[0], S.plan[0]};
+  m.y = {S.grid[1], S.plan[1]};
+  m.z = {S.grid[2], S.plan[2]};
+  m.kzh = S.kzh;
+  m.charge = p.grid;
+  m.spectrum = p.spectrum;
+  m.potential = p.potential;
+  m.twx = p.twiddles;
+  m.twy = p.twiddles + kNoAllocMaxAxis;
+  m.twz = p.twiddles + 2 * kNoAllocMaxAxis;
+  return m;
+}
+
+// The engine's passes over this mesh: block b of each takes plane b, or strip
+// b of a plane.
+__global__ void __launch_bounds__(kPlaneThreads) k_na_planes_forward(SysDev S, NaPtrs p) {
+  wait_for_predecessor();
   extern __shared__ float2 smem[];
-  const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2], kzh = S.kzh;
-  const int line0 = blockIdx.x * lines_per_block;
-  const int nl = min(lines_per_block, Kx * Ky - line0);
-  if (nl <= 0) return;
-  float2* A = smem;
-  float2* B = smem + nl * Kz;
-  const float2* in = p.spectrum + static_cast<long long>(line0) * kzh;
-  for (int i = threadIdx.x; i < nl * kzh; i += blockDim.x) {
-    const int line = i / kzh, k = i - line * kzh;
-    A[line * Kz + k] = in[i];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < nl * (Kz - kzh); i += blockDim.x) {
-    const int line = i / (Kz - kzh), k = kzh + (i - line * (Kz - kzh));
-    const float2 c = A[line * Kz + (Kz - k)];
-    A[line * Kz + k] = make_float2(c.x, -c.y);
-  }
-  __syncthreads();
-  const float2* R = fft_lines(A, B, Kz, nl, S.radices[2], S.nradix[2], p.twiddles + 2 * kNoAllocMaxAxis, +1);
-  float* out = p.potential + static_cast<long long>(line0) * Kz;
-  for (int i = threadIdx.x; i < nl * Kz; i += blockDim.x) out[i] = R[i].x;
+  plane_forward(mesh_of(S, p), blockIdx.x, smem);
+}
+__global__ void __launch_bounds__(kPlaneThreads) k_na_planes_inverse(SysDev S, NaPtrs p) {
+  wait_for_predecessor();
+  extern __shared__ float2 smem[];
+  plane_inverse(mesh_of(S, p), blockIdx.x, smem);
+}
+// z and y passes for planes that do not fit shared memory: `lines` (even) z
+// lines of a plane, kFftTile columns of one
+__global__ void __launch_bounds__(kThreads) k_na_z_forward(SysDev S, NaPtrs p, int lines) {
+  wait_for_predecessor();
+  extern __shared__ float2 smem[];
+  const int Ky = S.grid[1], per = (Ky + lines - 1) / lines, x = blockIdx.x / per, y = (blockIdx.x - x * per) * lines;
+  z_forward(mesh_of(S, p), x * Ky + y, min(lines, Ky - y), smem);
+}
+__global__ void __launch_bounds__(kThreads) k_na_z_inverse(SysDev S, NaPtrs p, int lines) {
+  wait_for_predecessor();
+  extern __shared__ float2 smem[];
+  const int Ky = S.grid[1], per = (Ky + lines - 1) / lines, x = blockIdx.x / per, y = (blockIdx.x - x * per) * lines;
+  z_inverse(mesh_of(S, p), x * Ky + y, min(lines, Ky - y), smem);
+}
+template <int SIGN>
+__global__ void __launch_bounds__(kThreads) k_na_y(SysDev S, NaPtrs p) {
+  wait_for_predecessor();
+  extern __shared__ float2 smem[];
+  const int per = (S.kzh + kFftTile - 1) / kFftTile, x = blockIdx.x / per, kz0 = (blockIdx.x - x * per) * kFftTile;
+  y_pass<SIGN>(mesh_of(S, p), x, kz0, min(kFftTile, S.kzh - kz0), smem);
 }
 
-__global__ void k_na_gather(SysDev S, NaPtrs p, int n, const double* pos, const double* charge, double* forces) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float q = float(charge[i]);
-    if (q == 0.f) {
-      forces[3 * i] = forces[3 * i + 1] = forces[3 * i + 2] = 0.0;
-      continue;
-    }
-    Spline sp;
-    spline_for(S, fixed_from_double(pos[3 * i]), fixed_from_double(pos[3 * i + 1]),
-               fixed_from_double(pos[3 * i + 2]), sp, true);
-    const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2];
-    float ga = 0.f, gb = 0.f, gc = 0.f;
-    for (int ix = 0; ix < kPmeOrder; ++ix) {
-      int gx = sp.base[0] + ix;
-      if (gx >= Kx) gx -= Kx;
-      for (int iy = 0; iy < kPmeOrder; ++iy) {
-        int gy = sp.base[1] + iy;
-        if (gy >= Ky) gy -= Ky;
-        const float* row = p.potential + (static_cast<long long>(gx) * Ky + gy) * Kz;
-        const float wxy = sp.th[0][ix] * sp.th[1][iy];
-        const float dxy = sp.dth[0][ix] * sp.th[1][iy];
-        const float xdy = sp.th[0][ix] * sp.dth[1][iy];
-        for (int iz = 0; iz < kPmeOrder; ++iz) {
-          int gz = sp.base[2] + iz;
-          if (gz >= Kz) gz -= Kz;
-          const float v = row[gz];
-          ga = fmaf(v * dxy, sp.th[2][iz], ga);
-          gb = fmaf(v * xdy, sp.th[2][iz], gb);
-          gc = fmaf(v * wxy, sp.dth[2][iz], gc);
-        }
-      }
-    }
-    const float* U = S.umat_f;
-    forces[3 * i] = -q * (ga * U[0] + gb * U[1] + gc * U[2]);
-    forces[3 * i + 1] = -q * (ga * U[3] + gb * U[4] + gc * U[5]);
-    forces[3 * i + 2] = -q * (ga * U[6] + gb * U[7] + gc * U[8]);
-  }
+__global__ void __launch_bounds__(kXThreads) k_na_x_convolve(SysDev S, NaPtrs p) {
+  wait_for_predecessor();
+  extern __shared__ float2 smem[];
+  const int per = (S.kzh + kFftTile - 1) / kFftTile, my = blockIdx.x / per, kz0 = (blockIdx.x - my * per) * kFftTile;
+  const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2], mb = my <= Ky / 2 ? my : my - Ky;
+  double energy[1] = {0.0};
+  x_pass(mesh_of(S, p), my, kz0, min(kFftTile, S.kzh - kz0), smem, [&](int mx, int l, float2 v) {
+    const int kz = kz0 + l;
+    float kx, ky, kzv, k2;
+    const float f = influence(S, p.moduli, p.moduli + kNoAllocMaxAxis, p.moduli + 2 * kNoAllocMaxAxis, Kx, mx, mb, my, kz,
+                              kx, ky, kzv, k2);
+    const double weight = (kz == 0 || (2 * kz == Kz)) ? 1.0 : 2.0;
+    energy[0] += weight * double(f) * (double(v.x) * v.x + double(v.y) * v.y);
+    const float g = 2.f * f;
+    return make_float2(__fmul_rn(v.x, g), __fmul_rn(v.y, g));
+  });
+  block_sums<1>(energy, [&](int, double total) { p.partials[blockIdx.x] = total; });
 }
 
-__global__ void k_na_energy(NaPtrs p, int count, double* energy) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double total = 0.0;
-    for (int k = 0; k < count; ++k) total += p.partials[k];
-    *energy = total;
+// Forces; and, by the last block's first warp, the energy from the x pass'
+// `count` partial sums, in a fixed order.
+__global__ void __launch_bounds__(kGatherThreads) k_na_gather(SysDev S, NaPtrs p, int n, const double* pos,
+                                                              const double* charge, double* forces, int count,
+                                                              double* energy) {
+  wait_for_predecessor();
+  __shared__ GatherTable table;
+  if (blockIdx.x == gridDim.x - 1) {  // the whole block
+    if (threadIdx.x < 32) {
+      double total = 0.0;
+      for (int k = threadIdx.x; k < count; k += 32) total += p.partials[k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+      if (threadIdx.x == 0) *energy = total;
+    }
+    return;
   }
+  const int i = blockIdx.x * kGatherAtoms + (threadIdx.x & 31);
+  const float q = i < n ? float(charge[i]) : 0.f;
+  const bool live = q != 0.f;
+  if (i < n && !live && threadIdx.x < 32) forces[3 * i] = forces[3 * i + 1] = forces[3 * i + 2] = 0.0;
+  float ga, gb, gc;
+  if (!gather_block(table, live, S, p.potential, live ? fixed_from_double(pos[3 * i]) : 0,
+                    live ? fixed_from_double(pos[3 * i + 1]) : 0, live ? fixed_from_double(pos[3 * i + 2]) : 0, ga, gb,
+                    gc))
+    return;
+  const float3 f = mesh_force(S, q, ga, gb, gc);
+  forces[3 * i] = f.x;
+  forces[3 * i + 1] = f.y;
+  forces[3 * i + 2] = f.z;
 }
 
 // The scratch array's device address, looked up with the device current.  In
@@ -1224,7 +1402,7 @@ extern "C" int mdb_reciprocal_noalloc(int32_t n, const double* positions, const 
   std::memset(&S, 0, sizeof(S));
   for (int k = 0; k < 3; ++k) {
     S.grid[k] = mesh[k];
-    if (!plan_radices(mesh[k], S.radices[k], &S.nradix[k])) return MDB_ERR_NOT_SMOOTH;
+    if (!plan_radices(mesh[k], &S.plan[k])) return MDB_ERR_NOT_SMOOTH;
   }
   S.kzh = mesh[2] / 2 + 1;
   double B[9], M[9];
@@ -1258,21 +1436,25 @@ extern "C" int mdb_reciprocal_noalloc(int32_t n, const double* positions, const 
   p.twiddles = reinterpret_cast<float2*>(base + kNaTwiddles);
   p.partials = reinterpret_cast<double*>(base + kNaPartials);
 
-  const int lines = std::max(1, 2048 / mesh[2]);
-  const int z_blocks = int((mesh[0] * mesh[1] + lines - 1) / lines);
-  const int tiles = (S.kzh + 15) / 16;
-  const int z_smem = 2 * lines * mesh[2] * int(sizeof(float2));
-  const int y_smem = 2 * 16 * mesh[1] * int(sizeof(float2));
-  const int x_smem = 2 * 16 * mesh[0] * int(sizeof(float2));
-  const int atom_blocks = std::max(1, std::min((n + kThreads - 1) / kThreads, 148 * 8));
-  k_na_setup<<<std::max(1, int(std::min<long long>((points + kThreads - 1) / kThreads, 148 * 8))), kThreads, 0, st>>>(S, p);
-  if (n > 0) k_na_spread<<<atom_blocks, kThreads, 0, st>>>(S, p, n, positions, charges);
-  k_na_z_forward<<<z_blocks, kThreads, z_smem, st>>>(S, p, lines);
-  k_na_y<<<mesh[0] * tiles, kThreads, y_smem, st>>>(S, p, -1);
-  k_na_x_convolve<<<mesh[1] * tiles, kThreads, x_smem, st>>>(S, p);
-  k_na_y<<<mesh[0] * tiles, kThreads, y_smem, st>>>(S, p, +1);
-  k_na_z_inverse<<<z_blocks, kThreads, z_smem, st>>>(S, p, lines);
-  if (n > 0) k_na_gather<<<atom_blocks, kThreads, 0, st>>>(S, p, n, positions, charges, forces);
-  k_na_energy<<<1, 32, 0, st>>>(p, mesh[1] * tiles, energy);
+  const int Kx = mesh[0], Ky = mesh[1], Kz = mesh[2];
+  const int tiles = (S.kzh + kFftTile - 1) / kFftTile;
+  k_na_setup<<<std::max(3, int(std::min<long long>((points + 1023) / 1024, 148 * 4))), kThreads, 0, st>>>(S, p);
+  if (n > 0) launch_chained(k_na_spread, (n + kNaAtoms - 1) / kNaAtoms, kThreads, 0, st, S, p, n, positions, charges);
+  const int plane = plane_smem(Ky, Kz), lines = std::max(2, 2048 / Kz & ~1);
+  if (plane <= kNoAllocPlaneSmem) {
+    launch_chained(k_na_planes_forward, Kx, kPlaneThreads, plane, st, S, p);
+  } else {
+    launch_chained(k_na_z_forward, Kx * ((Ky + lines - 1) / lines), kThreads, z_smem(lines, Kz), st, S, p, lines);
+    launch_chained(k_na_y<-1>, Kx * tiles, kThreads, strip_smem(kFftTile, Ky), st, S, p);
+  }
+  launch_chained(k_na_x_convolve, Ky * tiles, kXThreads, strip_smem(kFftTile, Kx), st, S, p);
+  if (plane <= kNoAllocPlaneSmem) {
+    launch_chained(k_na_planes_inverse, Kx, kPlaneThreads, plane, st, S, p);
+  } else {
+    launch_chained(k_na_y<+1>, Kx * tiles, kThreads, strip_smem(kFftTile, Ky), st, S, p);
+    launch_chained(k_na_z_inverse, Kx * ((Ky + lines - 1) / lines), kThreads, z_smem(lines, Kz), st, S, p, lines);
+  }
+  launch_chained(k_na_gather, (n + kGatherAtoms - 1) / kGatherAtoms + 1, kGatherThreads, 0, st, S, p, n, positions, charges,
+                 forces, Ky * tiles, energy);
   return cudaGetLastError() == cudaSuccess ? MDB_OK : MDB_ERR_DEVICE;
 }

@@ -116,13 +116,37 @@ std::vector<double> bspline_moduli(int n) {
 
 // Stages for the shared-memory Stockham FFT: radix 4 where it divides, then
 // 7, 5, 3, 2.  False for a length that is not 2/3/5/7-smooth.
-bool plan_radices(int n, int* radices, int* count) {
-  int c = 0, r = n;
-  while (r % 4 == 0 && c < kMaxRadices) { radices[c++] = 4; r /= 4; }
-  for (int p : {7, 5, 3, 2})
-    while (r % p == 0 && c < kMaxRadices) { radices[c++] = p; r /= p; }
-  *count = c;
-  return r == 1;
+bool plan_radices(int n, unsigned* plan) {
+  // the fewest stages (a stage is a pass through shared memory and a barrier),
+  // and among those the smallest largest radix: n <= 10^8 in eight of them
+  *plan = 0;
+  unsigned best[9];
+  int count = 0;
+  std::array<unsigned, 9> now{};
+  int least_max = 99;
+  const auto search = [&](auto&& self, int rest, int depth, unsigned low) -> void {
+    if (rest == 1) {
+      if (depth == 0) return;
+      const int top = int(now[depth - 1]);  // ascending
+      if (count == 0 || depth < count || (depth == count && top < least_max)) {
+        count = depth;
+        least_max = top;
+        std::copy(now.begin(), now.begin() + depth, best);
+      }
+      return;
+    }
+    if (depth == 8 || (count > 0 && depth >= count)) return;
+    for (unsigned r = low; r <= 10; ++r)
+      if (rest % int(r) == 0) {
+        now[depth] = r;
+        self(self, rest / int(r), depth + 1, r);
+      }
+  };
+  if (n < 1) return false;
+  if (n == 1) return true;
+  search(search, n, 0, 2);
+  for (int k = 0; k < count; ++k) *plan |= best[k] << (4 * k);
+  return count > 0;
 }
 
 // nonbonded.ts:107 (dispersion, grouped by class), :594 (net charge), :610 (self)
@@ -218,8 +242,8 @@ int prepare_system(const mdb_system_desc& in, const mdb_state_desc& state, const
     int g = opt.mesh[k] > 0 ? opt.mesh[k] : in.grid[k];
     // potential.ts:79 -- the mesh from the box *diagonal*
     if (g <= 0) g = smooth_size(pme_minimum_grid(h.alpha, h.box[k * 4], h.tolerance));
-    int rad[kMaxRadices], nr = 0;
-    if (!plan_radices(g, rad, &nr)) {
+    unsigned plan = 0;
+    if (!plan_radices(g, &plan)) {
       msg << "mesh size " << g << " is not 2/3/5/7-smooth, so the transform cannot do it";
       error = msg.str();
       return MDB_ERR_NOT_SMOOTH;

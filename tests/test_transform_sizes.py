@@ -1,0 +1,84 @@
+"""The mesh transforms and the charge spread at the sizes where they can go
+wrong: axes of one, two and three stages, odd planes (whose last z line has no
+partner), planes that fit shared memory and planes that do not, charges past
+the range of the spread's f32 fixed-point split, and spread blocks that hold
+the end of one system and the start of the next.
+
+Bounds: reciprocal forces against the f64 oracle at the 1e-5 relative RMS the
+oracle's own PME forces are pinned to (an f32 transform of n points loses
+about log2(n) 2^-24, a few 1e-7); grids are integers, so routes that only
+differ in the order of the spread agree to the bit.
+"""
+
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from test_zz_no_alloc import ENERGY_REL, RECIPROCAL_FORCE_REL_RMS, separated_charges
+
+pytestmark = pytest.mark.gpu
+
+# one stage; odd; three stages (7^3 is past 128, 98 = 2 7^2 is three); both
+# sides of the plane kernels' shared memory; the largest
+MESHES = [(10, 9, 8), (21, 15, 25), (35, 27, 49), (98, 27, 14), (20, 100, 128), (18, 125, 63), (64, 64, 64)]
+
+
+@pytest.mark.parametrize("mesh", MESHES)
+def test_mesh_forces_and_energy(mesh):
+    import torch
+
+    from mdb200 import abi
+    from oracle import oracle
+
+    system, state, alpha = separated_charges()
+    want, want_forces = oracle.potential(system, state.positions, grid=mesh)
+    n = system.particle_count
+    pos, q = torch.from_numpy(state.positions).cuda(), torch.from_numpy(system.nonbonded.charge).cuda()
+    forces = torch.full((n, 3), 7.0, dtype=torch.float64, device="cuda")
+    energy = torch.full((1,), 7.0, dtype=torch.float64, device="cuda")
+    for _ in range(2):  # the second call finds the first one's scratch
+        status = abi.load().mdb_reciprocal_noalloc(
+            n, pos.data_ptr(), q.data_ptr(), (C.c_double * 9)(*np.asarray(state.box).reshape(9)), alpha,
+            (C.c_int32 * 3)(*mesh), forces.data_ptr(), energy.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert status == abi.OK
+        got = forces.cpu().numpy()
+        # the charges are farther apart than the cutoff: direct forces are zero
+        assert np.sqrt(((got - want_forces) ** 2).sum() / (want_forces**2).sum()) < RECIPROCAL_FORCE_REL_RMS
+        assert abs(energy.item() - want["reciprocal_mesh"]) < ENERGY_REL * abs(want["reciprocal_mesh"])
+
+
+@pytest.mark.parametrize("mesh", [(21, 15, 25), (24, 120, 120)])
+@pytest.mark.parametrize("charge", [1.0, 1500.0])
+def test_engine_mesh_forces(mesh, charge):
+    """The engine's own passes, whole planes and strips, and charges beyond
+    1,000 e, which the spread converts the long way."""
+    from mdb200 import steploop
+    from oracle import oracle
+
+    system, state, _ = separated_charges()
+    system.nonbonded.charge = system.nonbonded.charge * charge
+    _, want = oracle.potential(system, state.positions, grid=mesh)
+    loop = steploop.StepLoop.from_parsed(system, state, steploop.RunOptions(mesh=mesh))
+    _, got = loop.evaluate()
+    loop.destroy()
+    assert np.sqrt(((got - want) ** 2).sum() / (want**2).sum()) < RECIPROCAL_FORCE_REL_RMS
+
+
+@pytest.mark.parametrize("counts", [(672, 700), (672, 683, 691, 705, 672, 690, 750)])
+def test_spread_blocks_across_systems(counts):
+    """Systems whose slots are no multiple of a spread block's: the batch
+    moves each as it moves alone, to the bit."""
+    from mdb200 import steploop, synth
+
+    members = [synth.water_box(n_waters=n, width=2.9, seed=40 + k, grid=(28, 27, 30)) for k, n in enumerate(counts)]
+    batch = steploop.StepLoop.batch([m[0] for m in members], [m[1] for m in members], steploop.RunOptions(seed=5))
+    batch.run(12)
+    for k, (system, state) in enumerate(members):
+        alone = steploop.StepLoop.from_parsed(system, state, steploop.RunOptions(seed=5))
+        alone.run(12)
+        assert np.array_equal(batch.positions(k), alone.positions()), k
+        alone.destroy()
+    batch.destroy()
