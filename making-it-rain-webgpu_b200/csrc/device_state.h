@@ -152,6 +152,8 @@ struct Dev {
   const int* iblk_atom0;  // first table entry of each integrate block in `iatom`
   const int* iblk_natom;
   const int* iatom;       // global atom index of every table entry, block by block
+  const int* entry;       // per atom: its table entry
+  int* islot;             // per table entry: its atom's slot (global), as the last rebuild sorted it
   double* mom_partial;  // 3 per integrate block
   float4* vcom;         // per system, for the next step's COM removal
   long long* step;      // per system

@@ -925,6 +925,11 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   d.iblk_natom = tmp_i;
   TRY(upload(e, "integrate block table", tmp_i, iatom));
   d.iatom = tmp_i;
+  std::vector<int> entry(iatom.size());
+  for (size_t k = 0; k < iatom.size(); ++k) entry[size_t(iatom[k])] = int(k);
+  TRY(upload(e, "integrate table entry", tmp_i, entry));
+  d.entry = tmp_i;
+  TRY(alloc(e, "integrate table slot", d.islot, iatom.size()));
   TRY(alloc(e, "momentum partials", d.mom_partial, size_t(iblk) * 3));
   TRY(alloc(e, "com velocity", d.vcom, n));
   std::vector<long long> steps(n);

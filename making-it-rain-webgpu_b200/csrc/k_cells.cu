@@ -162,6 +162,7 @@ __device__ void phase_cells_order(const Dev& d) {
     for (int k = 0; k < cnt; ++k) r += d.tmp_order[S.slot_off + st + k] < a;
     d.order[S.slot_off + st + r] = a;
     d.rank[a] = st + r;
+    d.islot[d.entry[a]] = S.slot_off + st + r;
   }
 }
 

@@ -240,60 +240,80 @@ __device__ __forceinline__ long long displace(float wanted, float& left_over) {
 // atom 0, to one spoke, atom c + 1): C-H, CH2, CH3, N-H, NH3+.  Written for
 // that shape with the constraint count known at compile time, the FP64 solves
 // stay in registers; the general `rattle`/`shake` above index their arrays at
-// run time and spill to local memory.  Same Jacobi iterations, same order.
-template <int NC>
-__device__ bool rattle_star(const long long* x, const long long* y, const long long* z, float* vx, float* vy,
-                            float* vz, const float* im, float tol) {
-  constexpr int NA = NC + 1;
-  double v[NA][3];
+// run time and spill to local memory.  The one to three multipliers of a star
+// come from their linear system at once, where the Jacobi sweeps of the
+// general solver need a dozen or two rounds of a dependent chain for CH2 and
+// CH3: the velocities exactly, the positions by Newton's method (three
+// rounds) on the same equations, to the same convergence window.
+
+// x of A x = b (n = 1 to 3, A row-major) by elimination without pivoting: the
+// stars' matrices are dominated by the spokes' own terms.  A zero row (both
+// atoms massless) gives zero.
+template <int N>
+__device__ __forceinline__ void solve_small(double (*A)[N], double* b) {
 #pragma unroll
-  for (int k = 0; k < NA; ++k) {
-    v[k][0] = vx[k]; v[k][1] = vy[k]; v[k][2] = vz[k];
+  for (int i = 0; i < N; ++i) {
+    const double inv = A[i][i] == 0.0 ? 0.0 : 1.0 / A[i][i];
+#pragma unroll
+    for (int j = i + 1; j < N; ++j) A[i][j] *= inv;
+    b[i] *= inv;
+#pragma unroll
+    for (int k = i + 1; k < N; ++k) {
+#pragma unroll
+      for (int j = i + 1; j < N; ++j) A[k][j] -= A[k][i] * A[i][j];
+      b[k] -= A[k][i] * b[i];
+    }
   }
-  // the reference bond vectors are f32 values (from_fixed) and the inverse
-  // masses f32: kept as f32 and widened where used, to save registers
+#pragma unroll
+  for (int i = N - 2; i >= 0; --i)
+#pragma unroll
+    for (int j = i + 1; j < N; ++j) b[i] -= A[i][j] * b[j];
+}
+
+template <int NC>
+__device__ __forceinline__ void rattle_star(const long long* x, const long long* y, const long long* z, float* vx,
+                                            float* vy, float* vz, const float* im) {
+  // the reference bond vectors are f32 values (from_fixed)
   float rv[NC][3];
-  double rl[NC], rm[NC], delta[NC];
+  double A[NC][NC], l[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     rv[c][0] = from_fixed(x[0] - x[c + 1]);
     rv[c][1] = from_fixed(y[0] - y[c + 1]);
     rv[c][2] = from_fixed(z[0] - z[c + 1]);
-    rl[c] = double(rv[c][0]) * rv[c][0] + double(rv[c][1]) * rv[c][1] + double(rv[c][2]) * rv[c][2];
-    const double sum = double(im[0]) + double(im[c + 1]);
-    rm[c] = sum == 0.0 ? 0.0 : 0.5 / sum;
+    l[c] = (double(vx[c + 1]) - vx[0]) * rv[c][0] + (double(vy[c + 1]) - vy[0]) * rv[c][1] +
+           (double(vz[c + 1]) - vz[0]) * rv[c][2];
   }
-  bool ok = false;
-  for (int it = 0; it < kMaxShakeIterations; ++it) {
-    int conv = 0;
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const double proj = (v[0][0] - v[c + 1][0]) * rv[c][0] + (v[0][1] - v[c + 1][1]) * rv[c][1] +
-                          (v[0][2] - v[c + 1][2]) * rv[c][2];
-      delta[c] = rl[c] == 0.0 ? 0.0 : (-2.0 * rm[c] * proj) / rl[c];
-      conv += fabs(delta[c]) <= tol;
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      const double dot = double(rv[c][0]) * rv[e][0] + double(rv[c][1]) * rv[e][1] + double(rv[c][2]) * rv[e][2];
+      A[c][e] = dot * (c == e ? double(im[0]) + double(im[c + 1]) : double(im[0]));
     }
-    if (conv == NC) { ok = true; break; }
+  solve_small<NC>(A, l);
+  double v0[3] = {vx[0], vy[0], vz[0]};
 #pragma unroll
-    for (int c = 0; c < NC; ++c)
+  for (int c = 0; c < NC; ++c) {
+    const double to0 = l[c] * double(im[0]), toc = l[c] * double(im[c + 1]);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const double dr = rv[c][k] * delta[c];
-        v[0][k] += dr * double(im[0]);
-        v[c + 1][k] -= dr * double(im[c + 1]);
-      }
+    for (int k = 0; k < 3; ++k) v0[k] += to0 * rv[c][k];
+    vx[c + 1] = float(vx[c + 1] - toc * rv[c][0]);
+    vy[c + 1] = float(vy[c + 1] - toc * rv[c][1]);
+    vz[c + 1] = float(vz[c + 1] - toc * rv[c][2]);
   }
-#pragma unroll
-  for (int k = 0; k < NA; ++k) {
-    vx[k] = float(v[k][0]); vy[k] = float(v[k][1]); vz[k] = float(v[k][2]);
-  }
-  return ok;
+  vx[0] = float(v0[0]);
+  vy[0] = float(v0[1]);
+  vz[0] = float(v0[2]);
 }
 
-// `dp` holds the trial displacements on input and the constrained ones on output.
+// `dp` holds the trial displacements on input and the constrained ones on
+// output.  False (dp untouched) if Newton's method has not converged in a few
+// rounds: the general solver's sweeps then take the cluster.
 template <int NC>
-__device__ bool shake_star(const long long* x, const long long* y, const long long* z, const float* im,
-                           const float* dist, float3* dp, float tol) {
+__device__ __forceinline__ bool shake_star(const long long* x, const long long* y, const long long* z, const float* im,
+                                           const float* dist, float3* dp, float tol) {
+  constexpr int kRounds = 8;
   constexpr int NA = NC + 1;
   double q[NA][3];
 #pragma unroll
@@ -301,42 +321,47 @@ __device__ bool shake_star(const long long* x, const long long* y, const long lo
     q[k][0] = dp[k].x; q[k][1] = dp[k].y; q[k][2] = dp[k].z;
   }
   float rv[NC][3];  // f32 values (from_fixed), widened where used
-  double rm[NC], delta[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     rv[c][0] = from_fixed(x[0] - x[c + 1]);
     rv[c][1] = from_fixed(y[0] - y[c + 1]);
     rv[c][2] = from_fixed(z[0] - z[c + 1]);
-    const double sum = double(im[0]) + double(im[c + 1]);
-    rm[c] = sum == 0.0 ? 0.0 : 0.5 / sum;
   }
   const double lo = 1.0 - 2.0 * tol + double(tol) * tol, hi = 1.0 + 2.0 * tol + double(tol) * tol;
   bool ok = false;
-  for (int it = 0; it < kMaxShakeIterations; ++it) {
+#pragma unroll 1
+  for (int it = 0; it <= kRounds; ++it) {
     int conv = 0;
+    double A[NC][NC], l[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const double d2 = double(dist[c]) * dist[c];
       const double ex = rv[c][0] + q[0][0] - q[c + 1][0], ey = rv[c][1] + q[0][1] - q[c + 1][1],
                    ez = rv[c][2] + q[0][2] - q[c + 1][2];
       const double l2 = ex * ex + ey * ey + ez * ez;
-      const double proj = ex * rv[c][0] + ey * rv[c][1] + ez * rv[c][2];
-      delta[c] = proj == 0.0 ? 0.0 : rm[c] * (d2 - l2) / proj;
       conv += (l2 >= lo * d2 && l2 <= hi * d2);
+      l[c] = 0.5 * (d2 - l2);
+#pragma unroll
+      for (int e = 0; e < NC; ++e)
+        A[c][e] = (ex * rv[e][0] + ey * rv[e][1] + ez * rv[e][2]) *
+                  (c == e ? double(im[0]) + double(im[c + 1]) : double(im[0]));
     }
     if (conv == NC) { ok = true; break; }
+    if (it == kRounds) break;
+    solve_small<NC>(A, l);
 #pragma unroll
     for (int c = 0; c < NC; ++c)
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        const double dr = rv[c][k] * delta[c];
+        const double dr = rv[c][k] * l[c];
         q[0][k] += dr * double(im[0]);
         q[c + 1][k] -= dr * double(im[c + 1]);
       }
   }
+  if (!ok) return false;
 #pragma unroll
   for (int k = 0; k < NA; ++k) dp[k] = make_float3(float(q[k][0]), float(q[k][1]), float(q[k][2]));
-  return ok;
+  return true;
 }
 
 __device__ void block_sum3(double* v, double (*red)[kThreads / 32]) {
@@ -355,47 +380,62 @@ __device__ void block_sum3(double* v, double (*red)[kThreads / 32]) {
     }
 }
 
+// A block's ticket: thread 0 has written the block's momentum and its rebuild
+// and prune requests; the fence orders them before the count.  The block that
+// draws its system's last number has every block's.
+__device__ __forceinline__ void take_ticket(const Dev& d, int s, const SysDev& S, int* last_of_system) {
+  if (threadIdx.x == 0) {
+    __threadfence();
+    *last_of_system = atomicAdd(&d.done_count[s], 1) == S.n_iblk - 1;
+  }
+}
+
 // The last block of a system turns the block momenta into the next step's
 // COM velocity (a fixed-order block reduction, so runs stay bit-identical) and
-// advances the step; the last block of the launch snapshots the rebuild
-// requests for the next step's list kernels.
-__device__ void finish_block(const Dev& d, int s, const SysDev& S, bool advance, double (*red)[kThreads / 32]) {
-  __shared__ int last_of_system, last_of_launch;
-  __threadfence();
-  if (threadIdx.x == 0) last_of_system = atomicAdd(&d.done_count[s], 1) == S.n_iblk - 1;
+// advances the step; the last of those blocks snapshots the rebuild requests
+// for the next step's list kernels.  Only a system's last block goes on to the
+// second ticket, and an engine of one system needs none.
+__device__ void finish_block(const Dev& d, int s, const SysDev& S, bool advance, const int* last_of_system,
+                             double (*red)[kThreads / 32]) {
+  __shared__ int last_of_launch;
   __syncthreads();
-  if (last_of_system) {
-    __threadfence();
-    double p[3] = {0, 0, 0};
-    for (int i = threadIdx.x; i < S.n_iblk; i += kThreads)
-      for (int k = 0; k < 3; ++k) p[k] += __ldcg(&d.mom_partial[(S.iblk_off + i) * 3 + k]);
-    block_sum3(p, red);
-    if (threadIdx.x == 0) {
-      const double m = S.total_mass > 0 ? S.total_mass : 1.0;
-      d.vcom[s] = make_float4(float(p[0] / m), float(p[1] / m), float(p[2] / m), 0.f);
-      if (advance) d.step[s] += 1;
-      d.done_count[s] = 0;
+  if (!*last_of_system) return;
+  __threadfence();
+  double p[3] = {0, 0, 0};
+  for (int i = threadIdx.x; i < S.n_iblk; i += kThreads)
+    for (int k = 0; k < 3; ++k) p[k] += __ldcg(&d.mom_partial[(S.iblk_off + i) * 3 + k]);
+  block_sum3(p, red);
+  if (threadIdx.x == 0) {
+    const double m = S.total_mass > 0 ? S.total_mass : 1.0;
+    d.vcom[s] = make_float4(float(p[0] / m), float(p[1] / m), float(p[2] / m), 0.f);
+    if (advance) d.step[s] += 1;
+    d.done_count[s] = 0;
+    last_of_launch = 1;
+    if (advance && d.S > 1) {
+      __threadfence();
+      last_of_launch = atomicAdd(d.global_ticket, 1) == d.S - 1;
     }
   }
   if (!advance) return;
-  __threadfence();
-  if (threadIdx.x == 0) last_of_launch = atomicAdd(d.global_ticket, 1) == int(gridDim.x) - 1;
   __syncthreads();
-  if (last_of_launch && threadIdx.x == 0) {
-    __threadfence();
-    int any = 0, any_prune = 0;
-    for (int k = 0; k < d.S; ++k) {
-      const int f = __ldcg(&d.rebuild_flag[k]) | d.run.always_rebuild;
-      d.rebuild_now[k] = f;
-      d.rebuild_flag[k] = 0;
-      any |= f;
-      if (d.inner) {
-        const int p = __ldcg(&d.prune_flag[k]);
-        d.prune_now[k] = p;
-        d.prune_flag[k] = 0;
-        any_prune |= p;
-      }
+  if (!last_of_launch) return;
+  __threadfence();
+  int any = 0, any_prune = 0;
+  for (int k = threadIdx.x; k < d.S; k += kThreads) {
+    const int f = __ldcg(&d.rebuild_flag[k]) | d.run.always_rebuild;
+    d.rebuild_now[k] = f;
+    d.rebuild_flag[k] = 0;
+    any |= f;
+    if (d.inner) {
+      const int q = __ldcg(&d.prune_flag[k]);
+      d.prune_now[k] = q;
+      d.prune_flag[k] = 0;
+      any_prune |= q;
     }
+  }
+  any = __syncthreads_or(any);
+  any_prune = __syncthreads_or(any_prune);
+  if (threadIdx.x == 0) {
     *d.any_rebuild = any;
     if (d.inner) *d.any_prune = any_prune;
     *d.global_ticket = 0;
@@ -412,7 +452,18 @@ struct Stage {
   long long cx[kIntegrateTable], cy[kIntegrateTable], cz[kIntegrateTable];  // constrained drift
   float vx[kIntegrateTable], vy[kIntegrateTable], vz[kIntegrateTable], im[kIntegrateTable];
   float rx[kIntegrateTable], ry[kIntegrateTable], rz[kIntegrateTable];     // drift residuals
+  // what the last phase reads, on its way in (cp.async) during the others
+  long long ref[3][kIntegrateTable];    // the list's reference position
+  long long prune[3][kIntegrateTable];  // the inner list's
+  int atom[kIntegrateTable], slot[kIntegrateTable], fold[kIntegrateTable];
 };
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src), "n"(BYTES)
+               : "memory");
+}
 
 constexpr int kPerThread = kIntegrateTable / kThreads;
 
@@ -444,9 +495,9 @@ __device__ void unit_velocities(Stage& sh, const UnitDev& u, float tol, bool& ba
     for (int k = 0; k < 3; ++k) { sh.vx[e + k] = at[k].vx; sh.vy[e + k] = at[k].vy; sh.vz[e + k] = at[k].vz; }
   } else if (u.kind == kUnitStar) {
     switch (u.nc) {
-      case 1: bad |= !rattle_star<1>(sh.x + e, sh.y + e, sh.z + e, sh.vx + e, sh.vy + e, sh.vz + e, sh.im + e, tol); break;
-      case 2: bad |= !rattle_star<2>(sh.x + e, sh.y + e, sh.z + e, sh.vx + e, sh.vy + e, sh.vz + e, sh.im + e, tol); break;
-      default: bad |= !rattle_star<3>(sh.x + e, sh.y + e, sh.z + e, sh.vx + e, sh.vy + e, sh.vz + e, sh.im + e, tol); break;
+      case 1: rattle_star<1>(sh.x + e, sh.y + e, sh.z + e, sh.vx + e, sh.vy + e, sh.vz + e, sh.im + e); break;
+      case 2: rattle_star<2>(sh.x + e, sh.y + e, sh.z + e, sh.vx + e, sh.vy + e, sh.vz + e, sh.im + e); break;
+      default: rattle_star<3>(sh.x + e, sh.y + e, sh.z + e, sh.vx + e, sh.vy + e, sh.vz + e, sh.im + e); break;
     }
   } else if (u.kind == kUnitShake) {
     cluster_velocities(sh, u, tol, bad);
@@ -465,17 +516,6 @@ __device__ __forceinline__ float3 staged_drift(const Stage& sh, int e) {
   return make_float3(from_fixed(sh.tx[e]), from_fixed(sh.ty[e]), from_fixed(sh.tz[e]));
 }
 
-template <int NC>
-__device__ __forceinline__ void star_positions(Stage& sh, const UnitDev& u, float tol, bool& bad) {
-  const int e = u.base;
-  float3 dp[NC + 1];
-#pragma unroll
-  for (int k = 0; k <= NC; ++k) dp[k] = staged_drift(sh, e + k);
-  bad |= !shake_star<NC>(sh.x + e, sh.y + e, sh.z + e, sh.im + e, u.dist, dp, tol);
-#pragma unroll
-  for (int k = 0; k <= NC; ++k) store_constrained(sh, e + k, dp[k]);
-}
-
 __device__ __noinline__ void cluster_positions(Stage& sh, const UnitDev& u, float tol, bool& bad) {
   const int e = u.base;
   Atom at[kMaxClusterAtoms];
@@ -486,6 +526,20 @@ __device__ __noinline__ void cluster_positions(Stage& sh, const UnitDev& u, floa
   }
   bad |= !shake(at, dp, u, tol);
   for (int k = 0; k < u.na; ++k) store_constrained(sh, e + k, dp[k]);
+}
+
+template <int NC>
+__device__ __forceinline__ void star_positions(Stage& sh, const UnitDev& u, float tol, bool& bad) {
+  const int e = u.base;
+  float3 dp[NC + 1];
+#pragma unroll
+  for (int k = 0; k <= NC; ++k) dp[k] = staged_drift(sh, e + k);
+  if (!shake_star<NC>(sh.x + e, sh.y + e, sh.z + e, sh.im + e, u.dist, dp, tol)) {
+    cluster_positions(sh, u, tol, bad);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k <= NC; ++k) store_constrained(sh, e + k, dp[k]);
 }
 
 // Position constraints of one unit: cx = constrained drift (the unconstrained
@@ -518,6 +572,7 @@ __device__ void unit_positions(Stage& sh, const UnitDev& u, float tol, bool& bad
 
 __global__ void __launch_bounds__(kThreads) k_integrate(Dev d) {
   __shared__ Stage sh;
+  __shared__ int last_of_system;
   __shared__ double red[3][kThreads / 32];
   wait_for_predecessor();
   const int b = blockIdx.x;
@@ -529,7 +584,7 @@ __global__ void __launch_bounds__(kThreads) k_integrate(Dev d) {
     // slots are cleared for the next step, which the host runs after it has
     // grown and rebuilt the list
     for (int e = threadIdx.x; e < d.iblk_natom[b]; e += kThreads) {
-      const int gs = S.slot_off + d.rank[d.iatom[d.iblk_atom0[b] + e]];
+      const int gs = d.islot[d.iblk_atom0[b] + e];
       d.fx[gs] = 0ull; d.fy[gs] = 0ull; d.fz[gs] = 0ull;
     }
     return;
@@ -552,10 +607,22 @@ __global__ void __launch_bounds__(kThreads) k_integrate(Dev d) {
   for (int j = 0; j < kPerThread; ++j) {
     const int e = threadIdx.x + j * kThreads;
     if (e >= natom) continue;
-    const int a = d.iatom[atom0 + e];
+    // the atom and its slot come from tables in this order, so everything else
+    // is one round of loads
+    const int a = d.iatom[atom0 + e], gs = d.islot[atom0 + e];
     float vx = d.vx[a], vy = d.vy[a], vz = d.vz[a];
     const float im = d.invm[a];
-    const int gs = S.slot_off + d.rank[a];
+    sh.atom[e] = a;
+    sh.slot[e] = gs;
+    copy_async<4>(&sh.fold[e], &d.fold[gs]);
+    copy_async<8>(&sh.ref[0][e], &d.refx[a]);
+    copy_async<8>(&sh.ref[1][e], &d.refy[a]);
+    copy_async<8>(&sh.ref[2][e], &d.refz[a]);
+    if (d.inner) {
+      copy_async<8>(&sh.prune[0][e], &d.prx[a]);
+      copy_async<8>(&sh.prune[1][e], &d.pry[a]);
+      copy_async<8>(&sh.prune[2][e], &d.prz[a]);
+    }
     const float fx = from_fixed(static_cast<long long>(d.fx[gs]));
     const float fy = from_fixed(static_cast<long long>(d.fy[gs]));
     const float fz = from_fixed(static_cast<long long>(d.fz[gs]));
@@ -596,7 +663,7 @@ __global__ void __launch_bounds__(kThreads) k_integrate(Dev d) {
       if (lfm) {
         float n0 = 0.f, n1 = 0.f, n2 = 0.f;
         if (R.draw_noise) {
-          const unsigned p = static_cast<unsigned>(d.iatom[atom0 + e] - S.atom_off);
+          const unsigned p = static_cast<unsigned>(sh.atom[e] - S.atom_off);
           const uint2 key = make_uint2(R.seed, kThermostatDomain);
           const float2 g0 = normal_pair(make_uint2(p * 2u, static_cast<unsigned>(step)), key);
           const float2 g1 = normal_pair(make_uint2(p * 2u + 1u, static_cast<unsigned>(step)), key);
@@ -629,15 +696,16 @@ __global__ void __launch_bounds__(kThreads) k_integrate(Dev d) {
   if (threadIdx.x < nunit) unit_positions(sh, units[threadIdx.x], R.tolerance, bad);
   __syncthreads();
 
-  // ---- atoms: velocity correction, store, rebuild test, momentum
+  // ---- atoms: velocity correction, rebuild test, momentum; the final state
+  // stays in the table until the block's sums are on their way
   const float idt = 1.f / dt;
   double mom[3] = {0, 0, 0};
   bool moved = false, strayed = false;
+  asm volatile("cp.async.wait_all;" ::: "memory");  // every thread reads only what it copied
 #pragma unroll
   for (int j = 0; j < kPerThread; ++j) {
     const int e = threadIdx.x + j * kThreads;
     if (e >= natom) continue;
-    const int a = d.iatom[atom0 + e];
     const float im = sh.im[e];
     const long long cx = sh.cx[e], cy = sh.cy[e], cz = sh.cz[e];
     long long px = sh.x[e], py = sh.y[e], pz = sh.z[e];
@@ -653,46 +721,60 @@ __global__ void __launch_bounds__(kThreads) k_integrate(Dev d) {
         vz = idt * from_fixed(cz);
       }
       px += cx; py += cy; pz += cz;
-      d.px[a] = px; d.py[a] = py; d.pz[a] = pz;
-      d.vx[a] = vx; d.vy[a] = vy; d.vz[a] = vz;
-      d.rx[a] = sh.rx[e]; d.ry[a] = sh.ry[e]; d.rz[a] = sh.rz[e];
+      sh.x[e] = px; sh.y[e] = py; sh.z[e] = pz;
+      sh.vx[e] = vx; sh.vy[e] = vy; sh.vz[e] = vz;
       const double m = 1.0 / im;
       mom[0] += m * vx; mom[1] += m * vy; mom[2] += m * vz;
       bad |= !isfinite(vx + vy + vz);
-    } else if (com) {
-      d.vx[a] = vx; d.vy[a] = vy; d.vz[a] = vz;
     }
-    {
-      // the next step's pair coordinates under this list's fold, so the list
-      // kernel need not wrap again unless a rebuild or a prune is due
-      const int gs = S.slot_off + d.rank[a];
-      long long na, nb, nc;
-      unpack_fold(d.fold[gs], na, nb, nc);
-      d.pc[gs] = pair_coordinate(S, px, py, pz, na, nb, nc);
-      d.spread_atom[gs] = a;  // the next step's spread reads this, not the order a rebuild rewrites
-    }
-    const float ex = from_fixed(px - d.refx[a]), ey = from_fixed(py - d.refy[a]),
-                ez = from_fixed(pz - d.refz[a]);
+    const float ex = from_fixed(px - sh.ref[0][e]), ey = from_fixed(py - sh.ref[1][e]),
+                ez = from_fixed(pz - sh.ref[2][e]);
     moved |= ex * ex + ey * ey + ez * ez > S.half_skin2;
     if (d.inner) {
-      const float qx = from_fixed(px - d.prx[a]), qy = from_fixed(py - d.pry[a]),
-                  qz = from_fixed(pz - d.prz[a]);
+      const float qx = from_fixed(px - sh.prune[0][e]), qy = from_fixed(py - sh.prune[1][e]),
+                  qz = from_fixed(pz - sh.prune[2][e]);
       strayed |= qx * qx + qy * qy + qz * qz > S.half_inner2;
     }
   }
-  if (moved) atomicOr(&d.rebuild_flag[s], 1);
-  if (strayed) atomicOr(&d.prune_flag[s], 1);
   if (bad) atomicAdd(&d.shake_failures[s], 1);
+  const bool any_moved = __syncthreads_or(moved), any_strayed = __syncthreads_or(strayed);
   block_sum3(mom, red);
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0) {
     for (int k = 0; k < 3; ++k) d.mom_partial[b * 3 + k] = mom[k];
-  finish_block(d, s, S, true, red);
+    if (any_moved) atomicOr(&d.rebuild_flag[s], 1);
+    if (any_strayed) atomicOr(&d.prune_flag[s], 1);
+  }
+  take_ticket(d, s, S, &last_of_system);
+
+  // ---- atoms: store, while the ticket is out
+#pragma unroll
+  for (int j = 0; j < kPerThread; ++j) {
+    const int e = threadIdx.x + j * kThreads;
+    if (e >= natom) continue;
+    const int a = sh.atom[e], gs = sh.slot[e];
+    const long long px = sh.x[e], py = sh.y[e], pz = sh.z[e];
+    if (sh.im[e] != 0.f) {
+      d.px[a] = px; d.py[a] = py; d.pz[a] = pz;
+      d.vx[a] = sh.vx[e]; d.vy[a] = sh.vy[e]; d.vz[a] = sh.vz[e];
+      d.rx[a] = sh.rx[e]; d.ry[a] = sh.ry[e]; d.rz[a] = sh.rz[e];
+    } else if (com) {
+      d.vx[a] = sh.vx[e]; d.vy[a] = sh.vy[e]; d.vz[a] = sh.vz[e];
+    }
+    // the next step's pair coordinates under this list's fold, so the list
+    // kernel need not wrap again unless a rebuild or a prune is due
+    long long na, nb, nc;
+    unpack_fold(sh.fold[e], na, nb, nc);
+    d.pc[gs] = pair_coordinate(S, px, py, pz, na, nb, nc);
+    d.spread_atom[gs] = a;  // the next step's spread reads this, not the order a rebuild rewrites
+  }
+  finish_block(d, s, S, true, &last_of_system, red);
 }
 
 // The momentum of the current velocities, for the first COM removal after the
 // host set them.
 __global__ void __launch_bounds__(kThreads) k_momentum(Dev d) {
   __shared__ double red[3][kThreads / 32];
+  __shared__ int last_of_system;
   const int b = blockIdx.x;
   const int s = d.iblk_sys[b];
   const SysDev& S = d.sys[s];
@@ -707,7 +789,8 @@ __global__ void __launch_bounds__(kThreads) k_momentum(Dev d) {
   block_sum3(mom, red);
   if (threadIdx.x == 0)
     for (int k = 0; k < 3; ++k) d.mom_partial[b * 3 + k] = mom[k];
-  finish_block(d, s, S, false, red);
+  take_ticket(d, s, S, &last_of_system);
+  finish_block(d, s, S, false, &last_of_system, red);
 }
 
 }  // namespace
