@@ -23,6 +23,7 @@ namespace mdb {
 constexpr double kOne4PiEps0 = 138.93545764498457;  // src/engine/units.ts:18
 constexpr double kBoltzmann = 0.008314462618153242;  // units.ts:15
 constexpr int kTile = 32;
+constexpr int kCellChunk = 512;  // cells of the spatial sort one block scans
 constexpr int kPmeOrder = 5;
 constexpr int kMaxClusterAtoms = 8;
 constexpr int kMaxClusterConstraints = 8;
@@ -81,6 +82,7 @@ struct SysDev {
   int n_blocks, block_off;
   int n_cells, cell_off;
   int cdim[3];
+  int chunk_off;     // first of its chunks of kCellChunk cells
   int tile_off, tile_cap;
   int triclinic;
   int energy_base;
@@ -98,6 +100,7 @@ struct SysDev {
   int pc_half[3];    // half of the diagonal in pair-coordinate units
   float pc_inv_diag[3];  // 1/diagonal in pair-coordinate units
   float cut2, list2, half_skin2, alpha, alpha_2_sqrtpi;
+  float one_image2;  // boxes whose half-extents' squares sum to less need no search over images
   float gauss_scale;  // -alpha^2 log2(e): exp(-(alpha r)^2) = 2^(r^2 gauss_scale)
   // the inner list: tiles with a pair inside (cutoff + inner skin)^2, re-pruned
   // from the outer list once an atom has moved (inner skin / 2)^2 since the last prune

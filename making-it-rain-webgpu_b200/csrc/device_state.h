@@ -60,19 +60,18 @@ struct Dev {
   float4 *bb_lo, *bb_hi;  // per cluster
   float4 *sb_lo, *sb_hi;  // per 32-slot super-cluster (the cluster boxes themselves when clusters are 32)
   int* fold;              // per slot: the lattice translation of the last rebuild's fold (3 x 10 bits)
-  int2* raw_tiles;        // the fill pass's list, before pruning
-  unsigned int* raw_masks;
-  int4* raw_shift;
-  unsigned char* tile_alive;  // per raw tile: some pair within cutoff + skin
-  int* row_alive;         // per cluster: surviving tiles of its row
-  int* alive_start;       // per cluster: their start after pruning
   int4* tile_shift;       // per tile: lattice shift of J in pair-coordinate units; w = 1: per-pair minimum image
-  int* tile_cnt;
+  int* tile_cnt;          // per segment of a row (row_segments to a row): its tiles and where they start
   int* tile_start;
+  int row_supers, row_segments;  // super-clusters of J to a segment; segments of the longest row
   const int* block_sys;
 
   // cells
-  int *cell_cnt, *cell_start, *cell_cur;
+  int *cell_cnt, *cell_start;
+  int* cell_arrival;      // per atom: its number among its cell's atoms, in the order they were counted
+  int* chunk_cnt;         // per chunk of kCellChunk cells: atoms in it
+  const int* chunk_sys;
+  int n_chunks;
   const int* cell_sys;
   const int* cell_map;
 
@@ -102,6 +101,7 @@ struct Dev {
   int* any_prune;
   long long* prune_count;  // per system: prunes between rebuilds
   int* inner_ticket;       // blocks of the inner-list kernel that have finished
+  int* list_ticket;        // and of the list's last phase
 
   // flags and status
   int* rebuild_flag;  // set by the integrator: some atom moved skin/2
@@ -196,10 +196,10 @@ constexpr int kFftTile = 8;  // kz columns per y- and x-pass CTA of the PME tran
 
 // ---- launchers (one per kernel file) ----
 int prepare_list_kernel(int device);                      // 0: no cooperative launch
-bool launch_list(const Dev& d, cudaStream_t s);            // sort + wrap + tiles, one launch
-void launch_rebuild_sort(const Dev& d, cudaStream_t s);     // phases 0-4
-void launch_wrap(const Dev& d, cudaStream_t s);
-void launch_rebuild_tiles(const Dev& d, cudaStream_t s);    // phases 5-9
+bool launch_list(const Dev& d, cudaStream_t s);            // all of the following, one launch
+void launch_prune_references(const Dev& d, cudaStream_t s);  // of the systems due a prune only
+void launch_rebuild_sort(const Dev& d, cudaStream_t s);      // cells, slots and what is kept by slot
+void launch_rebuild_tiles(const Dev& d, cudaStream_t s);     // boxes, rows, exclusions
 void launch_inner_prune(const Dev& d, cudaStream_t s);      // the inner list, when one is due
 void launch_nonbonded(const Dev& d, bool energy, cudaStream_t s);
 void launch_listed(const Dev& d, bool energy, cudaStream_t s);

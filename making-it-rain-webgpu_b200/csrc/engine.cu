@@ -46,6 +46,9 @@ constexpr double kDefaultInnerSkin = -1.0;  // nm; <= 0: no inner list unless a 
 // twice that at a 0.2 nm skin (~90 for 32).  A list that needs more stops the
 // integrator and is grown and rebuilt by the host (grow_tile_list).
 int row_cap_for(int cluster) { return cluster == 8 ? 384 : 192; }
+// Warps the row search of a rebuild should have at least: rows of a small
+// system are split until there are as many.
+constexpr long long kRowTasks = 8192;
 // the exact stage switches the screening network off once its running RMS
 // error exceeds this many kT (the plain barostat takes over)
 constexpr double kSurrogateMaxRmsKT = 1.5;
@@ -184,10 +187,6 @@ int alloc_tile_list(mdb_engine* e) {
   if ((st = alloc(e, "tiles", d.tiles, n))) return st;
   if ((st = alloc(e, "tile masks", d.masks, n * words))) return st;
   if ((st = alloc(e, "tile image shifts", d.tile_shift, n))) return st;
-  if ((st = alloc(e, "raw tiles", d.raw_tiles, n))) return st;
-  if ((st = alloc(e, "raw tile masks", d.raw_masks, n * words))) return st;
-  if ((st = alloc(e, "raw tile shifts", d.raw_shift, n))) return st;
-  if ((st = alloc(e, "tile survives", d.tile_alive, n))) return st;
   if (d.inner) {
     if ((st = alloc(e, "inner tiles", d.in_tiles, n))) return st;
     if ((st = alloc(e, "inner tile masks", d.in_masks, n * words))) return st;
@@ -261,6 +260,9 @@ void fill_box(const HostSystem& h, SysDev& S, bool keep_shift) {
   double widths[3];
   perpendicular_widths(B, widths);
   S.min_width = float(std::min({widths[0], widths[1], widths[2]}));
+  // a rectangular cell's nearest image is the one the reduction finds
+  const double spare = 0.5 * std::min({widths[0], widths[1], widths[2]}) - std::sqrt(double(S.list2));
+  S.one_image2 = S.triclinic ? float(spare > 0 ? spare * spare * (1 - 1e-5) : 0.0) : 3.0e38f;
   // cells narrower than cutoff + list radius + 1 nm flag most tiles per-pair
   S.prune_per_pair = S.min_width < std::sqrt(S.cut2) + std::sqrt(S.list2) + 1.0f ? 1 : 0;
   // Pair coordinates: the folded extent plus one box stays below 2^31.
@@ -300,6 +302,10 @@ int check_device_status(mdb_engine* e) {
     // the list kernel's grid barrier gave up: its count holds the blocks that
     // arrived; clear it and the bit so the next list build starts afresh
     CUDA_TRY(e, cudaMemset(e->d.list_barrier, 0, 2 * sizeof(unsigned int)));
+    // and what the phases it cut short would have cleared
+    CUDA_TRY(e, cudaMemset(e->d.cell_cnt, 0, sizeof(int) * size_t(std::max(1, e->d.n_cells))));
+    CUDA_TRY(e, cudaMemset(e->d.chunk_cnt, 0, sizeof(int) * size_t(std::max(1, e->d.n_chunks))));
+    CUDA_TRY(e, cudaMemset(e->d.list_ticket, 0, sizeof(int)));
     for (int& f : flags) f &= ~kErrTimeout;
     CUDA_TRY(e, cudaMemcpy(e->d.err, flags.data(), sizeof(int) * e->d.S, cudaMemcpyHostToDevice));
     request_rebuild(e, -1);
@@ -313,8 +319,8 @@ int check_device_status(mdb_engine* e) {
 // the phase kernels one by one.
 void list_kernels(mdb_engine* e, cudaStream_t st) {
   if (!(e->coop_list && launch_list(e->d, st))) {
+    launch_prune_references(e->d, st);
     launch_rebuild_sort(e->d, st);
-    launch_wrap(e->d, st);
     launch_rebuild_tiles(e->d, st);
   }
   launch_inner_prune(e->d, st);
@@ -406,8 +412,8 @@ int grow_tile_list(mdb_engine* e) {
   if (total > std::numeric_limits<int>::max()) return fail(e, MDB_ERR_CAPACITY, "the tile list cannot grow further");
   for (auto& g : e->graphs) cudaGraphExecDestroy(g.second);
   e->graphs.clear();
-  for (void* p : {(void*)d.tiles, (void*)d.masks, (void*)d.tile_shift, (void*)d.raw_tiles, (void*)d.raw_masks,
-                  (void*)d.raw_shift, (void*)d.tile_alive, (void*)d.in_tiles, (void*)d.in_masks, (void*)d.in_shift})
+  for (void* p : {(void*)d.tiles, (void*)d.masks, (void*)d.tile_shift, (void*)d.in_tiles, (void*)d.in_masks,
+                  (void*)d.in_shift})
     release(e, p);
   d.tile_cap_total = int(total);
   if (const int st = alloc_tile_list(e)) return st;
@@ -491,7 +497,7 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   e->baro.resize(n);
   std::vector<long long> px, py, pz;
   std::vector<float> vx, vy, vz, invm;
-  std::vector<int> atom_sys, slot_sys, block_sys, cell_sys, cell_map;
+  std::vector<int> atom_sys, slot_sys, block_sys, cell_sys, cell_map, chunk_sys;
   std::vector<float4> prm_atom;
   std::vector<int2> excl;
   std::vector<int> excl_sys;
@@ -606,6 +612,8 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
     for (int k = 0; k < S.n_slots; ++k) slot_sys.push_back(s);
     for (int k = 0; k < S.n_blocks; ++k) block_sys.push_back(s);
     for (int k = 0; k < S.n_cells; ++k) cell_sys.push_back(s);
+    S.chunk_off = int(chunk_sys.size());
+    chunk_sys.resize(chunk_sys.size() + (S.n_cells + kCellChunk - 1) / kCellChunk, s);
     const std::vector<int> mm = cell_order_map(S.cdim);
     cell_map.insert(cell_map.end(), mm.begin(), mm.end());
 
@@ -787,26 +795,44 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
     d.sb_hi = d.bb_hi;
   }
 
-  TRY(alloc(e, "tile row count", d.tile_cnt, blocks));
-  TRY(alloc(e, "tile row start", d.tile_start, blocks));
+  {
+    // the longest row segments that still give the row search kRowTasks warps
+    // (half a row's segments lie below its diagonal)
+    int longest = 1;
+    for (const SysDev& S : e->sd) longest = std::max(longest, S.n_slots / 32);
+    auto segments = [&](const SysDev& S, int p) { return (S.n_slots / 32 + p - 1) / p; };
+    d.row_supers = longest;
+    while (d.row_supers > 8) {
+      long long tasks = 0;
+      for (const SysDev& S : e->sd) tasks += (long long)S.n_blocks * (segments(S, d.row_supers) + 1) / 2;
+      if (tasks >= kRowTasks) break;
+      d.row_supers = std::max(8, (d.row_supers + 1) / 2);
+    }
+    d.row_segments = (longest + d.row_supers - 1) / d.row_supers;
+  }
+  TRY(alloc(e, "tile row count", d.tile_cnt, size_t(blocks) * d.row_segments));
+  TRY(alloc(e, "tile row start", d.tile_start, size_t(blocks) * d.row_segments));
   TRY(upload(e, "block system", tmp_i, block_sys));
   d.block_sys = tmp_i;
   TRY(alloc(e, "cell count", d.cell_cnt, cells));
   TRY(alloc(e, "cell start", d.cell_start, cells));
-  TRY(alloc(e, "cell cursor", d.cell_cur, cells));
+  TRY(alloc(e, "cell arrival", d.cell_arrival, atoms));
+  TRY(alloc(e, "cell chunk count", d.chunk_cnt, chunk_sys.size()));
+  TRY(upload(e, "cell chunk system", tmp_i, chunk_sys));
+  d.chunk_sys = tmp_i;
+  d.n_chunks = int(chunk_sys.size());
   TRY(upload(e, "cell system", tmp_i, cell_sys));
   d.cell_sys = tmp_i;
   TRY(upload(e, "cell order map", tmp_i, cell_map));
   d.cell_map = tmp_i;
   if (const int st_ = alloc_tile_list(e)) return st_;
-  TRY(alloc(e, "surviving tiles per row", d.row_alive, blocks));
-  TRY(alloc(e, "surviving tiles start", d.alive_start, blocks));
   TRY(alloc(e, "fold translations", d.fold, slots));
   TRY(alloc(e, "inner prune flag", d.prune_flag, n));
   TRY(alloc(e, "inner prune now", d.prune_now, n));
   TRY(alloc(e, "any inner prune", d.any_prune, 1));
   TRY(alloc(e, "inner prune count", d.prune_count, n));
   TRY(alloc(e, "inner prune ticket", d.inner_ticket, 1));
+  TRY(alloc(e, "list ticket", d.list_ticket, 1));
   if (d.inner) {
     TRY(alloc(e, "inner tile count", d.in_count, n));
     TRY(alloc(e, "inner tile prefix", d.in_prefix, n + 1));
@@ -966,7 +992,6 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   if (const int st = request_rebuild(e, -1)) return st;
   for (int attempt = 0;; ++attempt) {
     launch_rebuild_sort(e->d, e->s0);
-    launch_wrap(e->d, e->s0);
     launch_rebuild_tiles(e->d, e->s0);
     launch_inner_prune(e->d, e->s0);
     CUDA_TRY(e, cudaGetLastError());
@@ -1638,12 +1663,12 @@ int run(mdb_engine* e, int64_t steps) {
 bool bad_system(const mdb_engine* e, int32_t s) { return !e || s < 0 || s >= int32_t(e->hs.size()); }
 
 // Kernels one graph-replayed step launches: the list kernels (one cooperative
-// launch, or 5 sort + 1 wrap + 6 tile-list kernels, 3 more when rebuilds
-// prune), the inner-list kernel, PME (spread, 3 transform passes or 5 without
+// launch, or 4 sort + 3 tile-list kernels, one more with an inner list), the
+// inner-list kernel, PME (spread, 3 transform passes or 5 without
 // the plane kernels, gather), listed, nonbonded, integrator.
 int launches_per_step(const mdb_engine* e) {
   const Dev& d = e->d;
-  return (e->coop_list ? 1 : 5 + 1 + 6 + (d.prune ? 3 : 0)) + (d.inner ? 1 : 0) +
+  return (e->coop_list ? 1 : 4 + 3 + (d.inner ? 1 : 0)) + (d.inner ? 1 : 0) +
          (d.n_fft_z ? (d.fft_planes ? 5 : 7) : 0) +
          (d.n_bonds + d.n_angles + d.n_torsions + d.n_exceptions + d.n_restraints > 0 ? 1 : 0) + 1 + 1;
 }

@@ -4,13 +4,14 @@
 // Replaces the reference's wrap + counting-sort cell list + sort_cells
 // (src/gpu/kernels/cell-list.wgsl:140-331) and its three-pass Verlet list
 // (nonbonded-pairs.wgsl:412-497) with a B200-shaped design:
-//   * atoms are sorted along a Morton curve of ~0.3 nm fractional cells, so 32
+//   * atoms are sorted along a Hilbert curve of ~0.25 nm fractional cells, so 32
 //     consecutive slots form a compact cluster (a "block");
 //   * the list holds block pairs (tiles) whose bounding boxes come within
 //     cutoff + skin, plus one 32-bit interaction mask per tile row that removes
 //     exclusions, padding and the lower triangle of diagonal tiles;
 //   * the order inside a cell is ascending atom index, written by rank rather
-//     than by atomics, so two runs build bit-identical lists.
+//     than by atomics, so two runs hold the same tiles (their rows in any
+//     order, which the pair kernel's sums do not depend on).
 // A rebuild happens only when the integrator saw an atom move more than skin/2
 // (verlet.wgsl:57), decided on the device; every phase kernel returns at once
 // when no system asked for one.
@@ -60,75 +61,106 @@ __device__ __forceinline__ int cell_index(unsigned int frac, int dim) {
 
 // ---------------------------------------------------------------- phases --
 
-__device__ void phase_cells_clear(const Dev& d) {
-  for (int c = grid_stride_start(); c < d.n_cells; c += grid_stride()) {
-    if (!d.rebuild_now[d.cell_sys[c]]) continue;
-    d.cell_cnt[c] = 0;
-    d.cell_cur[c] = 0;
+// A rebuild is a chain of phases with a grid barrier (or a launch) between
+// them, so their number counts as much as their work: counters are cleared by
+// the phase that last reads them, an atom's place in its cell comes with the
+// count, everything written by slot is written where the slot is decided, and
+// a row is searched, pruned and written by one pass:
+//   cells assigned | scan | scatter | slots placed | boxes | rows | exclusions
+//
+// Every system about to be pruned only (no rebuild) gets its references here
+// too: its atoms' positions, its clusters' boxes at the pair coordinates the
+// integrator wrote, and an empty inner list.
+__device__ void phase_prune_references(const Dev& d) {
+  if (blockIdx.x == 0)
+    for (int s = threadIdx.x; s < d.S; s += blockDim.x)
+      if (d.prune_now[s] && !d.rebuild_now[s]) d.in_count[s] = 0;
+  // Lanes of a warp hold 32 consecutive slots (n_slots is a multiple of 32),
+  // one system's, so the branch below is warp-uniform.
+  for (int gs = grid_stride_start(); gs < d.n_slots; gs += grid_stride()) {
+    const int s = d.slot_sys[gs];
+    if (!d.prune_now[s] || d.rebuild_now[s]) continue;
+    const int a = d.order[gs];
+    const float inv = d.sys[s].pc_inv;
+    float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+    if (a >= 0) {
+      d.prx[a] = d.px[a];
+      d.pry[a] = d.py[a];
+      d.prz[a] = d.pz[a];
+      const int4 p = d.pc[gs];
+      lo[0] = hi[0] = p.x * inv;
+      lo[1] = hi[1] = p.y * inv;
+      lo[2] = hi[2] = p.z * inv;
+    }
+    const int C = d.cluster;
+    for (int o = C / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o, C));
+        hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o, C));
+      }
+    if ((gs & (C - 1)) == 0) {
+      d.cb_lo[gs / C] = make_float4(lo[0], lo[1], lo[2], 0.f);
+      d.cb_hi[gs / C] = make_float4(hi[0], hi[1], hi[2], 0.f);
+    }
   }
 }
 
+// Each atom's cell and its arrival number there; the cells' counts and the
+// counts of each chunk of kCellChunk consecutive cells.
 __device__ void phase_cells_assign(const Dev& d) {
-  for (int a = grid_stride_start(); a < d.n_atoms; a += grid_stride()) {
-    const int s = d.atom_sys[a];
+  const int lane = threadIdx.x & 31;
+  for (int a0 = grid_stride_start() - lane; a0 < d.n_atoms; a0 += grid_stride()) {
+    const int a = a0 + lane, s = a < d.n_atoms ? d.atom_sys[a] : 0;
+    int chunk = -1;
+    if (a < d.n_atoms && d.rebuild_now[s]) {
+      const SysDev& S = d.sys[s];
+      const Folded f = fold(S, d.px[a], d.py[a], d.pz[a]);
+      const int cx = cell_index(f.fa, S.cdim[0]), cy = cell_index(f.fb, S.cdim[1]),
+                cz = cell_index(f.fc, S.cdim[2]);
+      const int local = d.cell_map[S.cell_off + (cx * S.cdim[1] + cy) * S.cdim[2] + cz];
+      const int gc = S.cell_off + local;
+      d.cell_of[a] = gc;
+      d.cell_arrival[a] = atomicAdd(&d.cell_cnt[gc], 1);
+      chunk = S.chunk_off + local / kCellChunk;
+    }
+    // neighbours in index are neighbours in space: one atomic for the lanes of
+    // a chunk (one each took 96 us over the ensemble's 627k atoms, on 1,300 words)
+    const unsigned int same = __match_any_sync(0xffffffffu, chunk);
+    if (chunk >= 0 && lane == __ffs(same) - 1) atomicAdd(&d.chunk_cnt[chunk], __popc(same));
+  }
+}
+
+// The cells' starts: a block to a chunk, from the sum of the chunks before it
+// (a block to a system took 106 us over the 64,000 cells of a 100k-atom box).
+__device__ void phase_cells_scan(const Dev& d) {
+  static_assert(kCellChunk == 2 * kThreads, "two cells a thread");
+  __shared__ int part[kThreads / 32], before[kThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int ch = blockIdx.x; ch < d.n_chunks; ch += gridDim.x) {
+    const int s = d.chunk_sys[ch];
     if (!d.rebuild_now[s]) continue;
     const SysDev& S = d.sys[s];
-    const Folded f = fold(S, d.px[a], d.py[a], d.pz[a]);
-    const int cx = cell_index(f.fa, S.cdim[0]), cy = cell_index(f.fb, S.cdim[1]),
-              cz = cell_index(f.fc, S.cdim[2]);
-    const int local = d.cell_map[S.cell_off + (cx * S.cdim[1] + cy) * S.cdim[2] + cz];
-    const int gc = S.cell_off + local;
-    d.cell_of[a] = gc;
-    atomicAdd(&d.cell_cnt[gc], 1);
-  }
-}
-
-// Exclusive scan of `in[0..n)` into `out`, one block, in order.  Returns the
-// total.  Each warp owns a contiguous segment: pass one sums the segments
-// (coalesced), the block adds up the warps before each, pass two scans every
-// segment 32 elements at a time from its carry.
-__device__ int block_exclusive_scan(const int* in, int* out, int n) {
-  __shared__ int warp_total[kThreads / 32];
-  __shared__ int total;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int per = ((n + nw - 1) / nw + 31) / 32 * 32;
-  const int lo = min(n, warp * per), hi = min(n, lo + per);
-  int sum = 0;
-  for (int i = lo + lane; i < hi; i += 32) sum += in[i];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if (lane == 0) warp_total[warp] = sum;
-  __syncthreads();
-  int carry = 0;
-  for (int w = 0; w < warp; ++w) carry += warp_total[w];
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < nw; ++w) t += warp_total[w];
-    total = t;
-  }
-  for (int base = lo; base < hi; base += 32) {
-    const int i = base + lane;
-    const int v = i < hi ? in[i] : 0;
-    int x = v;
+    const int c = ch - S.chunk_off, first = c * kCellChunk + 2 * threadIdx.x;
+    int sum = 0;
+    for (int i = threadIdx.x; i < c; i += kThreads) sum += d.chunk_cnt[S.chunk_off + i];
+    const int v0 = first < S.n_cells ? d.cell_cnt[S.cell_off + first] : 0;
+    const int v1 = first + 1 < S.n_cells ? d.cell_cnt[S.cell_off + first + 1] : 0;
+    int x = v0 + v1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
-    if (i < hi) out[i] = carry + x - v;
-    carry += __shfl_sync(0xffffffffu, x, 31);
-  }
-  __syncthreads();
-  const int t = total;
-  __syncthreads();  // the shared words are free for the next call
-  return t;
-}
-
-__device__ void phase_cells_scan(const Dev& d) {
-  for (int s = blockIdx.x; s < d.S; s += gridDim.x) {
-    if (!d.rebuild_now[s]) continue;
-    const SysDev& S = d.sys[s];
-    block_exclusive_scan(d.cell_cnt + S.cell_off, d.cell_start + S.cell_off, S.n_cells);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 31) part[warp] = x;
+    if (lane == 0) before[warp] = sum;
+    __syncthreads();
+    int start = x - v0 - v1;
+    for (int w = 0; w < kThreads / 32; ++w) start += before[w] + (w < warp ? part[w] : 0);
+    if (first < S.n_cells) d.cell_start[S.cell_off + first] = start;
+    if (first + 1 < S.n_cells) d.cell_start[S.cell_off + first + 1] = start + v0;
+    __syncthreads();  // the shared words are free for the next chunk
   }
 }
 
@@ -136,129 +168,87 @@ __device__ void phase_cells_scatter(const Dev& d) {
   for (int a = grid_stride_start(); a < d.n_atoms; a += grid_stride()) {
     const int s = d.atom_sys[a];
     if (!d.rebuild_now[s]) continue;
-    const int gc = d.cell_of[a];
-    const int slot = d.cell_start[gc] + atomicAdd(&d.cell_cur[gc], 1);
-    d.tmp_order[d.sys[s].slot_off + slot] = a;
+    d.tmp_order[d.sys[s].slot_off + d.cell_start[d.cell_of[a]] + d.cell_arrival[a]] = a;
   }
 }
 
 // Ascending atom index inside each cell, by rank: the order is a function of
-// the positions alone, whatever order the scatter's atomics landed in
-// (cell-list.wgsl:319 sort_cells).
-__device__ void phase_cells_order(const Dev& d) {
+// the positions alone, whatever order the counts' atomics landed in
+// (cell-list.wgsl:319 sort_cells).  With its slot an atom gets everything kept
+// by slot: pair coordinates as int32 at 2^pc_shift per nm under the lattice
+// translation that folds it into the cell now (cell-list.wgsl:140 `wrap`;
+// three signed 10-bit counts, applied until the next rebuild, so the
+// coordinates move continuously and the tiles' lattice shifts stay valid),
+// parameters, and the positions the displacement tests measure against.
+__device__ void phase_place(const Dev& d) {
   for (int gs = grid_stride_start(); gs < d.n_slots; gs += grid_stride()) {
     const int s = d.slot_sys[gs];
     if (!d.rebuild_now[s]) continue;
     const SysDev& S = d.sys[s];
-    const int local = gs - S.slot_off;
-    if (local >= S.n_atoms) {
+    if (gs - S.slot_off >= S.n_atoms) {
       d.order[gs] = -1;
+      d.pc[gs] = make_int4(0, 0, 0, 0);
+      d.prm[gs] = make_float4(0.f, 0.f, 0.f, 0.f);
       continue;
     }
     const int a = d.tmp_order[gs];
     const int gc = d.cell_of[a];
+    const long long x = d.px[a], y = d.py[a], z = d.pz[a];
+    const float4 prm = d.prm_atom[a];
     const int st = d.cell_start[gc], cnt = d.cell_cnt[gc];
-    int r = 0;
+    int r = st;
     for (int k = 0; k < cnt; ++k) r += d.tmp_order[S.slot_off + st + k] < a;
-    d.order[S.slot_off + st + r] = a;
-    d.rank[a] = st + r;
-    d.islot[d.entry[a]] = S.slot_off + st + r;
-  }
-}
-
-// Every step, every system: pair coordinates of each slot as int32 at
-// 2^pc_shift per nm (cell-list.wgsl:140 `wrap`).  A rebuild folds each atom
-// into the cell and records the lattice translation it took (three signed
-// 10-bit counts); between rebuilds the same translation is applied, so the
-// coordinates move continuously (an atom leaves the cell by at most half the
-// skin before the next rebuild) and the tiles' lattice shifts stay valid.
-//
-// With an inner list, a system about to be pruned (or rebuilt) also takes its
-// atoms' positions as the new prune reference and empties its inner list.
-__device__ void phase_wrap(const Dev& d) {
-  if (d.inner && blockIdx.x == 0)
-    for (int s = threadIdx.x; s < d.S; s += blockDim.x)
-      if (d.rebuild_now[s] || d.prune_now[s]) d.in_count[s] = 0;
-  // Lanes of a warp hold 32 consecutive slots (n_slots is a multiple of 32),
-  // one system's, so the inner-list branch below is warp-uniform.
-  for (int gs = grid_stride_start(); gs < d.n_slots; gs += grid_stride()) {
-    const int a = d.order[gs];
-    const int s = d.slot_sys[gs];
-    const SysDev& S = d.sys[s];
-    int4 p = make_int4(0, 0, 0, 0);
-    if (a >= 0) {
-      if (d.inner && (d.rebuild_now[s] || d.prune_now[s])) {
-        d.prx[a] = d.px[a];
-        d.pry[a] = d.py[a];
-        d.prz[a] = d.pz[a];
-      }
-      long long na, nb, nc;
-      if (d.rebuild_now[s]) {
-        const Folded f = fold(S, d.px[a], d.py[a], d.pz[a]);
-        na = f.na;
-        nb = f.nb;
-        nc = f.nc;
-        d.fold[gs] = int((na & 1023) | ((nb & 1023) << 10) | ((nc & 1023) << 20));
-      } else {
-        unpack_fold(d.fold[gs], na, nb, nc);
-      }
-      p = pair_coordinate(S, d.px[a], d.py[a], d.pz[a], na, nb, nc);
-    }
-    d.pc[gs] = p;
-    if (d.inner && (d.rebuild_now[s] || d.prune_now[s])) {
-      // the cluster's bounding box at these coordinates, for the inner prune
-      const int C = d.cluster;
-      float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-      if (a >= 0) {
-        lo[0] = hi[0] = p.x * S.pc_inv;
-        lo[1] = hi[1] = p.y * S.pc_inv;
-        lo[2] = hi[2] = p.z * S.pc_inv;
-      }
-      for (int o = C / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o, C));
-          hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o, C));
-        }
-      if ((gs & (C - 1)) == 0) {
-        d.cb_lo[gs / C] = make_float4(lo[0], lo[1], lo[2], 0.f);
-        d.cb_hi[gs / C] = make_float4(hi[0], hi[1], hi[2], 0.f);
-      }
+    const int to = S.slot_off + r;
+    const Folded f = fold(S, x, y, z);
+    d.order[to] = a;
+    d.rank[a] = r;
+    d.islot[d.entry[a]] = to;
+    d.fold[to] = int((f.na & 1023) | ((f.nb & 1023) << 10) | ((f.nc & 1023) << 20));
+    d.pc[to] = pair_coordinate(S, x, y, z, f.na, f.nb, f.nc);
+    d.prm[to] = prm;
+    d.refx[a] = x;
+    d.refy[a] = y;
+    d.refz[a] = z;
+    if (d.inner) {
+      d.prx[a] = x;
+      d.pry[a] = y;
+      d.prz[a] = z;
     }
   }
 }
 
-// A group of C lanes per cluster (32/C clusters per warp): parameters in slot
-// order, the cluster's bounding box, and the reference positions the
-// displacement test measures against.  Every lane takes part in every
+// A group of C lanes per cluster (32/C clusters per warp): the cluster's
+// bounding box and its super-cluster's.  Every lane takes part in every
 // shuffle; only the writes depend on whether the cluster's system rebuilds.
+// The sort's counters are cleared for the next rebuild, the lists emptied.
 template <int C>
-__device__ void phase_tiles_blocks(const Dev& d) {
+__device__ void phase_boxes(const Dev& d) {
   constexpr int G = 32 / C;
   const int lane = threadIdx.x & 31, g = lane / C, l = lane & (C - 1);
   const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int c = grid_stride_start(); c < d.n_cells; c += grid_stride())
+    if (d.rebuild_now[d.cell_sys[c]]) d.cell_cnt[c] = 0;
+  for (int c = grid_stride_start(); c < d.n_chunks; c += grid_stride())
+    if (d.rebuild_now[d.chunk_sys[c]]) d.chunk_cnt[c] = 0;
+  if (blockIdx.x == 0)
+    for (int s = threadIdx.x; s < d.S; s += blockDim.x)
+      if (d.rebuild_now[s]) {
+        d.tile_need[s] = 0;
+        if (d.inner) d.in_count[s] = 0;
+      }
   for (int wb = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; wb * G < d.n_blocks; wb += warps) {
     const int b = wb * G + g;
     const bool valid = b < d.n_blocks;
     const int s = valid ? d.block_sys[b] : 0;
     const bool work = valid && d.rebuild_now[s];
-    const SysDev& S = d.sys[s];
+    const float inv = d.sys[s].pc_inv;
     const int gs = b * C + l;
-    const int a = work ? d.order[gs] : -1;
     float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
-    if (work) {
-      if (a >= 0) {
-        d.prm[gs] = d.prm_atom[a];
-        d.refx[a] = d.px[a];
-        d.refy[a] = d.py[a];
-        d.refz[a] = d.pz[a];
-        const int4 p = d.pc[gs];
-        lo[0] = hi[0] = p.x * S.pc_inv;
-        lo[1] = hi[1] = p.y * S.pc_inv;
-        lo[2] = hi[2] = p.z * S.pc_inv;
-      } else {
-        d.prm[gs] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+    if (work && d.order[gs] >= 0) {
+      const int4 p = d.pc[gs];
+      lo[0] = hi[0] = p.x * inv;
+      lo[1] = hi[1] = p.y * inv;
+      lo[2] = hi[2] = p.z * inv;
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k)
@@ -268,8 +258,13 @@ __device__ void phase_tiles_blocks(const Dev& d) {
         hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o, C));
       }
     if (work && l == 0) {
-      d.bb_lo[b] = make_float4(lo[0], lo[1], lo[2], 0.f);
-      d.bb_hi[b] = make_float4(hi[0], hi[1], hi[2], 0.f);
+      const float4 low = make_float4(lo[0], lo[1], lo[2], 0.f), high = make_float4(hi[0], hi[1], hi[2], 0.f);
+      d.bb_lo[b] = low;
+      d.bb_hi[b] = high;
+      if (d.inner) {
+        d.cb_lo[b] = low;
+        d.cb_hi[b] = high;
+      }
     }
     if (C < 32) {
       // the warp's 32/C clusters form one super-cluster (a system's clusters
@@ -289,42 +284,75 @@ __device__ void phase_tiles_blocks(const Dev& d) {
   }
 }
 
+// What the box tests of a row need of its system, in registers.
+struct Cell {
+  float b0, b3, b4, b6, b7, b8;  // the lattice, reduced form
+  float i0, i4, i8;              // reciprocals of its diagonal
+  float list2;
+  float one_image2;  // see S.one_image2
+};
+__device__ __forceinline__ Cell cell_of_system(const SysDev& S) {
+  return Cell{S.box_f[0], S.box_f[3], S.box_f[4], S.box_f[6], S.box_f[7], S.box_f[8],
+              S.inv_f[0], S.inv_f[4], S.inv_f[8], S.list2, S.one_image2};
+}
+
+// Centre separation and half-extents of two boxes, the separation reduced
+// sequentially against c, b, a (src/reference/forces/nonbonded.ts:241); the
+// counts taken off come back in n.
+struct BoxPair {
+  float dx, dy, dz, hx, hy, hz;
+};
+__device__ __forceinline__ BoxPair box_pair(const Cell& B, float4 li, float4 hi_, float4 lj, float4 hj, float* n) {
+  BoxPair p;
+  p.hx = 0.5f * (hi_.x - li.x) + 0.5f * (hj.x - lj.x);
+  p.hy = 0.5f * (hi_.y - li.y) + 0.5f * (hj.y - lj.y);
+  p.hz = 0.5f * (hi_.z - li.z) + 0.5f * (hj.z - lj.z);
+  p.dx = 0.5f * (lj.x + hj.x) - 0.5f * (li.x + hi_.x);
+  p.dy = 0.5f * (lj.y + hj.y) - 0.5f * (li.y + hi_.y);
+  p.dz = 0.5f * (lj.z + hj.z) - 0.5f * (li.z + hi_.z);
+  n[2] = rintf(p.dz * B.i8);
+  p.dx -= n[2] * B.b6; p.dy -= n[2] * B.b7; p.dz -= n[2] * B.b8;
+  n[1] = rintf(p.dy * B.i4);
+  p.dx -= n[1] * B.b3; p.dy -= n[1] * B.b4;
+  n[0] = rintf(p.dx * B.i0);
+  p.dx -= n[0] * B.b0;
+  return p;
+}
+
+__device__ __forceinline__ float gap2(float d, float h) {
+  const float g = fmaxf(fabsf(d) - h, 0.f);
+  return g * g;
+}
+
+// When every centre distance that could pass (list + both half-diagonals) is
+// below half the cell's narrowest width, the sequential reduction already
+// gives the minimum image, as it does for the reference's cutoff: in
+// one_image2, (half the width - list)^2, the bound on the half-diagonals'
+// square (without bound in a rectangular cell, where it always does).
+__device__ __forceinline__ bool one_image(const Cell& B, const BoxPair& p) {
+  return p.hx * p.hx + p.hy * p.hy + p.hz * p.hz < B.one_image2;
+}
+
 // Do two boxes of one system come within cutoff + skin under some periodic
 // image?  Box-to-box gap distance, minimised over images.  An empty
 // cluster's box is inverted (lo = +3e38, hi = -3e38): its gap is infinite.
-__device__ __forceinline__ bool boxes_near(const SysDev& S, float4 li, float4 hi_, float4 lj, float4 hj) {
-  const float hx = 0.5f * (hi_.x - li.x) + 0.5f * (hj.x - lj.x);
-  const float hy = 0.5f * (hi_.y - li.y) + 0.5f * (hj.y - lj.y);
-  const float hz = 0.5f * (hi_.z - li.z) + 0.5f * (hj.z - lj.z);
-  float dx = 0.5f * (lj.x + hj.x) - 0.5f * (li.x + hi_.x);
-  float dy = 0.5f * (lj.y + hj.y) - 0.5f * (li.y + hi_.y);
-  float dz = 0.5f * (lj.z + hj.z) - 0.5f * (li.z + hi_.z);
-  const float* B = S.box_f;
-  // sequential reduction c, b, a (src/reference/forces/nonbonded.ts:241)
-  const float kc = rintf(dz / B[8]);
-  dx -= kc * B[6]; dy -= kc * B[7]; dz -= kc * B[8];
-  const float kb = rintf(dy / B[4]);
-  dx -= kb * B[3]; dy -= kb * B[4];
-  dx -= rintf(dx / B[0]) * B[0];
-  // When every centre distance that could pass (list + both half-diagonals)
-  // is below half the cell's narrowest width, the sequential reduction above
-  // already gives the minimum image, as it does for the reference's cutoff.
-  const bool one_image = !S.triclinic || sqrtf(S.list2) + sqrtf(hx * hx + hy * hy + hz * hz) < 0.5f * S.min_width;
-  if (one_image) {
-    const float gx = fmaxf(fabsf(dx) - hx, 0.f), gy = fmaxf(fabsf(dy) - hy, 0.f), gz = fmaxf(fabsf(dz) - hz, 0.f);
-    return gx * gx + gy * gy + gz * gz < S.list2;
+// Images out of reach along one axis are not tried along the others (small
+// triclinic cells: 27 images a test otherwise).
+__device__ __forceinline__ bool boxes_near(const Cell& B, float4 li, float4 hi_, float4 lj, float4 hj) {
+  float n[3];
+  const BoxPair p = box_pair(B, li, hi_, lj, hj, n);
+  if (one_image(B, p)) return gap2(p.dx, p.hx) + gap2(p.dy, p.hy) + gap2(p.dz, p.hz) < B.list2;
+  for (int k = -1; k <= 1; ++k) {
+    const float z2 = gap2(p.dz + k * B.b8, p.hz);
+    if (!(z2 < B.list2)) continue;
+    for (int j = -1; j <= 1; ++j) {
+      const float y2 = z2 + gap2(p.dy + j * B.b4 + k * B.b7, p.hy);
+      if (!(y2 < B.list2)) continue;
+      for (int i = -1; i <= 1; ++i)
+        if (y2 + gap2(p.dx + i * B.b0 + j * B.b3 + k * B.b6, p.hx) < B.list2) return true;
+    }
   }
-  float best = 3.0e38f;
-  for (int k = -1; k <= 1; ++k)
-    for (int j = -1; j <= 1; ++j)
-      for (int i = -1; i <= 1; ++i) {
-        const float x = dx + i * B[0] + j * B[3] + k * B[6];
-        const float y = dy + j * B[4] + k * B[7];
-        const float z = dz + k * B[8];
-        const float gx = fmaxf(fabsf(x) - hx, 0.f), gy = fmaxf(fabsf(y) - hy, 0.f), gz = fmaxf(fabsf(z) - hz, 0.f);
-        best = fminf(best, gx * gx + gy * gy + gz * gz);
-      }
-  return best < S.list2;
+  return false;
 }
 
 // The lattice shift (in pair-coordinate units, applied to J) of the image
@@ -335,32 +363,21 @@ __device__ __forceinline__ bool boxes_near(const SysDev& S, float4 li, float4 hi
 // 2 (|h_I| + |h_J|) + list + cutoff reaches the cell's narrowest width (h the
 // half-diagonals), another image of some pair could come inside the cutoff,
 // and the pair kernel takes the minimum image per pair instead.
-__device__ __forceinline__ int4 tile_image(const SysDev& S, float4 li, float4 hi_, float4 lj, float4 hj) {
-  float dx = 0.5f * (lj.x + hj.x) - 0.5f * (li.x + hi_.x);
-  float dy = 0.5f * (lj.y + hj.y) - 0.5f * (li.y + hi_.y);
-  float dz = 0.5f * (lj.z + hj.z) - 0.5f * (li.z + hi_.z);
-  const float* B = S.box_f;
-  const float kc = rintf(dz / B[8]);
-  dx -= kc * B[6]; dy -= kc * B[7]; dz -= kc * B[8];
-  const float kb = rintf(dy / B[4]);
-  dx -= kb * B[3]; dy -= kb * B[4];
-  const float ka = rintf(dx / B[0]);
-  dx -= ka * B[0];
-  int na = -int(ka), nb = -int(kb), nc = -int(kc);
-  const float hx = 0.5f * (hi_.x - li.x) + 0.5f * (hj.x - lj.x);
-  const float hy = 0.5f * (hi_.y - li.y) + 0.5f * (hj.y - lj.y);
-  const float hz = 0.5f * (hi_.z - li.z) + 0.5f * (hj.z - lj.z);
-  if (S.triclinic && sqrtf(S.list2) + sqrtf(hx * hx + hy * hy + hz * hz) >= 0.5f * S.min_width) {
+__device__ __forceinline__ int4 tile_image(const SysDev& S, const Cell& B, float4 li, float4 hi_, float4 lj, float4 hj) {
+  float n[3];
+  const BoxPair p = box_pair(B, li, hi_, lj, hj, n);
+  int na = -int(n[0]), nb = -int(n[1]), nc = -int(n[2]);
+  if (!one_image(B, p)) {
     float best = 3.0e38f;
     int bi = 0, bj = 0, bk = 0;
-    for (int k = -1; k <= 1; ++k)
-      for (int j = -1; j <= 1; ++j)
+    for (int k = -1; k <= 1; ++k) {
+      const float z2 = gap2(p.dz + k * B.b8, p.hz);
+      if (!(z2 < best)) continue;
+      for (int j = -1; j <= 1; ++j) {
+        const float y2 = z2 + gap2(p.dy + j * B.b4 + k * B.b7, p.hy);
+        if (!(y2 < best)) continue;
         for (int i = -1; i <= 1; ++i) {
-          const float x = dx + i * B[0] + j * B[3] + k * B[6];
-          const float y = dy + j * B[4] + k * B[7];
-          const float z = dz + k * B[8];
-          const float gx = fmaxf(fabsf(x) - hx, 0.f), gy = fmaxf(fabsf(y) - hy, 0.f), gz = fmaxf(fabsf(z) - hz, 0.f);
-          const float g = gx * gx + gy * gy + gz * gz;
+          const float g = y2 + gap2(p.dx + i * B.b0 + j * B.b3 + k * B.b6, p.hx);
           if (g < best) {
             best = g;
             bi = i;
@@ -368,22 +385,20 @@ __device__ __forceinline__ int4 tile_image(const SysDev& S, float4 li, float4 hi
             bk = k;
           }
         }
+      }
+    }
     na += bi;
     nb += bj;
     nc += bk;
   }
-  // wrapping 32-bit arithmetic: the pair kernel adds this to a coordinate and
-  // subtracts another; the result, a separation inside the cutoff, fits
-  const unsigned int sx = unsigned(na) * unsigned(S.pc_box[0]) + unsigned(nb) * unsigned(S.pc_box[3]) +
-                          unsigned(nc) * unsigned(S.pc_box[6]);
-  const unsigned int sy = unsigned(nb) * unsigned(S.pc_box[4]) + unsigned(nc) * unsigned(S.pc_box[7]);
-  const unsigned int sz = unsigned(nc) * unsigned(S.pc_box[8]);
   const float ei = 0.5f * sqrtf((hi_.x - li.x) * (hi_.x - li.x) + (hi_.y - li.y) * (hi_.y - li.y) +
                                 (hi_.z - li.z) * (hi_.z - li.z));
   const float ej = 0.5f * sqrtf((hj.x - lj.x) * (hj.x - lj.x) + (hj.y - lj.y) * (hj.y - lj.y) +
                                 (hj.z - lj.z) * (hj.z - lj.z));
   const bool per_pair = 2.f * (ei + ej) + sqrtf(S.list2) + sqrtf(S.cut2) >= S.min_width;
-  return make_int4(int(sx), int(sy), int(sz), tile_flags(per_pair, na, nb, nc));
+  // wrapping 32-bit arithmetic: the pair kernel adds the shift to a coordinate
+  // and subtracts another; the result, a separation inside the cutoff, fits
+  return tile_shift_for(S, tile_flags(per_pair, na, nb, nc));
 }
 
 // Position of the k-th (from 0) set bit of m, or -1.
@@ -392,235 +407,239 @@ __device__ __forceinline__ int nth_set_bit(unsigned int m, int k) {
   return m ? __ffs(m) - 1 : -1;
 }
 
-// Tiles of row I, in ascending J.  The search is two-level: the 32-slot
-// super-cluster of J (kSub = 32 / C clusters) must come near I's cluster
-// before the clusters inside it are tested, 32 / kSub super-clusters to a
-// pass of the warp, and every near tile is written by its own lane.  The
-// count pass (WRITE false) sizes the rows; after the scan the fill pass
-// (WRITE true) writes them at their place in the dense list.  Rows vary a lot:
-// a cluster that straddles a jump of the space-filling curve (where it leaves
-// the sort grid and comes back) has a large box and a long row.
-template <int C, bool WRITE>
-__device__ void phase_tiles_find(const Dev& d) {
-  constexpr int kSub = 32 / C;         // clusters per super-cluster
-  constexpr int kBatch = 32 / kSub;    // super-clusters per pass
-  constexpr int kWords = C * C / 32;   // mask words per tile
-  constexpr unsigned kRowAll = C == 32 ? 0xffffffffu : ((1u << C) - 1u);
+// Row `r` of the mask of tile (I, J) (indices within their system): every pair
+// of atoms, without padding and, on the diagonal, one half.
+template <int C>
+__device__ __forceinline__ unsigned int valid_row(const SysDev& S, int I, int J, int r) {
+  constexpr unsigned kAll = C == 32 ? 0xffffffffu : ((1u << C) - 1u);
+  const int nj = max(0, min(C, S.n_atoms - J * C));
+  unsigned int row = nj >= C ? kAll : ((1u << nj) - 1u);
+  if (J == I) row &= r == C - 1 ? 0u : ((kAll << (r + 1)) & kAll);
+  return I * C + r < S.n_atoms ? row : 0u;
+}
+
+// The candidates of row I among super-clusters [sI, sEnd), in ascending J: the
+// 32-slot super-cluster of J (kSub = 32 / C clusters) must come near I's
+// cluster before the clusters inside it are tested, 32 / kSub super-clusters to
+// a pass of the warp.
+// `batch(J)` is called by the whole warp, J < 0 in lanes without a candidate.
+template <int C, class Batch>
+__device__ __forceinline__ void walk_row(const Dev& d, const Cell& B, int I, float4 li, float4 hi_, int sI, int sEnd,
+                                         Batch batch) {
+  constexpr int kSub = 32 / C, kBatch = 32 / kSub;
   const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  const unsigned below = (1u << lane) - 1u;
-  for (int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; I < d.n_blocks; I += warps) {
-    const int s = d.block_sys[I];
-    if (!d.rebuild_now[s]) continue;
-    const SysDev& S = d.sys[s];
-    // the row's tiles go to [base, base + cap) of the dense list
-    const long long base = static_cast<long long>(S.tile_off) + (WRITE ? d.tile_start[I] : 0);
-    const int cap = WRITE ? min(d.tile_cnt[I], S.tile_cap - d.tile_start[I]) : 0;
-    const int sI = I / kSub, sEnd = (S.block_off + S.n_blocks) / kSub;
-    const float4 li = d.bb_lo[I], hi_ = d.bb_hi[I];
-    const int Il = I - S.block_off;
-    int count = 0;
-    for (int J0 = sI; J0 < sEnd; J0 += 32) {
-      const int SJ = J0 + lane;
-      const bool near = SJ < sEnd && boxes_near(S, li, hi_, d.sb_lo[SJ], d.sb_hi[SJ]);
-      const unsigned int supers = __ballot_sync(0xffffffffu, near);
-      if (C == 32) {
-        // no super level: the boxes tested are the clusters themselves, and a
-        // 32x32 tile's mask is one word per row, so every lane writes its row
-        const unsigned int found = __ballot_sync(0xffffffffu, near && SJ >= I);
-        unsigned int f = found;
-        while (f) {
-          const int src = __ffs(f) - 1;
-          f &= f - 1;
-          const int Jt = J0 + src;
-          const int pos = count + __popc(found & ((1u << src) - 1u));
-          if (WRITE && pos < cap) {
-            if (lane == 0) {
-              (d.prune ? d.raw_tiles : d.tiles)[base + pos] = make_int2(I, Jt);
-              (d.prune ? d.raw_shift : d.tile_shift)[base + pos] = tile_image(S, li, hi_, d.bb_lo[Jt], d.bb_hi[Jt]);
-            }
-            const int Jl = Jt - S.block_off;
-            const int nj = max(0, min(C, S.n_atoms - Jl * C));
-            unsigned int valid = nj >= C ? kRowAll : ((1u << nj) - 1u);
-            if (Jt == I) valid &= lane == C - 1 ? 0u : (kRowAll << (lane + 1));
-            if (Il * C + lane >= S.n_atoms) valid = 0u;
-            (d.prune ? d.raw_masks : d.masks)[(base + pos) * kWords + lane] = valid;
-          }
-        }
-        count += __popc(found);
-        continue;
-      }
-      unsigned int rest = supers;
-      while (rest) {
-        // lanes k * kSub .. k * kSub + kSub - 1 take the k-th remaining near super-cluster
-        const int k = lane / kSub, sub = lane % kSub;
-        const int nth = nth_set_bit(rest, k);
-        const int J = nth >= 0 ? (J0 + nth) * kSub + sub : -1;
-        const bool tile = J >= I && boxes_near(S, li, hi_, d.bb_lo[J], d.bb_hi[J]);
-        const unsigned int found = __ballot_sync(0xffffffffu, tile);
-        const int at = count + __popc(found & below);
-        if (WRITE && tile && at < cap) {
-          (d.prune ? d.raw_tiles : d.tiles)[base + at] = make_int2(I, J);
-          (d.prune ? d.raw_shift : d.tile_shift)[base + at] = tile_image(S, li, hi_, d.bb_lo[J], d.bb_hi[J]);
-          const int Jl = J - S.block_off;
-          const int nj = max(0, min(C, S.n_atoms - Jl * C));
-          const unsigned int cols = nj >= C ? kRowAll : ((1u << nj) - 1u);
-          unsigned int words[kWords];
-#pragma unroll
-          for (int w = 0; w < kWords; ++w) words[w] = 0u;
-#pragma unroll
-          for (int r = 0; r < C; ++r) {
-            unsigned int row = Il * C + r < S.n_atoms ? cols : 0u;
-            if (J == I) row &= r == C - 1 ? 0u : ((kRowAll << (r + 1)) & kRowAll);
-            words[(r * C) >> 5] |= row << ((r * C) & 31);
-          }
-#pragma unroll
-          unsigned int* masks = d.prune ? d.raw_masks : d.masks;
-#pragma unroll
-          for (int w = 0; w < kWords; ++w) masks[(base + at) * kWords + w] = words[w];
-        }
-        count += __popc(found);
-        for (int b = 0; b < kBatch && rest; ++b) rest &= rest - 1;  // the super-clusters this pass took
-      }
+  for (int J0 = sI; J0 < sEnd; J0 += 32) {
+    const int SJ = J0 + lane;
+    const bool near = SJ < sEnd && boxes_near(B, li, hi_, d.sb_lo[SJ], d.sb_hi[SJ]);
+    if (C == 32) {
+      batch(near ? SJ : -1);  // no super level: the boxes tested are the clusters themselves
+      continue;
     }
-    if (!WRITE && lane == 0) {
-      d.tile_cnt[I] = count;
-      d.row_alive[I] = 0;
+    unsigned int rest = __ballot_sync(0xffffffffu, near);
+    while (rest) {
+      // lanes k * kSub .. k * kSub + kSub - 1 take the k-th remaining near super-cluster
+      const int nth = nth_set_bit(rest, lane / kSub);
+      const int J = nth >= 0 ? (J0 + nth) * kSub + lane % kSub : -1;
+      batch(J >= I && boxes_near(B, li, hi_, d.bb_lo[J], d.bb_hi[J]) ? J : -1);
+      for (int b = 0; b < kBatch && rest; ++b) rest &= rest - 1;  // the super-clusters this pass took
     }
   }
 }
 
-__device__ void phase_tiles_scan(const Dev& d) {
-  for (int s = blockIdx.x; s < d.S; s += gridDim.x) {
-    if (!d.rebuild_now[s]) continue;
-    const SysDev& S = d.sys[s];
-    const int total = block_exclusive_scan(d.tile_cnt + S.block_off, d.tile_start + S.block_off, S.n_blocks);
-    if (threadIdx.x == 0) {
-      // a list that needs more tiles than the system's capacity is cut there,
-      // and the engine's halt word stops the integrator, so no step runs on
-      // the cut list: the host grows the capacity to `tile_need` and rebuilds
-      // before it runs the remaining steps
-      d.tile_need[s] = total;
-      if (total > S.tile_cap) {
-        atomicOr(&d.err[s], kErrTileCapacity);
-        atomicExch(d.halt, 1);
-      }
-      d.tile_count[s] = total < S.tile_cap ? total : S.tile_cap;
-    }
-  }
-}
-
-// Drop the tiles whose atoms are all farther apart than cutoff + skin (the
-// box test is conservative: about a fifth of 8x8 tiles have no pair inside).
-// Tiles are spread over every warp, 32/C at a time, one group of C lanes per
-// tile running the pair kernel's rotation on distances only; the verdict goes
-// to tile_alive and the row's survivor count.
+// Which of a warp's candidate tiles of row I (lane's J and shift; `here`: the
+// lanes that have one) hold a pair closer than reach: 32/C tiles at a time, C
+// lanes to a tile, the pair kernel's rotation on distances only.  `pi` is the
+// row's atom lane mod C.
 template <int C>
-__device__ void phase_tiles_prune(const Dev& d) {
+__device__ __forceinline__ unsigned int tiles_with_pair(const Dev& d, const SysDev& S, int I, int4 pi, int J, int4 sh,
+                                                        unsigned int here, float reach2) {
   constexpr int G = 32 / C;
-  const int lane = threadIdx.x & 31, g = lane / C, l = lane & (C - 1);
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int src = (l + 1) & (C - 1);
   constexpr unsigned kGroup = C == 32 ? 0xffffffffu : ((1u << C) - 1u);
-  for (int s = 0; s < d.S; ++s) {
-    if (!d.rebuild_now[s]) continue;
-    const SysDev& S = d.sys[s];
-    const int n = d.tile_count[s];
-    const float inv = S.pc_inv, list2 = S.list2 * (1.0f + 1e-5f);
-    for (int b = warp * G; b < n; b += warps * G) {
-      const int t = b + g;
-      const bool active = t < n;
-      const long long ti = S.tile_off + (active ? t : 0);
-      const int2 tile = d.raw_tiles[ti];
-      const int4 sh = d.raw_shift[ti];
-      unsigned int mask = active ? row_bits<C>(d.raw_masks, ti, l) : 0u;
-      mask = (mask >> l) | (mask << ((C - l) & (C - 1)));  // bit k <-> j = l + k (mod C)
-      const int4 pi = d.pc[tile.x * C + l];
-      int4 pj = d.pc[tile.y * C + l];
-      if (!tile_per_pair(sh.w)) {
-        pj.x = int(unsigned(pj.x) + unsigned(sh.x));
-        pj.y = int(unsigned(pj.y) + unsigned(sh.y));
-        pj.z = int(unsigned(pj.z) + unsigned(sh.z));
-      }
-      bool hit = false;
-#pragma unroll
-      for (int k = 0; k < C; ++k) {
-        int dx = int(unsigned(pj.x) - unsigned(pi.x)), dy = int(unsigned(pj.y) - unsigned(pi.y)),
-            dz = int(unsigned(pj.z) - unsigned(pi.z));
-        if (tile_per_pair(sh.w)) {
-          if (S.triclinic) min_image<true>(S, dx, dy, dz);
-          else min_image<false>(S, dx, dy, dz);
-        }
-        const float rx = dx * inv, ry = dy * inv, rz = dz * inv;
-        hit |= ((mask >> k) & 1u) && rx * rx + ry * ry + rz * rz < list2;
-        pj.x = __shfl_sync(0xffffffffu, pj.x, src, C);
-        pj.y = __shfl_sync(0xffffffffu, pj.y, src, C);
-        pj.z = __shfl_sync(0xffffffffu, pj.z, src, C);
-      }
-      const unsigned int hits = __ballot_sync(0xffffffffu, hit);
-      const bool alive = ((hits >> (g * C)) & kGroup) != 0u;
-      if (active && l == 0) {
-        d.tile_alive[ti] = alive ? 1 : 0;
-        if (alive) atomicAdd(&d.row_alive[tile.x], 1);
+  const int lane = threadIdx.x & 31, g = lane / C, l = lane & (C - 1), src = (l + 1) & (C - 1);
+  const float inv = S.pc_inv;
+  unsigned int keep = 0u;
+  // the next group's atoms are on their way while one group is tested
+  struct Group {
+    int J, w;
+    int4 pj;
+  };
+  auto fetch = [&](int t0) {
+    Group r;
+    const int from = (t0 + g) & 31;
+    r.J = t0 < 32 ? __shfl_sync(0xffffffffu, J, from) : -1;
+    const int sx = __shfl_sync(0xffffffffu, sh.x, from), sy = __shfl_sync(0xffffffffu, sh.y, from),
+              sz = __shfl_sync(0xffffffffu, sh.z, from);
+    r.w = __shfl_sync(0xffffffffu, sh.w, from);
+    r.pj = make_int4(0, 0, 0, 0);
+    if (r.J >= 0) {
+      r.pj = d.pc[r.J * C + l];
+      if (!tile_per_pair(r.w)) {
+        r.pj.x = int(unsigned(r.pj.x) + unsigned(sx));
+        r.pj.y = int(unsigned(r.pj.y) + unsigned(sy));
+        r.pj.z = int(unsigned(r.pj.z) + unsigned(sz));
       }
     }
+    return r;
+  };
+  Group next = fetch(0);
+  const int end = 32 - __clz(here);  // no candidate from here on
+  for (int t0 = 0; t0 < end; t0 += G) {
+    const Group now = next;
+    next = fetch(t0 + G);
+    if (!__any_sync(0xffffffffu, now.J >= 0)) continue;
+    const bool per_pair = now.J >= 0 && tile_per_pair(now.w);
+    unsigned int mask = now.J >= 0 ? valid_row<C>(S, I - S.block_off, now.J - S.block_off, l) : 0u;
+    int4 pj = now.pj;
+    // bit k <-> j = l + k (mod C)
+    mask = C == 32 ? __funnelshift_r(mask, mask, l) : (mask >> l) | (mask << ((C - l) & (C - 1)));
+    const bool images = __any_sync(0xffffffffu, per_pair);
+    bool hit = false;
+#pragma unroll 8
+    for (int k = 0; k < C; ++k) {
+      int dx = int(unsigned(pj.x) - unsigned(pi.x)), dy = int(unsigned(pj.y) - unsigned(pi.y)),
+          dz = int(unsigned(pj.z) - unsigned(pi.z));
+      if (images) {
+        // (a tile that needs none is left as it is: see the pair kernel)
+        if (S.triclinic) min_image<true>(S, dx, dy, dz);
+        else min_image<false>(S, dx, dy, dz);
+      }
+      const float rx = dx * inv, ry = dy * inv, rz = dz * inv;
+      hit |= ((mask >> k) & 1u) && rx * rx + ry * ry + rz * rz < reach2;
+      pj.x = __shfl_sync(0xffffffffu, pj.x, src, C);
+      pj.y = __shfl_sync(0xffffffffu, pj.y, src, C);
+      pj.z = __shfl_sync(0xffffffffu, pj.z, src, C);
+    }
+    const unsigned int hits = __ballot_sync(0xffffffffu, hit);
+#pragma unroll
+    for (int q = 0; q < G; ++q)
+      if ((hits >> (q * C)) & kGroup) keep |= 1u << (t0 + q);
   }
+  return keep;
 }
 
-__device__ void phase_tiles_rescan(const Dev& d) {
-  for (int s = blockIdx.x; s < d.S; s += gridDim.x) {
-    if (!d.rebuild_now[s]) continue;
-    const SysDev& S = d.sys[s];
-    const int total = block_exclusive_scan(d.row_alive + S.block_off, d.alive_start + S.block_off, S.n_blocks);
-    if (threadIdx.x == 0) d.tile_count[s] = total;
-  }
-}
+// A warp to a segment of a row (row_supers super-clusters of J: whole rows in
+// large engines, fewer where rows alone would leave warps idle; row_segments
+// to a row): its candidates are found once, into shared memory; with pruning, those whose atoms are all farther apart than cutoff + skin are
+// dropped (the box test is conservative: about a fifth of 8x8 tiles have no
+// pair inside); one atomic reserves its place in its system's list, and
+// the tiles are written there, in ascending J.  Rows land in any order: the
+// pair kernel's sums do not depend on it (per-tile f32 partials become int64
+// fixed point).  A row longer than the buffer (a cluster that straddles a jump
+// of the space-filling curve has a large box and may reach half the system)
+// is walked again instead.  Measured alone against a count pass, a scan, a fill
+// pass that tested every box again, and prune, scan and copy passes: 2,652
+// atoms 83 -> 23 us, 12k 115 -> 77, 27k (no pruning) 164 -> 70, 100k 316 -> 206,
+// the 64-system ensemble 1.52 -> 0.71 ms.  Reserving by block (one atomic for its
+// eight warps, between two barriers) was slower: 12k 119 us, the warps wait for
+// the longest of the eight.
+constexpr int kRowBuffer = 512;
 
-// Warp per row: the row's surviving tiles, in order, into the list the pair
-// kernel reads; the row's start and count follow them.
 template <int C>
-__device__ void phase_tiles_compact(const Dev& d) {
+__device__ void phase_rows(const Dev& d, int (*buffers)[kRowBuffer]) {
   constexpr int kWords = C * C / 32;
   const int lane = threadIdx.x & 31;
+  int* buf = buffers[threadIdx.x >> 5];
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int I = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; I < d.n_blocks; I += warps) {
+  const unsigned below = (1u << lane) - 1u;
+  constexpr int kSub = 32 / C;
+  const int tasks = d.n_blocks * d.row_segments;
+  for (int task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < tasks; task += warps) {
+    const int I = task / d.row_segments, seg = task - I * d.row_segments;
     const int s = d.block_sys[I];
     if (!d.rebuild_now[s]) continue;
     const SysDev& S = d.sys[s];
-    const int old_start = d.tile_start[I], old_n = min(d.tile_cnt[I], S.tile_cap - old_start);
-    const int new_start = d.alive_start[I];
-    int written = 0;
-    for (int k0 = 0; k0 < old_n; k0 += 32) {
-      const int k = k0 + lane;
-      const long long src = static_cast<long long>(S.tile_off) + old_start + k;
-      const bool keep = k < old_n && d.tile_alive[src];
-      const unsigned int keepers = __ballot_sync(0xffffffffu, keep);
-      const long long dst = static_cast<long long>(S.tile_off) + new_start + written +
-                            __popc(keepers & ((1u << lane) - 1u));
-      if (keep) {
-        d.tiles[dst] = d.raw_tiles[src];
-        d.tile_shift[dst] = d.raw_shift[src];
-        if (C < 32)
-          for (int w = 0; w < kWords; ++w) d.masks[dst * kWords + w] = d.raw_masks[src * kWords + w];
+    const int super0 = S.block_off / kSub, supers = S.n_blocks / kSub;
+    const int sI = max(I / kSub, super0 + seg * d.row_supers), sEnd = super0 + min(supers, (seg + 1) * d.row_supers);
+    if (sI >= sEnd) continue;  // no J from I up: the exclusions never look here
+    const Cell B = cell_of_system(S);
+    const float4 li = d.bb_lo[I], hi_ = d.bb_hi[I];
+    const float reach2 = S.list2 * (1.0f + 1e-5f);
+    const int4 pi = d.prune ? d.pc[I * C + (lane & (C - 1))] : make_int4(0, 0, 0, 0);
+    // which of a batch's candidates (a lane's J, or none: J < 0) stay, as a
+    // warp mask: with pruning, those with a pair within cutoff + skin
+    auto keepers = [&](int J) {
+      const unsigned int here = __ballot_sync(0xffffffffu, J >= 0);
+      if (!d.prune) return here;
+      int4 sh = make_int4(0, 0, 0, 0);
+      if (J >= 0) sh = tile_image(S, B, li, hi_, d.bb_lo[J], d.bb_hi[J]);
+      return tiles_with_pair<C>(d, S, I, pi, J, sh, here, reach2);
+    };
+    int found = 0;
+    walk_row<C>(d, B, I, li, hi_, sI, sEnd, [&](int J) {
+      const unsigned int here = __ballot_sync(0xffffffffu, J >= 0);
+      const int at = found + __popc(here & below);
+      if (J >= 0 && at < kRowBuffer) buf[at] = J;
+      found += __popc(here);
+    });
+    __syncwarp();
+    const bool fits = found <= kRowBuffer;
+    int count = found;
+    if (d.prune && fits) {
+      count = 0;
+      for (int k0 = 0; k0 < found; k0 += 32) {
+        const int J = k0 + lane < found ? buf[k0 + lane] : -1;
+        const unsigned int keep = keepers(J);
+        if ((keep >> lane) & 1u) buf[count + __popc(keep & below)] = J;  // never past what was read
+        count += __popc(keep);
+        __syncwarp();
       }
-      if (C == 32) {
-        // a 32x32 tile's mask is 32 words: the warp copies each kept tile's
-        unsigned int f = keepers;
-        while (f) {
-          const int from = __ffs(f) - 1;
-          f &= f - 1;
-          const long long sidx = static_cast<long long>(S.tile_off) + old_start + k0 + from;
-          const long long didx = static_cast<long long>(S.tile_off) + new_start + written +
-                                 __popc(keepers & ((1u << from) - 1u));
-          d.masks[didx * kWords + lane] = d.raw_masks[sidx * kWords + lane];
-        }
-      }
-      written += __popc(keepers);
+    } else if (d.prune) {
+      count = 0;
+      walk_row<C>(d, B, I, li, hi_, sI, sEnd, [&](int J) { count += __popc(keepers(J)); });
     }
+    int start = 0;
     if (lane == 0) {
-      d.tile_start[I] = new_start;
-      d.tile_cnt[I] = written;
+      if (count) start = atomicAdd(&d.tile_need[s], count);
+      d.tile_start[task] = start;
+      d.tile_cnt[task] = count;
+    }
+    start = __shfl_sync(0xffffffffu, start, 0);
+    const long long base = static_cast<long long>(S.tile_off) + start;
+    const int cap = S.tile_cap - start;
+    // tiles past the system's capacity are dropped; the finish phase sees the
+    // count and stops the step
+    auto write = [&](int at, int J) {
+      if (C == 8) {
+        if (J < 0 || at >= cap) return;
+        d.tiles[base + at] = make_int2(I, J);
+        d.tile_shift[base + at] = tile_image(S, B, li, hi_, d.bb_lo[J], d.bb_hi[J]);
+        unsigned int words[2] = {0u, 0u};
+#pragma unroll
+        for (int r = 0; r < 8; ++r) words[r >> 2] |= valid_row<8>(S, I - S.block_off, J - S.block_off, r) << ((r & 3) * 8);
+        *reinterpret_cast<uint2*>(d.masks + (base + at) * kWords) = make_uint2(words[0], words[1]);
+      }
+    };
+    auto write_batch = [&](int at0, int J, unsigned int keep) {
+      if (C == 8) {
+        write(at0 + __popc(keep & below), (keep >> lane) & 1u ? J : -1);
+        return;
+      }
+      // a 32x32 tile's mask is one word per row: every lane writes its row
+      for (int n = 0; keep; ++n) {
+        const int src = __ffs(keep) - 1;
+        keep &= keep - 1;
+        const int Jt = __shfl_sync(0xffffffffu, J, src), at = at0 + n;
+        if (at >= cap) continue;
+        if (lane == 0) {
+          d.tiles[base + at] = make_int2(I, Jt);
+          d.tile_shift[base + at] = tile_image(S, B, li, hi_, d.bb_lo[Jt], d.bb_hi[Jt]);
+        }
+        d.masks[(base + at) * kWords + lane] = valid_row<C>(S, I - S.block_off, Jt - S.block_off, lane);
+      }
+    };
+    if (fits) {
+      for (int k0 = 0; k0 < count; k0 += 32) {
+        const int J = k0 + lane < count ? buf[k0 + lane] : -1;
+        write_batch(k0, J, __ballot_sync(0xffffffffu, J >= 0));
+      }
+      __syncwarp();  // the buffer is free for the warp's next row
+    } else {
+      int written = 0;
+      walk_row<C>(d, B, I, li, hi_, sI, sEnd, [&](int J) {
+        const unsigned int keep = keepers(J);
+        write_batch(written, J, keep);
+        written += __popc(keep);
+      });
     }
   }
 }
@@ -637,17 +656,19 @@ __device__ void phase_tiles_exclusions(const Dev& d) {
     if (sa > sb) { const int t = sa; sa = sb; sb = t; }
     const int I = S.block_off + sa / C, J = S.block_off + sb / C;
     const int row = sa % C, bit = sb % C;
-    int lo = d.tile_start[I];
-    int hi = lo + d.tile_cnt[I];
+    // the row's segment that would hold the tile, in ascending J
+    const int task = I * d.row_segments + (J - S.block_off) / (32 / C) / d.row_supers;
+    int lo = d.tile_start[task];
+    const int end = lo + d.tile_cnt[task];
+    int hi = end;
     if (hi > S.tile_cap) hi = S.tile_cap;
-    // tiles of row I are in ascending J
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
       const int Jm = d.tiles[S.tile_off + mid].y;
       if (Jm < J) lo = mid + 1;
       else hi = mid;
     }
-    if (lo < d.tile_start[I] + d.tile_cnt[I] && lo < S.tile_cap && d.tiles[S.tile_off + lo].y == J) {
+    if (lo < end && lo < S.tile_cap && d.tiles[S.tile_off + lo].y == J) {
       const long long t = static_cast<long long>(S.tile_off) + lo;
       if (C == 32) atomicAnd(&d.masks[t * 32 + row], ~(1u << bit));
       else atomicAnd(&d.masks[t * (C * C / 32) + (row >> 2)], ~(1u << ((row & 3) * 8 + bit)));
@@ -680,20 +701,17 @@ __device__ void phase_tiles_exclusions(const Dev& d) {
 template <int C>
 __device__ bool tile_within_reach(const Dev& d, const SysDev& S, long long ti, float reach2, int lane);
 
-template <>
-__device__ bool tile_within_reach<8>(const Dev& d, const SysDev& S, long long ti, float reach2, int) {
-  const int2 tile = __ldcg(&d.tiles[ti]);
-  const int4 sh = __ldcg(&d.tile_shift[ti]);
+// Some pair of an 8x8 tile's mask closer than reach (a lane's own tile; every
+// pair's minimum image if the tile is flagged for it).
+__device__ __forceinline__ bool tile_has_pair(const Dev& d, const SysDev& S, int2 tile, int4 sh,
+                                              const unsigned int* mask, float reach2) {
   const float inv = S.pc_inv;
   if (tile_per_pair(sh.w)) {
-    if (!S.prune_per_pair) return true;
-    // per-pair images (small cells): the pair kernel's own minimum image of each pair
-    const unsigned int w0 = __ldcg(&d.masks[ti * 2]), w1 = __ldcg(&d.masks[ti * 2 + 1]);
     int4 qj[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) qj[j] = d.pc[tile.y * 8 + j];
     for (int i = 0; i < 8; ++i) {
-      const unsigned int row = ((i < 4 ? w0 : w1) >> ((i & 3) * 8)) & 0xFFu;
+      const unsigned int row = ((i < 4 ? mask[0] : mask[1]) >> ((i & 3) * 8)) & 0xFFu;
       if (!row) continue;
       const int4 qi = d.pc[tile.x * 8 + i];
 #pragma unroll
@@ -709,18 +727,6 @@ __device__ bool tile_within_reach<8>(const Dev& d, const SysDev& S, long long ti
     }
     return false;
   }
-  {
-    // the clusters' current boxes first: most outer tiles of a long skin are
-    // out of reach box to box and need no pair loop (the margin covers the
-    // boxes' f32 rounding)
-    const float4 ilo = d.cb_lo[tile.x], ihi = d.cb_hi[tile.x], jlo = d.cb_lo[tile.y], jhi = d.cb_hi[tile.y];
-    const float sx = sh.x * inv, sy = sh.y * inv, sz = sh.z * inv;
-    const float gx = fmaxf(fmaxf(jlo.x + sx - ihi.x, ilo.x - (jhi.x + sx)), 0.f);
-    const float gy = fmaxf(fmaxf(jlo.y + sy - ihi.y, ilo.y - (jhi.y + sy)), 0.f);
-    const float gz = fmaxf(fmaxf(jlo.z + sz - ihi.z, ilo.z - (jhi.z + sz)), 0.f);
-    if (gx * gx + gy * gy + gz * gz >= reach2 * (1.0f + 4e-5f)) return false;
-  }
-  const unsigned int w0 = __ldcg(&d.masks[ti * 2]), w1 = __ldcg(&d.masks[ti * 2 + 1]);
   // both clusters' sixteen atoms in one round of loads, then the 64 tests
   // (loading each i atom inside the loop made a chain of eight round trips)
   int4 qi[8], qj[8];
@@ -741,7 +747,7 @@ __device__ bool tile_within_reach<8>(const Dev& d, const SysDev& S, long long ti
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const unsigned int row = ((i < 4 ? w0 : w1) >> ((i & 3) * 8)) & 0xFFu;
+    const unsigned int row = ((i < 4 ? mask[0] : mask[1]) >> ((i & 3) * 8)) & 0xFFu;
     const float ix = int(unsigned(qi[i].x) - unsigned(r0.x)) * inv,
                 iy = int(unsigned(qi[i].y) - unsigned(r0.y)) * inv,
                 iz = int(unsigned(qi[i].z) - unsigned(r0.z)) * inv;
@@ -754,6 +760,28 @@ __device__ bool tile_within_reach<8>(const Dev& d, const SysDev& S, long long ti
     if (hit) return true;  // most kept tiles stop at their first rows
   }
   return false;
+}
+
+template <>
+__device__ bool tile_within_reach<8>(const Dev& d, const SysDev& S, long long ti, float reach2, int) {
+  const int2 tile = __ldcg(&d.tiles[ti]);
+  const int4 sh = __ldcg(&d.tile_shift[ti]);
+  const bool per_pair = tile_per_pair(sh.w);
+  if (per_pair && !S.prune_per_pair) return true;
+  if (!per_pair) {
+    // the clusters' current boxes first: most outer tiles of a long skin are
+    // out of reach box to box and need no pair loop (the margin covers the
+    // boxes' f32 rounding)
+    const float inv = S.pc_inv;
+    const float4 ilo = d.cb_lo[tile.x], ihi = d.cb_hi[tile.x], jlo = d.cb_lo[tile.y], jhi = d.cb_hi[tile.y];
+    const float sx = sh.x * inv, sy = sh.y * inv, sz = sh.z * inv;
+    const float gx = fmaxf(fmaxf(jlo.x + sx - ihi.x, ilo.x - (jhi.x + sx)), 0.f);
+    const float gy = fmaxf(fmaxf(jlo.y + sy - ihi.y, ilo.y - (jhi.y + sy)), 0.f);
+    const float gz = fmaxf(fmaxf(jlo.z + sz - ihi.z, ilo.z - (jhi.z + sz)), 0.f);
+    if (gx * gx + gy * gy + gz * gz >= reach2 * (1.0f + 4e-5f)) return false;
+  }
+  const unsigned int mask[2] = {__ldcg(&d.masks[ti * 2]), __ldcg(&d.masks[ti * 2 + 1])};
+  return tile_has_pair(d, S, tile, sh, mask, reach2);
 }
 
 template <>
@@ -834,37 +862,79 @@ __device__ void phase_inner(const Dev& d) {
   }
 }
 
-// After the outer list: per-system offsets and rebuild counts.  Without an
-// inner list the rebuild requests are cleared here; with one, the inner-list
-// kernel that follows still needs them and clears them itself.
-__device__ void phase_tiles_finish(const Dev& d) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    int total = 0;
-    for (int s = 0; s < d.S; ++s) {
-      d.tile_prefix[s] = total;
-      total += d.tile_count[s];
-      if (d.rebuild_now[s]) d.rebuild_count[s] += 1;
-      if (!d.inner) d.rebuild_now[s] = 0;
+// Exclusive offsets of per-system counts (one warp): prefix[s] and, at
+// prefix[S], the total; `count(s)` is called once per system.
+template <class Count>
+__device__ __forceinline__ void system_offsets(const Dev& d, int* prefix, Count count) {
+  const int lane = threadIdx.x & 31;
+  int carry = 0;
+  for (int s0 = 0; s0 < d.S; s0 += 32) {
+    const int s = s0 + lane, n = s < d.S ? count(s) : 0;
+    int x = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
     }
-    d.tile_prefix[d.S] = total;
-    if (!d.inner) *d.any_rebuild = 0;
+    if (s < d.S) prefix[s] = carry + x - n;
+    carry += __shfl_sync(0xffffffffu, x, 31);
   }
+  if (lane == 0) prefix[d.S] = carry;
 }
 
-// After the inner list (one thread): its offsets, the prune count, and every
+// After the outer list (one warp): per-system counts, offsets and rebuild
+// counts.  Without an inner list the rebuild requests are cleared here; with
+// one, the inner-list kernel that follows still needs them and clears them
+// itself.
+__device__ void list_finish(const Dev& d) {
+  system_offsets(d, d.tile_prefix, [&](int s) {
+    int n = d.tile_count[s];
+    if (d.rebuild_now[s]) {
+      // a list that needs more tiles than the system's capacity is cut there,
+      // and the engine's halt word stops the integrator, so no step runs on
+      // the cut list: the host grows the capacity to `tile_need` and rebuilds
+      // before it runs the remaining steps
+      const int need = __ldcg(&d.tile_need[s]), cap = d.sys[s].tile_cap;
+      if (need > cap) {
+        atomicOr(&d.err[s], kErrTileCapacity);
+        atomicExch(d.halt, 1);
+      }
+      d.tile_count[s] = n = min(need, cap);
+      d.rebuild_count[s] += 1;
+      if (!d.inner) d.rebuild_now[s] = 0;
+    }
+    return n;
+  });
+  if (!d.inner && (threadIdx.x & 31) == 0) *d.any_rebuild = 0;
+}
+
+// After the inner list (one warp): its offsets, the prune count, and every
 // list request cleared for the next step.
 __device__ void inner_finish(const Dev& d) {
-  int total = 0;
-  for (int s = 0; s < d.S; ++s) {
-    d.in_prefix[s] = total;
-    total += d.in_count[s];
+  system_offsets(d, d.in_prefix, [&](int s) {
     if (d.prune_now[s] && !d.rebuild_now[s]) d.prune_count[s] += 1;
     d.prune_now[s] = 0;
     d.rebuild_now[s] = 0;
+    return __ldcg(&d.in_count[s]);
+  });
+  if ((threadIdx.x & 31) == 0) {
+    *d.any_rebuild = 0;
+    *d.any_prune = 0;
   }
-  d.in_prefix[d.S] = total;
-  *d.any_rebuild = 0;
-  *d.any_prune = 0;
+}
+
+// True in every thread of the block that finishes last, whose view of global
+// memory then holds every block's writes.
+__device__ __forceinline__ bool last_block(int* ticket) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == int(gridDim.x) - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  if (threadIdx.x == 0) *ticket = 0;
+  return true;
 }
 
 // Grid-wide barrier for the cooperative list kernel: arrive on a counter,
@@ -900,73 +970,68 @@ __device__ bool grid_barrier(unsigned int* bar, int* err) {
   return ok != 0;
 }
 
-// One launch per step.  With no rebuild requested it returns at once, or folds
-// the pair coordinates when a prune is due; otherwise it runs the sort and
+// The exclusions, and the list's finish by the last block to end: every block
+// has read the rebuild requests by then.
+template <int C>
+__device__ void phase_exclusions_finish(const Dev& d) {
+  phase_tiles_exclusions<C>(d);
+  if (last_block(d.list_ticket) && threadIdx.x < 32) list_finish(d);
+}
+
+// One launch per step.  With no rebuild requested it returns at once, or takes
+// the references of a prune that is due; otherwise it runs the sort and
 // tile-list phases with a grid barrier between them.
 template <int C>
-__global__ void __launch_bounds__(kThreads) k_list(Dev d) {
-  const bool rebuild = *d.any_rebuild != 0;
+__global__ void __launch_bounds__(kThreads, 4) k_list(Dev d) {
+  __shared__ int buffers[kThreads / 32][kRowBuffer];
+  const bool rebuild = *d.any_rebuild != 0, prune = d.inner && *d.any_prune != 0;
   int* err = d.err;  // system 0's word carries a barrier timeout
-  if (!rebuild) {
-    // the integrator wrote this step's pair coordinates; the wrap runs again
-    // only for a prune, which needs reference positions and cluster boxes
-    if (*d.any_prune) phase_wrap(d);
-    return;
-  }
-  phase_cells_clear(d);
-  if (!grid_barrier(d.list_barrier, err)) return;
+  if (prune) phase_prune_references(d);
+  if (!rebuild) return;
   phase_cells_assign(d);
   if (!grid_barrier(d.list_barrier, err)) return;
   phase_cells_scan(d);
   if (!grid_barrier(d.list_barrier, err)) return;
   phase_cells_scatter(d);
   if (!grid_barrier(d.list_barrier, err)) return;
-  phase_cells_order(d);
+  phase_place(d);
   if (!grid_barrier(d.list_barrier, err)) return;
-  phase_wrap(d);
+  phase_boxes<C>(d);
   if (!grid_barrier(d.list_barrier, err)) return;
-  phase_tiles_blocks<C>(d);
+  phase_rows<C>(d, buffers);
   if (!grid_barrier(d.list_barrier, err)) return;
-  phase_tiles_find<C, false>(d);
-  if (!grid_barrier(d.list_barrier, err)) return;
-  phase_tiles_scan(d);
-  if (!grid_barrier(d.list_barrier, err)) return;
-  phase_tiles_find<C, true>(d);
-  if (!grid_barrier(d.list_barrier, err)) return;
-  if (d.prune) {
-    phase_tiles_prune<C>(d);
-    if (!grid_barrier(d.list_barrier, err)) return;
-    phase_tiles_rescan(d);
-    if (!grid_barrier(d.list_barrier, err)) return;
-    phase_tiles_compact<C>(d);
-    if (!grid_barrier(d.list_barrier, err)) return;
-  }
-  phase_tiles_exclusions<C>(d);
-  if (!grid_barrier(d.list_barrier, err)) return;
-  phase_tiles_finish(d);
+  phase_exclusions_finish<C>(d);
 }
 
-// The same phases as separate launches (the path the graph-free debug mode
-// and devices without cooperative launch take).
-#define MDB_PHASE_KERNEL(name, guarded)                            \
-  __global__ void __launch_bounds__(kThreads) k_##name(Dev d) {   \
-    if (guarded && !*d.any_rebuild) return;                        \
-    phase_##name(d);                                               \
-  }
-MDB_PHASE_KERNEL(cells_clear, true)
-MDB_PHASE_KERNEL(cells_assign, true)
-MDB_PHASE_KERNEL(cells_scan, true)
-MDB_PHASE_KERNEL(cells_scatter, true)
-MDB_PHASE_KERNEL(cells_order, true)
-MDB_PHASE_KERNEL(tiles_scan, true)
-MDB_PHASE_KERNEL(tiles_rescan, true)
-MDB_PHASE_KERNEL(tiles_finish, true)
-#undef MDB_PHASE_KERNEL
-// the wrap, when a rebuild or a prune is due (otherwise the integrator wrote
-// the pair coordinates at the end of the previous step)
-__global__ void __launch_bounds__(kThreads) k_wrap(Dev d) {
-  if (!*d.any_rebuild && !*d.any_prune) return;
-  phase_wrap(d);
+// The same phases as separate launches (the path the graph-free debug mode,
+// large batches and devices without cooperative launch take).
+__global__ void __launch_bounds__(kThreads) k_prune_references(Dev d) {
+  if (d.inner && *d.any_prune) phase_prune_references(d);
+}
+__global__ void __launch_bounds__(kThreads) k_cells_assign(Dev d) {
+  if (*d.any_rebuild) phase_cells_assign(d);
+}
+__global__ void __launch_bounds__(kThreads) k_cells_scan(Dev d) {
+  if (*d.any_rebuild) phase_cells_scan(d);
+}
+__global__ void __launch_bounds__(kThreads) k_cells_scatter(Dev d) {
+  if (*d.any_rebuild) phase_cells_scatter(d);
+}
+__global__ void __launch_bounds__(kThreads) k_place(Dev d) {
+  if (*d.any_rebuild) phase_place(d);
+}
+template <int C>
+__global__ void __launch_bounds__(kThreads) k_boxes(Dev d) {
+  if (*d.any_rebuild) phase_boxes<C>(d);
+}
+template <int C>
+__global__ void __launch_bounds__(kThreads, 3) k_rows(Dev d) {
+  __shared__ int buffers[kThreads / 32][kRowBuffer];
+  if (*d.any_rebuild) phase_rows<C>(d, buffers);
+}
+template <int C>
+__global__ void __launch_bounds__(kThreads) k_exclusions(Dev d) {
+  if (*d.any_rebuild) phase_exclusions_finish<C>(d);
 }
 // The inner list, its own launch after the list kernels (a full grid, where
 // the cooperative list kernel has two blocks per SM): nothing to do unless a
@@ -979,38 +1044,8 @@ __global__ void __launch_bounds__(kThreads) k_inner_prune(Dev d) {
   release_successor();
   if (!*d.any_rebuild && !*d.any_prune) return;
   phase_inner<C>(d);
-  __shared__ int last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(d.inner_ticket, 1) == int(gridDim.x) - 1;
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
-    __threadfence();
-    inner_finish(d);
-    *d.inner_ticket = 0;
-  }
+  if (last_block(d.inner_ticket) && threadIdx.x < 32) inner_finish(d);
 }
-#define MDB_PHASE_KERNEL_C(name)                                   \
-  template <int C>                                                 \
-  __global__ void __launch_bounds__(kThreads) k_##name(Dev d) {   \
-    if (!*d.any_rebuild) return;                                   \
-    phase_##name<C>(d);                                            \
-  }
-MDB_PHASE_KERNEL_C(tiles_blocks)
-MDB_PHASE_KERNEL_C(tiles_prune)
-MDB_PHASE_KERNEL_C(tiles_compact)
-template <int C>
-__global__ void __launch_bounds__(kThreads) k_tiles_count(Dev d) {
-  if (!*d.any_rebuild) return;
-  phase_tiles_find<C, false>(d);
-}
-template <int C>
-__global__ void __launch_bounds__(kThreads) k_tiles_fill(Dev d) {
-  if (!*d.any_rebuild) return;
-  phase_tiles_find<C, true>(d);
-}
-MDB_PHASE_KERNEL_C(tiles_exclusions)
-#undef MDB_PHASE_KERNEL_C
 
 int blocks_for(int n, int threads, int cap = 148 * 8) {
   const int b = (n + threads - 1) / threads;
@@ -1038,7 +1073,16 @@ int prepare_list_kernel(int device) {
 bool launch_list(const Dev& d, cudaStream_t st) {
   if (g_list_grid <= 0) return false;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(g_list_grid);
+  // Two blocks per SM, or one where an inner list makes rebuilds rare and the
+  // system is small: most launches then find nothing to do, and the fewer
+  // blocks cost the spread beside them less (27k-atom octahedron: step 117 us
+  // with one, 123 with two, though its rebuild takes 267 instead of 219 us; 100k
+  // atoms: 400 and 392 us, rebuild 566 and 414).  Rebuilds before the phases
+  // were joined and the rows searched once: 2,652 atoms (defaults) 111 -> 72
+  // us, 12k 163 -> 146, 27k 305 -> 267, 100k 694 -> 414, the 64-system ensemble
+  // (all systems, separate launches) 2.58 -> 1.73 ms.
+  const bool few = d.inner && d.n_slots < (1 << 16) && g_list_grid > 1;
+  cfg.gridDim = dim3(few ? (g_list_grid + 1) / 2 : g_list_grid);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
@@ -1052,31 +1096,22 @@ bool launch_list(const Dev& d, cudaStream_t st) {
 }
 
 void launch_rebuild_sort(const Dev& d, cudaStream_t st) {
-  k_cells_clear<<<blocks_for(d.n_cells, kThreads), kThreads, 0, st>>>(d);
   k_cells_assign<<<blocks_for(d.n_atoms, kThreads), kThreads, 0, st>>>(d);
-  k_cells_scan<<<d.S < 148 ? d.S : 148, kThreads, 0, st>>>(d);
+  k_cells_scan<<<blocks_for(d.n_chunks, 1), kThreads, 0, st>>>(d);
   k_cells_scatter<<<blocks_for(d.n_atoms, kThreads), kThreads, 0, st>>>(d);
-  k_cells_order<<<blocks_for(d.n_slots, kThreads), kThreads, 0, st>>>(d);
+  k_place<<<blocks_for(d.n_slots, kThreads), kThreads, 0, st>>>(d);
 }
 
-void launch_wrap(const Dev& d, cudaStream_t st) {
-  k_wrap<<<blocks_for(d.n_slots, kThreads), kThreads, 0, st>>>(d);
+void launch_prune_references(const Dev& d, cudaStream_t st) {
+  if (d.inner) k_prune_references<<<blocks_for(d.n_slots, kThreads), kThreads, 0, st>>>(d);
 }
 
 template <int C>
 void rebuild_tiles(const Dev& d, cudaStream_t st) {
-  const int warp_blocks = blocks_for(d.n_blocks * 32, kThreads);
-  k_tiles_blocks<C><<<warp_blocks, kThreads, 0, st>>>(d);
-  k_tiles_count<C><<<warp_blocks, kThreads, 0, st>>>(d);
-  k_tiles_scan<<<d.S < 148 ? d.S : 148, kThreads, 0, st>>>(d);
-  k_tiles_fill<C><<<warp_blocks, kThreads, 0, st>>>(d);
-  if (d.prune) {
-    k_tiles_prune<C><<<148 * 4, kThreads, 0, st>>>(d);
-    k_tiles_rescan<<<d.S < 148 ? d.S : 148, kThreads, 0, st>>>(d);
-    k_tiles_compact<C><<<warp_blocks, kThreads, 0, st>>>(d);
-  }
-  k_tiles_exclusions<C><<<blocks_for(d.n_excl, kThreads), kThreads, 0, st>>>(d);
-  k_tiles_finish<<<1, 32, 0, st>>>(d);
+  const int warp_blocks = blocks_for(d.n_blocks * d.row_segments * 32, kThreads);
+  k_boxes<C><<<blocks_for(d.n_slots, kThreads), kThreads, 0, st>>>(d);
+  k_rows<C><<<warp_blocks, kThreads, 0, st>>>(d);
+  k_exclusions<C><<<blocks_for(d.n_excl, kThreads), kThreads, 0, st>>>(d);
 }
 
 void launch_inner_prune(const Dev& d, cudaStream_t st) {
