@@ -213,6 +213,13 @@ void launch_pme_fft(const Dev& d, bool energy, cudaStream_t s);
 void launch_pme_gather(const Dev& d, cudaStream_t s);
 void launch_influence(const Dev& d, int sys, cudaStream_t s);  // after a box change; sys < 0: every system
 void launch_integrate(const Dev& d, cudaStream_t s);
+// states to and from pinned host arrays of xyz-interleaved doubles
+void launch_positions_out(const Dev& d, int atom_off, int n, double* out, cudaStream_t st);
+void launch_velocities_out(const Dev& d, int atom_off, int n, double* out, cudaStream_t st);
+void launch_forces_out(const Dev& d, int atom_off, int slot_off, int n, double* out, cudaStream_t st);
+void launch_positions_in(const Dev& d, int atom_off, int n, const double* in, bool clear_residual, cudaStream_t st);
+void launch_velocities_in(const Dev& d, int atom_off, int n, const double* in, cudaStream_t st);
+void launch_request_rebuild(const Dev& d, int s, cudaStream_t st);  // s < 0: every system
 void launch_momentum(const Dev& d, cudaStream_t s);
 void launch_scale_molecules(const Dev& d, int first_mol, int n_mol, double scale, cudaStream_t st);
 void launch_restore_positions(const Dev& d, int atom_off, int n, cudaStream_t st);

@@ -110,7 +110,6 @@ struct mdb_engine {
   int64_t step = 0;
   std::string error;
   int n_mesh_items = 0;
-  std::vector<int> fft_x_sys;  // system of each x-pass work item
   bool coop_list = false;      // the list kernels run as one cooperative launch
   int cluster = 8;                 // atoms per cluster of the tile list (8 or 32), per engine
   bool prune = true;               // rebuilds drop tiles with no pair inside cutoff + skin
@@ -122,6 +121,18 @@ struct mdb_engine {
   std::vector<double> inner_skin;  // per system, nm; <= 0: that system's inner list is its outer list
   int64_t list_grown = 0;          // times an overflowing list was grown and rebuilt
   unsigned char* active = nullptr;  // device: per system, whether an evaluation computes it
+  // one block of pinned host memory the device reads and writes (k_io.cu), cut
+  // into a state array of the largest system and the small results of an
+  // evaluation.  A call uses it between waits on s0, so nothing of one call is
+  // left in it for another.
+  void* pinned = nullptr;
+  double* io_state = nullptr;               // 3 n doubles
+  float* io_velocities = nullptr;           // 3 n floats
+  unsigned long long* io_energy = nullptr;  // S x kECount
+  double *io_mesh = nullptr, *io_mesh_virial = nullptr, *io_mol = nullptr;
+  int *io_err = nullptr, *io_halt = nullptr;
+  unsigned char* io_active = nullptr;
+  std::vector<int> mesh_first;  // per system: its first x-pass work item; [S]: their number
   std::vector<std::array<double, 9>> box_at_rebuild;  // per system: the box when a box change last asked for a rebuild
 };
 
@@ -289,12 +300,18 @@ void fill_box(const HostSystem& h, SysDev& S, bool keep_shift) {
 }
 
 int request_rebuild(mdb_engine* e, int s);
+int report_device_status(mdb_engine* e);
 
 int check_device_status(mdb_engine* e) {
+  CUDA_TRY(e, cudaMemcpyAsync(e->io_err, e->d.err, sizeof(int) * e->d.S, cudaMemcpyDeviceToHost, e->s0));
   cudaError_t err = cudaStreamSynchronize(e->s0);
   if (err != cudaSuccess) return fail(e, MDB_ERR_DEVICE, std::string("device: ") + cudaGetErrorString(err));
-  std::vector<int> flags(e->d.S), shake(e->d.S);
-  CUDA_TRY(e, cudaMemcpy(flags.data(), e->d.err, sizeof(int) * e->d.S, cudaMemcpyDeviceToHost));
+  return report_device_status(e);
+}
+
+// The error code for the status words in the pinned block.
+int report_device_status(mdb_engine* e) {
+  std::vector<int> flags(e->io_err, e->io_err + e->d.S);
   int any = 0;
   for (int f : flags) any |= f;
   if (any & kErrTileCapacity) return fail(e, MDB_ERR_CAPACITY, "the cluster-pair tile list ran out of room");
@@ -376,13 +393,8 @@ int run_steps(mdb_engine* e, int64_t steps) {
 }
 
 int request_rebuild(mdb_engine* e, int s) {
-  std::vector<int> now(e->d.S, 0);
-  CUDA_TRY(e, cudaMemcpy(now.data(), e->d.rebuild_now, sizeof(int) * e->d.S, cudaMemcpyDeviceToHost));
-  if (s < 0) std::fill(now.begin(), now.end(), 1);
-  else now[s] = 1;
-  const int one = 1;
-  CUDA_TRY(e, cudaMemcpy(e->d.rebuild_now, now.data(), sizeof(int) * e->d.S, cudaMemcpyHostToDevice));
-  CUDA_TRY(e, cudaMemcpy(e->d.any_rebuild, &one, sizeof(int), cudaMemcpyHostToDevice));
+  launch_request_rebuild(e->d, s, e->s0);
+  CUDA_TRY(e, cudaGetLastError());
   return MDB_OK;
 }
 
@@ -426,10 +438,9 @@ int grow_tile_list(mdb_engine* e) {
 
 // Whether a list overflowed (the integrator has stopped): one 4-byte read.
 int list_halted(mdb_engine* e, bool* halted) {
-  int h = 0;
-  CUDA_TRY(e, cudaMemcpyAsync(&h, e->d.halt, sizeof(int), cudaMemcpyDeviceToHost, e->s0));
+  CUDA_TRY(e, cudaMemcpyAsync(e->io_halt, e->d.halt, sizeof(int), cudaMemcpyDeviceToHost, e->s0));
   CUDA_TRY(e, cudaStreamSynchronize(e->s0));
-  *halted = h != 0;
+  *halted = *e->io_halt != 0;
   return MDB_OK;
 }
 
@@ -584,10 +595,10 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
     for (int x = 0; x < Kx; ++x)
       for (int k = 0; k < S.kzh; k += kFftTile) wy.push_back({s, x, k, std::min(kFftTile, S.kzh - k)});
     smem_y = std::max(smem_y, strip_smem(kFftTile, Ky));
+    e->mesh_first.push_back(int(wx.size()));
     for (int y = 0; y < Ky; ++y)
       for (int k = 0; k < S.kzh; k += kFftTile) {
         wx.push_back({s, y, k, std::min(kFftTile, S.kzh - k)});
-        e->fft_x_sys.push_back(s);
       }
     smem_x = std::max(smem_x, strip_smem(kFftTile, Kx));
     for (int x = 0; x < Kx; ++x) wp.push_back({s, x, 0, 1});
@@ -908,6 +919,7 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   d.smem_y = smem_y;
   d.smem_x = smem_x;
   e->n_mesh_items = int(wx.size());
+  e->mesh_first.push_back(e->n_mesh_items);
   TRY(alloc(e, "energies", d.energy, size_t(n) * kECount));
   {
     std::vector<int> mol_off{0}, mol_atoms;
@@ -986,6 +998,35 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   CUDA_TRY(e, cudaEventCreate(&e->t1));
   CUDA_TRY(e, cudaDeviceSynchronize());
 
+  {
+    // the pinned block: every piece starts on a 16-byte boundary
+    size_t bytes = 0;
+    auto piece = [&](size_t n) {
+      const size_t at = bytes;
+      bytes += (n + 15) / 16 * 16;
+      return at;
+    };
+    size_t n = 1;
+    for (const HostSystem& h : e->hs) n = std::max(n, size_t(h.n));
+    const size_t systems = size_t(d.S), mols = size_t(e->mol_part_off.back() + molecular_offset_blocks(e->mol_count.back()));
+    const size_t at[] = {piece(3 * n * sizeof(double)),          piece(3 * n * sizeof(float)),
+                         piece(systems * kECount * sizeof(long long)), piece(size_t(e->n_mesh_items) * sizeof(double)),
+                         piece(size_t(e->n_mesh_items) * 6 * sizeof(double)), piece(mols * 9 * sizeof(double)),
+                         piece(systems * sizeof(int)),           piece(sizeof(int)),
+                         piece(systems)};
+    CUDA_TRY(e, cudaHostAlloc(&e->pinned, bytes, cudaHostAllocMapped));
+    char* base = static_cast<char*>(e->pinned);
+    e->io_state = reinterpret_cast<double*>(base + at[0]);
+    e->io_velocities = reinterpret_cast<float*>(base + at[1]);
+    e->io_energy = reinterpret_cast<unsigned long long*>(base + at[2]);
+    e->io_mesh = reinterpret_cast<double*>(base + at[3]);
+    e->io_mesh_virial = reinterpret_cast<double*>(base + at[4]);
+    e->io_mol = reinterpret_cast<double*>(base + at[5]);
+    e->io_err = reinterpret_cast<int*>(base + at[6]);
+    e->io_halt = reinterpret_cast<int*>(base + at[7]);
+    e->io_active = reinterpret_cast<unsigned char*>(base + at[8]);
+  }
+
   launch_influence(e->d, -1, e->s0);
   // first list and the first COM velocity, by the phase kernels (a list that
   // overflows its starting capacity is grown and built again)
@@ -1042,79 +1083,79 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
 int evaluate_many(mdb_engine* e, const std::vector<int>& systems, double* forces, mdb_energies* out,
                   bool kinetic) {
   const Dev& d = e->d;
-  CUDA_TRY(e, cudaMemsetAsync(d.energy, 0, sizeof(unsigned long long) * d.S * kECount, e->s0));
-  // the list first: one that overflows is grown and built again before any force
+  if (systems.empty()) return check_device_status(e);
+  const int mols = e->mol_part_off.back() + molecular_offset_blocks(e->mol_count.back());
+  // the force kernels skip the systems not asked for
+  Dev dv = d;
+  if (int(systems.size()) < d.S) {
+    CUDA_TRY(e, cudaStreamSynchronize(e->s0));  // an earlier evaluation may still be copying it
+    std::fill(e->io_active, e->io_active + d.S, 0);
+    for (int s : systems) e->io_active[s] = 1;
+    CUDA_TRY(e, cudaMemcpyAsync(e->active, e->io_active, d.S, cudaMemcpyHostToDevice, e->s0));
+    dv.active = e->active;
+  }
+  // Everything is queued behind one wait.  A list that overflowed makes the
+  // evaluation worthless (its forces come from a cut list): the list is then
+  // grown and all of it runs again.
+  const SysDev& S0 = e->sd[systems[0]];
   for (int attempt = 0;; ++attempt) {
+    CUDA_TRY(e, cudaMemsetAsync(d.energy, 0, sizeof(unsigned long long) * d.S * kECount, e->s0));
     list_kernels(e, e->s0);
+    // the spread goes by the list's order at these positions (they may be the caller's)
+    CUDA_TRY(e, cudaMemcpyAsync(d.spread_atom, d.order, sizeof(int) * size_t(d.n_slots), cudaMemcpyDeviceToDevice, e->s0));
+    launch_pme(dv, true, e->s0);
+    launch_listed(dv, true, e->s0);
+    launch_nonbonded(dv, true, e->s0);
+    if (forces) launch_forces_out(d, S0.atom_off, S0.slot_off, S0.n_atoms, e->io_state, e->s0);
+    if (out) {
+      for (int s : systems)
+        launch_molecular_offsets(d, e->mol_first[s], e->mol_count[s], e->sd[s].slot_off,
+                                 e->mol_partials + size_t(e->mol_part_off[s]) * 9, e->s0);
+      auto fetch = [&](void* to, const void* from, size_t bytes) {
+        return cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, e->s0);
+      };
+      CUDA_TRY(e, fetch(e->io_mol, e->mol_partials, sizeof(double) * size_t(mols) * 9));
+      CUDA_TRY(e, fetch(e->io_energy, d.energy, sizeof(long long) * size_t(d.S) * kECount));
+      CUDA_TRY(e, fetch(e->io_mesh, d.mesh_partial, sizeof(double) * size_t(e->n_mesh_items)));
+      CUDA_TRY(e, fetch(e->io_mesh_virial, d.mesh_virial, sizeof(double) * size_t(e->n_mesh_items) * 6));
+      if (kinetic) {
+        const size_t n = size_t(S0.n_atoms);
+        CUDA_TRY(e, fetch(e->io_velocities, d.vx + S0.atom_off, sizeof(float) * n));
+        CUDA_TRY(e, fetch(e->io_velocities + n, d.vy + S0.atom_off, sizeof(float) * n));
+        CUDA_TRY(e, fetch(e->io_velocities + 2 * n, d.vz + S0.atom_off, sizeof(float) * n));
+      }
+    }
+    // the step loop expects cleared accumulators
+    CUDA_TRY(e, cudaMemsetAsync(d.fx, 0, sizeof(long long) * d.n_slots, e->s0));
+    CUDA_TRY(e, cudaMemsetAsync(d.fy, 0, sizeof(long long) * d.n_slots, e->s0));
+    CUDA_TRY(e, cudaMemsetAsync(d.fz, 0, sizeof(long long) * d.n_slots, e->s0));
+    CUDA_TRY(e, cudaMemcpyAsync(e->io_err, d.err, sizeof(int) * d.S, cudaMemcpyDeviceToHost, e->s0));
+    CUDA_TRY(e, cudaGetLastError());
     bool halted = false;
     if (const int st = list_halted(e, &halted)) return st;
     if (!halted || attempt == 4) break;
     if (const int st = grow_tile_list(e)) return st;
+    dv = d;
+    if (int(systems.size()) < d.S) dv.active = e->active;
   }
-  // the force kernels skip the systems not asked for
-  Dev dv = d;
-  if (int(systems.size()) < d.S) {
-    std::vector<unsigned char> on(d.S, 0);
-    for (int s : systems) on[s] = 1;
-    CUDA_TRY(e, cudaMemcpyAsync(e->active, on.data(), d.S, cudaMemcpyHostToDevice, e->s0));
-    CUDA_TRY(e, cudaStreamSynchronize(e->s0));  // `on` is pageable host memory
-    dv.active = e->active;
-  }
-  // the spread goes by the list's order at these positions (they may be the caller's)
-  CUDA_TRY(e, cudaMemcpyAsync(d.spread_atom, d.order, sizeof(int) * size_t(d.n_slots), cudaMemcpyDeviceToDevice, e->s0));
-  launch_pme(dv, true, e->s0);
-  launch_listed(dv, true, e->s0);
-  launch_nonbonded(dv, true, e->s0);
-  CUDA_TRY(e, cudaGetLastError());
-  int st = check_device_status(e);
-  if (st) return st;
+  if (const int st = report_device_status(e)) return st;
+  if (forces) std::memcpy(forces, e->io_state, sizeof(double) * 3 * size_t(S0.n_atoms));
   if (out) {
-    for (int s : systems)
-      launch_molecular_offsets(d, e->mol_first[s], e->mol_count[s], e->sd[s].slot_off,
-                               e->mol_partials + size_t(e->mol_part_off[s]) * 9, e->s0);
-    CUDA_TRY(e, cudaGetLastError());
-    CUDA_TRY(e, cudaStreamSynchronize(e->s0));  // s0 does not order with the legacy stream
-  }
-  if (forces && !systems.empty()) {
-    const SysDev& S = e->sd[systems[0]];
-    std::vector<unsigned long long> f[3];
-    std::vector<int> order(S.n_slots);
-    for (auto& v : f) v.resize(S.n_slots);
-    CUDA_TRY(e, cudaMemcpy(f[0].data(), d.fx + S.slot_off, sizeof(long long) * S.n_slots, cudaMemcpyDeviceToHost));
-    CUDA_TRY(e, cudaMemcpy(f[1].data(), d.fy + S.slot_off, sizeof(long long) * S.n_slots, cudaMemcpyDeviceToHost));
-    CUDA_TRY(e, cudaMemcpy(f[2].data(), d.fz + S.slot_off, sizeof(long long) * S.n_slots, cudaMemcpyDeviceToHost));
-    CUDA_TRY(e, cudaMemcpy(order.data(), d.order + S.slot_off, sizeof(int) * S.n_slots, cudaMemcpyDeviceToHost));
-    for (int k = 0; k < S.n_slots; ++k) {
-      const int a = order[k];
-      if (a < 0) continue;
-      const int local = a - S.atom_off;
-      for (int ax = 0; ax < 3; ++ax) forces[3 * local + ax] = double((long long)f[ax][k]) / 4294967296.0;
-    }
-  }
-  if (out) {
-    std::vector<double> mol_all(size_t(e->mol_part_off.back() + molecular_offset_blocks(e->mol_count.back())) * 9);
-    CUDA_TRY(e, cudaMemcpy(mol_all.data(), e->mol_partials, sizeof(double) * mol_all.size(), cudaMemcpyDeviceToHost));
-    std::vector<unsigned long long> en(size_t(d.S) * kECount);
-    CUDA_TRY(e, cudaMemcpy(en.data(), d.energy, sizeof(long long) * en.size(), cudaMemcpyDeviceToHost));
-    std::vector<double> mesh(e->n_mesh_items), mesh_vir(size_t(e->n_mesh_items) * 6);
-    CUDA_TRY(e, cudaMemcpy(mesh.data(), d.mesh_partial, sizeof(double) * e->n_mesh_items, cudaMemcpyDeviceToHost));
-    CUDA_TRY(e, cudaMemcpy(mesh_vir.data(), d.mesh_virial, sizeof(double) * mesh_vir.size(), cudaMemcpyDeviceToHost));
     for (size_t i = 0; i < systems.size(); ++i) {
       const int s = systems[i];
       const HostSystem& h = e->hs[s];
       const SysDev& S = e->sd[s];
       mdb_energies& o = out[i];
       std::memset(&o, 0, sizeof(o));
-      const std::vector<double> mol_part(mol_all.begin() + size_t(e->mol_part_off[s]) * 9,
-                                         mol_all.begin() + size_t(e->mol_part_off[s] +
-                                                                  molecular_offset_blocks(e->mol_count[s])) * 9);
-      auto val = [&](int k) { return double((long long)en[size_t(S.energy_base) + k]) / 4294967296.0; };
+      const double* mol_part = e->io_mol + size_t(e->mol_part_off[s]) * 9;
+      const int mol_blocks = molecular_offset_blocks(e->mol_count[s]);
+      const unsigned long long* en = e->io_energy + S.energy_base;
+      auto val = [&](int k) { return double((long long)en[k]) / 4294967296.0; };
       double em = 0, wm[6] = {0, 0, 0, 0, 0, 0};
-      for (int k = 0; k < e->n_mesh_items; ++k)
-        if (e->fft_x_sys[k] == s) {
-          em += mesh[k];
-          for (int c = 0; c < 6; ++c) wm[c] += mesh_vir[size_t(k) * 6 + c];
-        }
+      for (int k = e->mesh_first[s]; k < e->mesh_first[s + 1]; ++k) {
+        em += e->io_mesh[k];
+        for (int c = 0; c < 6; ++c) wm[c] += e->io_mesh_virial[size_t(k) * 6 + c];
+      }
       o.bond = val(kEBond);
       o.angle = val(kEAngle);
       o.torsion = val(kETorsion);
@@ -1123,7 +1164,7 @@ int evaluate_many(mdb_engine* e, const std::vector<int>& systems, double* forces
       o.direct_lj = val(kELj);
       o.exclusion_correction = val(kEExclusion);
       o.exceptions = val(kEException);
-      o.pairs_within_cutoff = double(static_cast<long long>(en[size_t(S.energy_base) + kEPairs]));
+      o.pairs_within_cutoff = double(static_cast<long long>(en[kEPairs]));
       o.dispersion = h.dispersion_energy;
       o.reciprocal_mesh = em;
       o.self_energy = h.self_energy;
@@ -1143,32 +1184,29 @@ int evaluate_many(mdb_engine* e, const std::vector<int>& systems, double* forces
       // the molecular virial: minus the atoms' offsets from their molecule's centre
       for (int c = 0; c < 9; ++c) {
         double corr = 0;
-        for (size_t b = 0; b < mol_part.size() / 9; ++b) corr += mol_part[b * 9 + c];
+        for (int b = 0; b < mol_blocks; ++b) corr += mol_part[size_t(b) * 9 + c];
         o.molecular_virial[c] = o.virial[c] - corr;
       }
       o.potential = o.bond + o.angle + o.torsion + o.restraint + o.direct_group + o.reciprocal_group;
       // kinetic energy from the velocities as they are (kinetic.ts:31)
       if (kinetic) {
-        std::vector<float> v[3];
-        for (auto& x : v) x.resize(h.n);
-        CUDA_TRY(e, cudaMemcpy(v[0].data(), d.vx + S.atom_off, sizeof(float) * h.n, cudaMemcpyDeviceToHost));
-        CUDA_TRY(e, cudaMemcpy(v[1].data(), d.vy + S.atom_off, sizeof(float) * h.n, cudaMemcpyDeviceToHost));
-        CUDA_TRY(e, cudaMemcpy(v[2].data(), d.vz + S.atom_off, sizeof(float) * h.n, cudaMemcpyDeviceToHost));
+        if (i > 0) {  // the first system's came with the rest
+          const size_t n = size_t(h.n);
+          CUDA_TRY(e, cudaMemcpy(e->io_velocities, d.vx + S.atom_off, sizeof(float) * n, cudaMemcpyDeviceToHost));
+          CUDA_TRY(e, cudaMemcpy(e->io_velocities + n, d.vy + S.atom_off, sizeof(float) * n, cudaMemcpyDeviceToHost));
+          CUDA_TRY(e, cudaMemcpy(e->io_velocities + 2 * n, d.vz + S.atom_off, sizeof(float) * n, cudaMemcpyDeviceToHost));
+        }
+        const float *vx = e->io_velocities, *vy = vx + h.n, *vz = vy + h.n;
         double ke = 0;
         for (int a = 0; a < h.n; ++a)
           if (h.mass[a] > 0)
-            ke += h.mass[a] * (double(v[0][a]) * v[0][a] + double(v[1][a]) * v[1][a] + double(v[2][a]) * v[2][a]);
+            ke += h.mass[a] * (double(vx[a]) * vx[a] + double(vy[a]) * vy[a] + double(vz[a]) * vz[a]);
         o.kinetic = 0.5 * ke;
         o.degrees_of_freedom = h.dof;
         o.temperature = h.dof > 0 ? 2 * o.kinetic / (h.dof * kBoltzmann) : 0;
       }
     }
   }
-  // the step loop expects cleared accumulators
-  CUDA_TRY(e, cudaMemsetAsync(d.fx, 0, sizeof(long long) * d.n_slots, e->s0));
-  CUDA_TRY(e, cudaMemsetAsync(d.fy, 0, sizeof(long long) * d.n_slots, e->s0));
-  CUDA_TRY(e, cudaMemsetAsync(d.fz, 0, sizeof(long long) * d.n_slots, e->s0));
-  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
   return MDB_OK;
 }
 
@@ -1178,39 +1216,43 @@ int evaluate(mdb_engine* e, int s, double* forces, mdb_energies* out, bool kinet
 
 int get_positions(mdb_engine* e, int s, double* out) {
   const SysDev& S = e->sd[s];
-  const int n = S.n_atoms;
-  std::vector<long long> p[3];
-  for (auto& v : p) v.resize(n);
+  launch_positions_out(e->d, S.atom_off, S.n_atoms, e->io_state, e->s0);
+  CUDA_TRY(e, cudaGetLastError());
   CUDA_TRY(e, cudaStreamSynchronize(e->s0));
-  CUDA_TRY(e, cudaMemcpy(p[0].data(), e->d.px + S.atom_off, sizeof(long long) * n, cudaMemcpyDeviceToHost));
-  CUDA_TRY(e, cudaMemcpy(p[1].data(), e->d.py + S.atom_off, sizeof(long long) * n, cudaMemcpyDeviceToHost));
-  CUDA_TRY(e, cudaMemcpy(p[2].data(), e->d.pz + S.atom_off, sizeof(long long) * n, cudaMemcpyDeviceToHost));
-  for (int a = 0; a < n; ++a)
-    for (int k = 0; k < 3; ++k) out[3 * a + k] = double(p[k][a]) / 4294967296.0;
+  std::memcpy(out, e->io_state, sizeof(double) * 3 * size_t(S.n_atoms));
+  return MDB_OK;
+}
+
+int get_velocities(mdb_engine* e, int s, double* out) {
+  const SysDev& S = e->sd[s];
+  launch_velocities_out(e->d, S.atom_off, S.n_atoms, e->io_state, e->s0);
+  CUDA_TRY(e, cudaGetLastError());
+  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
+  std::memcpy(out, e->io_state, sizeof(double) * 3 * size_t(S.n_atoms));
   return MDB_OK;
 }
 
 int set_positions(mdb_engine* e, int s, const double* in, bool clear_residual) {
   const SysDev& S = e->sd[s];
-  const int n = S.n_atoms;
-  std::vector<long long> p[3];
-  for (auto& v : p) v.resize(n);
-  for (int a = 0; a < n; ++a)
-    for (int k = 0; k < 3; ++k) {
-      if (!std::isfinite(in[3 * a + k]) || std::fabs(in[3 * a + k]) > 1.0e6)
-        return fail(e, MDB_ERR_RANGE, "positions must be finite and inside the fixed-point range");
-      p[k][a] = to_fixed_host(in[3 * a + k]);
-    }
+  bool fine = true;
+  for (int k = 0; k < 3 * S.n_atoms; ++k) fine &= std::fabs(in[k]) <= 1.0e6;  // false for a NaN too
+  if (!fine) return fail(e, MDB_ERR_RANGE, "positions must be finite and inside the fixed-point range");
   CUDA_TRY(e, cudaStreamSynchronize(e->s0));
-  CUDA_TRY(e, cudaMemcpy(e->d.px + S.atom_off, p[0].data(), sizeof(long long) * n, cudaMemcpyHostToDevice));
-  CUDA_TRY(e, cudaMemcpy(e->d.py + S.atom_off, p[1].data(), sizeof(long long) * n, cudaMemcpyHostToDevice));
-  CUDA_TRY(e, cudaMemcpy(e->d.pz + S.atom_off, p[2].data(), sizeof(long long) * n, cudaMemcpyHostToDevice));
-  if (clear_residual) {
-    CUDA_TRY(e, cudaMemset(e->d.rx + S.atom_off, 0, sizeof(float) * n));
-    CUDA_TRY(e, cudaMemset(e->d.ry + S.atom_off, 0, sizeof(float) * n));
-    CUDA_TRY(e, cudaMemset(e->d.rz + S.atom_off, 0, sizeof(float) * n));
-  }
+  std::memcpy(e->io_state, in, sizeof(double) * 3 * size_t(S.n_atoms));
+  launch_positions_in(e->d, S.atom_off, S.n_atoms, e->io_state, clear_residual, e->s0);
+  CUDA_TRY(e, cudaGetLastError());
   return request_rebuild(e, s);
+}
+
+int set_velocities(mdb_engine* e, int s, const double* in) {
+  const SysDev& S = e->sd[s];
+  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
+  std::memcpy(e->io_state, in, sizeof(double) * 3 * size_t(S.n_atoms));
+  launch_velocities_in(e->d, S.atom_off, S.n_atoms, e->io_state, e->s0);
+  launch_momentum(e->d, e->s0);
+  CUDA_TRY(e, cudaGetLastError());
+  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
+  return MDB_OK;
 }
 
 int set_box(mdb_engine* e, int s, const double* box) {
@@ -1728,6 +1770,7 @@ int mdb_destroy(mdb_engine* e, int64_t* leaked_bytes) {
   int64_t leaked = 0;
   for (auto& a : e->allocs)
     if (cudaFree(a.ptr) != cudaSuccess) leaked += int64_t(a.bytes);
+  if (e->pinned) cudaFreeHost(e->pinned);
   for (cudaEvent_t ev : {e->fork, e->listed, e->join1, e->join2, e->t0, e->t1})
     if (ev) cudaEventDestroy(ev);
   for (cudaStream_t s : {e->s0, e->s1, e->s2})
@@ -1850,19 +1893,8 @@ int mdb_get_positions(mdb_engine* e, int32_t s, double* out) {
 
 int mdb_get_velocities(mdb_engine* e, int32_t s, double* out) {
   if (bad_system(e, s) || !out) return MDB_ERR_INVALID_ARGUMENT;
-  const SysDev& S = e->sd[s];
-  const int n = S.n_atoms;
-  std::vector<float> v[3];
-  for (auto& x : v) x.resize(n);
-  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
-  CUDA_TRY(e, cudaMemcpy(v[0].data(), e->d.vx + S.atom_off, sizeof(float) * n, cudaMemcpyDeviceToHost));
-  CUDA_TRY(e, cudaMemcpy(v[1].data(), e->d.vy + S.atom_off, sizeof(float) * n, cudaMemcpyDeviceToHost));
-  CUDA_TRY(e, cudaMemcpy(v[2].data(), e->d.vz + S.atom_off, sizeof(float) * n, cudaMemcpyDeviceToHost));
-  for (int a = 0; a < n; ++a)
-    for (int k = 0; k < 3; ++k) out[3 * a + k] = v[k][a];
-  return MDB_OK;
+  return get_velocities(e, s, out);
 }
-
 int mdb_set_positions(mdb_engine* e, int32_t s, const double* positions) {
   if (bad_system(e, s) || !positions) return MDB_ERR_INVALID_ARGUMENT;
   return set_positions(e, s, positions, true);
@@ -1870,19 +1902,7 @@ int mdb_set_positions(mdb_engine* e, int32_t s, const double* positions) {
 
 int mdb_set_velocities(mdb_engine* e, int32_t s, const double* velocities) {
   if (bad_system(e, s) || !velocities) return MDB_ERR_INVALID_ARGUMENT;
-  const SysDev& S = e->sd[s];
-  const int n = S.n_atoms;
-  std::vector<float> v[3];
-  for (auto& x : v) x.resize(n);
-  for (int a = 0; a < n; ++a)
-    for (int k = 0; k < 3; ++k) v[k][a] = float(velocities[3 * a + k]);
-  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
-  CUDA_TRY(e, cudaMemcpy(e->d.vx + S.atom_off, v[0].data(), sizeof(float) * n, cudaMemcpyHostToDevice));
-  CUDA_TRY(e, cudaMemcpy(e->d.vy + S.atom_off, v[1].data(), sizeof(float) * n, cudaMemcpyHostToDevice));
-  CUDA_TRY(e, cudaMemcpy(e->d.vz + S.atom_off, v[2].data(), sizeof(float) * n, cudaMemcpyHostToDevice));
-  launch_momentum(e->d, e->s0);
-  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
-  return MDB_OK;
+  return set_velocities(e, s, velocities);
 }
 
 int mdb_set_box(mdb_engine* e, int32_t s, const double box[9]) {
@@ -1909,13 +1929,19 @@ int mdb_evaluate(mdb_engine* e, int32_t s, double* forces, mdb_energies* energie
 
 int mdb_potential(mdb_engine* e, int32_t s, const double* positions, double* forces, mdb_energies* energies) {
   if (bad_system(e, s) || !positions) return MDB_ERR_INVALID_ARGUMENT;
-  const int n = e->hs[s].n;
-  std::vector<double> saved(3 * n);
-  int st = get_positions(e, s, saved.data());
+  // the positions wait in the volume moves' backup, free between barostat rounds
+  const SysDev& S = e->sd[s];
+  const size_t bytes = sizeof(long long) * size_t(S.n_atoms);
+  const Dev& d = e->d;
+  CUDA_TRY(e, cudaMemcpyAsync(d.bx + S.atom_off, d.px + S.atom_off, bytes, cudaMemcpyDeviceToDevice, e->s0));
+  CUDA_TRY(e, cudaMemcpyAsync(d.by + S.atom_off, d.py + S.atom_off, bytes, cudaMemcpyDeviceToDevice, e->s0));
+  CUDA_TRY(e, cudaMemcpyAsync(d.bz + S.atom_off, d.pz + S.atom_off, bytes, cudaMemcpyDeviceToDevice, e->s0));
+  int st = set_positions(e, s, positions, false);
   if (st) return st;
-  if ((st = set_positions(e, s, positions, false))) return st;
   st = evaluate(e, s, forces, energies);
-  const int restore = set_positions(e, s, saved.data(), false);
+  launch_restore_positions(d, S.atom_off, S.n_atoms, e->s0);
+  CUDA_TRY(e, cudaGetLastError());
+  const int restore = request_rebuild(e, s);
   return st ? st : restore;
 }
 
