@@ -5,9 +5,9 @@
 // replace the reference's per-step command-buffer encoding
 // (src/gpu/loop.ts:715-751).  One step is
 //
-//   list kernels (return at once unless a rebuild was asked for)
-//   wrap
-//   fork:  nonbonded tiles (s0) | listed terms (s2) | PME chain (s1)
+//   fork:  list kernels (s0; return at once unless a rebuild or a prune is due)
+//          | PME spread and transforms (s1)
+//          nonbonded tiles (s0) | listed terms (s2) | PME gather (s1)
 //   join:  fused integrator (s0)
 //
 // and `max_batch` such steps are captured once and replayed.  Nothing on this
@@ -332,8 +332,8 @@ int report_device_status(mdb_engine* e) {
   return MDB_OK;
 }
 
-// Sort, wrap and tile list: one cooperative launch when the device can, else
-// the phase kernels one by one.
+// The lists: one cooperative launch when the device can, else the phase kernels
+// one by one; then the inner list.
 void list_kernels(mdb_engine* e, cudaStream_t st) {
   if (!(e->coop_list && launch_list(e->d, st))) {
     launch_prune_references(e->d, st);

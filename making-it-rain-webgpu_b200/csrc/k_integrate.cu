@@ -4,15 +4,16 @@
 // SHAKE/SETTLE -> finish, one dispatch each, because its constraint solvers
 // are separate passes (src/gpu/kernels/integrate.wgsl:140-203, settle.wgsl,
 // shake.wgsl; oracle src/reference/integrator.ts:140-220).  Constraints never
-// couple two clusters, so here one thread owns one *integration unit* -- a
-// SETTLE water, a SHAKE cluster (<= 8 atoms, <= 8 constraints), or a free atom
-// -- and carries it through every phase in registers:
+// couple two clusters, so here a block takes 32 *integration units* -- SETTLE
+// waters, SHAKE clusters (<= 8 atoms, <= 8 constraints), free atoms -- through
+// every phase, their atoms in shared memory:
 //
 //   COM removal (com-motion.ts:48, on removesOnStep)
 //   kick          v += dt F / m
 //   SETTLE-v / RATTLE
 //   drift         x' = x + v dt/2 (+ residual); v = e^{-g dt} v + noise; x' += v dt/2
-//   SETTLE / SHAKE (Jacobi, reference bond vectors, FP64 convergence test)
+//   SETTLE / SHAKE (reference bond vectors, FP64 convergence test; Newton for
+//                   X-H_n stars, Jacobi sweeps for other clusters)
 //   finish        v += (x'' - x')/dt; x = x''
 //
 // and then the things the next step needs: the displacement test that asks for
