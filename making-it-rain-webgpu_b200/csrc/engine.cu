@@ -151,6 +151,16 @@ int fail(mdb_engine* e, int status, const std::string& message) {
     }                                                                                            \
   } while (0)
 
+// Everything the host writes to the engine's tables goes through its own
+// stream: s0 does not order with the legacy default stream, where a device
+// memset, and a copy from pageable memory, may still be at work when the call
+// that made it returns.  (Before the streams exist s0 is null: creation writes
+// on the legacy stream and waits for the device before the first launch.)
+cudaError_t put(mdb_engine* e, void* to, const void* from, size_t bytes) {
+  return cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, e->s0);
+}
+cudaError_t clear(mdb_engine* e, void* to, size_t bytes) { return cudaMemsetAsync(to, 0, bytes, e->s0); }
+
 template <typename T>
 int alloc(mdb_engine* e, const char* label, T*& out, size_t count) {
   out = nullptr;
@@ -158,10 +168,10 @@ int alloc(mdb_engine* e, const char* label, T*& out, size_t count) {
   void* p = nullptr;
   cudaError_t err = cudaMalloc(&p, bytes);
   if (err != cudaSuccess) return fail(e, MDB_ERR_DEVICE, std::string("cudaMalloc ") + label + ": " + cudaGetErrorString(err));
-  err = cudaMemset(p, 0, bytes);
+  err = clear(e, p, bytes);
   if (err != cudaSuccess) {
     cudaFree(p);
-    return fail(e, MDB_ERR_DEVICE, std::string("cudaMemset ") + label + ": " + cudaGetErrorString(err));
+    return fail(e, MDB_ERR_DEVICE, std::string("cudaMemsetAsync ") + label + ": " + cudaGetErrorString(err));
   }
   e->allocs.push_back({label, p, bytes});
   out = static_cast<T*>(p);
@@ -172,7 +182,7 @@ template <typename T>
 int upload(mdb_engine* e, const char* label, T*& out, const std::vector<T>& host) {
   int st = alloc(e, label, out, host.size());
   if (st) return st;
-  if (!host.empty()) CUDA_TRY(e, cudaMemcpy(out, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice));
+  if (!host.empty()) CUDA_TRY(e, put(e, out, host.data(), host.size() * sizeof(T)));
   return MDB_OK;
 }
 
@@ -318,13 +328,13 @@ int report_device_status(mdb_engine* e) {
   if (any & kErrTimeout) {
     // the list kernel's grid barrier gave up: its count holds the blocks that
     // arrived; clear it and the bit so the next list build starts afresh
-    CUDA_TRY(e, cudaMemset(e->d.list_barrier, 0, 2 * sizeof(unsigned int)));
+    CUDA_TRY(e, clear(e, e->d.list_barrier, 2 * sizeof(unsigned int)));
     // and what the phases it cut short would have cleared
-    CUDA_TRY(e, cudaMemset(e->d.cell_cnt, 0, sizeof(int) * size_t(std::max(1, e->d.n_cells))));
-    CUDA_TRY(e, cudaMemset(e->d.chunk_cnt, 0, sizeof(int) * size_t(std::max(1, e->d.n_chunks))));
-    CUDA_TRY(e, cudaMemset(e->d.list_ticket, 0, sizeof(int)));
+    CUDA_TRY(e, clear(e, e->d.cell_cnt, sizeof(int) * size_t(std::max(1, e->d.n_cells))));
+    CUDA_TRY(e, clear(e, e->d.chunk_cnt, sizeof(int) * size_t(std::max(1, e->d.n_chunks))));
+    CUDA_TRY(e, clear(e, e->d.list_ticket, sizeof(int)));
     for (int& f : flags) f &= ~kErrTimeout;
-    CUDA_TRY(e, cudaMemcpy(e->d.err, flags.data(), sizeof(int) * e->d.S, cudaMemcpyHostToDevice));
+    CUDA_TRY(e, put(e, e->d.err, flags.data(), sizeof(int) * e->d.S));
     request_rebuild(e, -1);
     return fail(e, MDB_ERR_TIMEOUT, "a bounded device wait gave up");
   }
@@ -429,9 +439,9 @@ int grow_tile_list(mdb_engine* e) {
     release(e, p);
   d.tile_cap_total = int(total);
   if (const int st = alloc_tile_list(e)) return st;
-  CUDA_TRY(e, cudaMemcpy(const_cast<SysDev*>(d.sys), e->sd.data(), sizeof(SysDev) * d.S, cudaMemcpyHostToDevice));
-  CUDA_TRY(e, cudaMemcpy(d.err, err.data(), sizeof(int) * d.S, cudaMemcpyHostToDevice));
-  CUDA_TRY(e, cudaMemset(d.halt, 0, sizeof(int)));
+  CUDA_TRY(e, put(e, const_cast<SysDev*>(d.sys), e->sd.data(), sizeof(SysDev) * d.S));
+  CUDA_TRY(e, put(e, d.err, err.data(), sizeof(int) * d.S));
+  CUDA_TRY(e, clear(e, d.halt, sizeof(int)));
   e->list_grown += 1;
   return request_rebuild(e, -1);
 }
@@ -1267,8 +1277,7 @@ int set_box(mdb_engine* e, int s, const double* box) {
   std::copy(reduced, reduced + 9, e->box_at_rebuild[s].begin());
   update_box_constants(h);
   fill_box(h, e->sd[s], true);
-  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
-  CUDA_TRY(e, cudaMemcpy(const_cast<SysDev*>(e->d.sys) + s, &e->sd[s], sizeof(SysDev), cudaMemcpyHostToDevice));
+  CUDA_TRY(e, put(e, const_cast<SysDev*>(e->d.sys) + s, &e->sd[s], sizeof(SysDev)));
   launch_influence(e->d, s, e->s0);
   CUDA_TRY(e, cudaGetLastError());
   return request_rebuild(e, s);
@@ -1306,23 +1315,14 @@ int move_boxes(mdb_engine* e, const std::vector<int>& sys, const std::vector<std
     }
   }
   // every system's constants in one copy, after the work already queued
-  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
-  CUDA_TRY(e, cudaMemcpy(const_cast<SysDev*>(e->d.sys), e->sd.data(), sizeof(SysDev) * e->d.S,
-                         cudaMemcpyHostToDevice));
+  CUDA_TRY(e, put(e, const_cast<SysDev*>(e->d.sys), e->sd.data(), sizeof(SysDev) * e->d.S));
   launch_influence(e->d, sys.size() == 1 ? sys[0] : -1, e->s0);
   for (int s : sys)
     if (std::find(rebuild.begin(), rebuild.end(), s) == rebuild.end())
       launch_after_box_change(e->d, s, e->sd[s].n_slots, e->sd[s].tile_cap, e->s0);
   CUDA_TRY(e, cudaGetLastError());
-  if (!rebuild.empty()) {
-    std::vector<int> now(e->d.S, 0);
-    CUDA_TRY(e, cudaStreamSynchronize(e->s0));
-    CUDA_TRY(e, cudaMemcpy(now.data(), e->d.rebuild_now, sizeof(int) * e->d.S, cudaMemcpyDeviceToHost));
-    for (int s : rebuild) now[s] = 1;
-    const int one = 1;
-    CUDA_TRY(e, cudaMemcpy(e->d.rebuild_now, now.data(), sizeof(int) * e->d.S, cudaMemcpyHostToDevice));
-    CUDA_TRY(e, cudaMemcpy(e->d.any_rebuild, &one, sizeof(int), cudaMemcpyHostToDevice));
-  }
+  for (int s : rebuild)
+    if (const int st = request_rebuild(e, s)) return st;
   return MDB_OK;
 }
 
@@ -1425,8 +1425,8 @@ int surrogate_train(mdb_engine* e, Surrogate& net, uint32_t seed, int epochs) {
       x[size_t(i) * kMlpIn + k] = float((feats[size_t(i) * kMlpIn + k] - net.mu[k]) / net.sd[k]);
     t[i] = float((target[i] - net.mu_t) / net.sd_t);
   }
-  CUDA_TRY(e, cudaMemcpy(net.x, x.data(), sizeof(float) * x.size(), cudaMemcpyHostToDevice));
-  CUDA_TRY(e, cudaMemcpy(net.t, t.data(), sizeof(float) * t.size(), cudaMemcpyHostToDevice));
+  CUDA_TRY(e, put(e, net.x, x.data(), sizeof(float) * x.size()));
+  CUDA_TRY(e, put(e, net.t, t.data(), sizeof(float) * t.size()));
   net.dev.lr = 2e-3f;
   net.dev.beta1 = 0.9f;
   net.dev.beta2 = 0.999f;
@@ -1873,9 +1873,8 @@ int mdb_run_timed(mdb_engine* e, int64_t steps, double* device_ms) {
 
 int mdb_set_step(mdb_engine* e, int64_t step) {
   if (!e || step < 0) return MDB_ERR_INVALID_ARGUMENT;
-  CUDA_TRY(e, cudaStreamSynchronize(e->s0));
   std::vector<long long> v(e->d.S, step);
-  CUDA_TRY(e, cudaMemcpy(e->d.step, v.data(), sizeof(long long) * e->d.S, cudaMemcpyHostToDevice));
+  CUDA_TRY(e, put(e, e->d.step, v.data(), sizeof(long long) * e->d.S));
   e->step = step;
   return MDB_OK;
 }

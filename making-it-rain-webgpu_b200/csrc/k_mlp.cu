@@ -265,13 +265,12 @@ cudaError_t mlp_upload_weights(const MlpDev& m, const float* w, cudaStream_t st)
 // minibatch loss.
 cudaError_t mlp_train(const MlpDev& m, const float* x, const float* t, int n, int epochs, uint32_t seed,
                       float* loss_dev, std::vector<double>* epoch_loss, cudaStream_t st) {
-  std::vector<float> w(kMlpParams), zeros(kMlpParams, 0.f);
+  std::vector<float> w(kMlpParams);
   mlp_init_weights(seed, w.data());
   cudaError_t err = mlp_upload_weights(m, w.data(), st);
-  const int zero = 0;
-  if (err == cudaSuccess) err = cudaMemcpy(m.m, zeros.data(), sizeof(float) * kMlpParams, cudaMemcpyHostToDevice);
-  if (err == cudaSuccess) err = cudaMemcpy(m.v, zeros.data(), sizeof(float) * kMlpParams, cudaMemcpyHostToDevice);
-  if (err == cudaSuccess) err = cudaMemcpy(m.step_count, &zero, sizeof(int), cudaMemcpyHostToDevice);
+  if (err == cudaSuccess) err = cudaMemsetAsync(m.m, 0, sizeof(float) * kMlpParams, st);
+  if (err == cudaSuccess) err = cudaMemsetAsync(m.v, 0, sizeof(float) * kMlpParams, st);
+  if (err == cudaSuccess) err = cudaMemsetAsync(m.step_count, 0, sizeof(int), st);
   static const int kPrimes[] = {7919, 104729, 15485863, 32452843, 49979687};
   const int batches = (n + kMlpBatch - 1) / kMlpBatch;
   std::vector<float> losses(batches);
