@@ -1702,6 +1702,25 @@ int run(mdb_engine* e, int64_t steps) {
   return check_device_status(e);
 }
 
+// The engine's device made the calling thread's for the length of a call: a
+// launch, unlike a copy, needs its stream's device current, and a program with
+// engines on several devices reads their states in any order.
+class OnDevice {
+ public:
+  explicit OnDevice(const mdb_engine* e) {
+    if (cudaGetDevice(&before_) != cudaSuccess || before_ == e->device) before_ = -1;
+    else cudaSetDevice(e->device);
+  }
+  ~OnDevice() {
+    if (before_ >= 0) cudaSetDevice(before_);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+
+ private:
+  int before_ = -1;
+};
+
 bool bad_system(const mdb_engine* e, int32_t s) { return !e || s < 0 || s >= int32_t(e->hs.size()); }
 
 // Kernels one graph-replayed step launches: the list kernels (one cooperative
@@ -1854,11 +1873,13 @@ int mdb_autotune_batch(int32_t n, const mdb_system_desc* systems, const mdb_stat
 
 int mdb_run(mdb_engine* e, int64_t steps) {
   if (!e || steps < 0) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   return run(e, steps);
 }
 
 int mdb_run_timed(mdb_engine* e, int64_t steps, double* device_ms) {
   if (!e || steps < 0 || !device_ms) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   CUDA_TRY(e, cudaStreamSynchronize(e->s0));
   CUDA_TRY(e, cudaEventRecord(e->t0, e->s0));
   int st = run(e, steps);
@@ -1873,6 +1894,7 @@ int mdb_run_timed(mdb_engine* e, int64_t steps, double* device_ms) {
 
 int mdb_set_step(mdb_engine* e, int64_t step) {
   if (!e || step < 0) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   std::vector<long long> v(e->d.S, step);
   CUDA_TRY(e, put(e, e->d.step, v.data(), sizeof(long long) * e->d.S));
   e->step = step;
@@ -1887,25 +1909,31 @@ int mdb_get_step(const mdb_engine* e, int64_t* step) {
 
 int mdb_get_positions(mdb_engine* e, int32_t s, double* out) {
   if (bad_system(e, s) || !out) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   return get_positions(e, s, out);
 }
 
 int mdb_get_velocities(mdb_engine* e, int32_t s, double* out) {
   if (bad_system(e, s) || !out) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   return get_velocities(e, s, out);
 }
+
 int mdb_set_positions(mdb_engine* e, int32_t s, const double* positions) {
   if (bad_system(e, s) || !positions) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   return set_positions(e, s, positions, true);
 }
 
 int mdb_set_velocities(mdb_engine* e, int32_t s, const double* velocities) {
   if (bad_system(e, s) || !velocities) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   return set_velocities(e, s, velocities);
 }
 
 int mdb_set_box(mdb_engine* e, int32_t s, const double box[9]) {
   if (bad_system(e, s) || !box) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   return set_box(e, s, box);
 }
 
@@ -1923,11 +1951,13 @@ int mdb_get_mesh(const mdb_engine* e, int32_t s, int32_t mesh[3]) {
 
 int mdb_evaluate(mdb_engine* e, int32_t s, double* forces, mdb_energies* energies) {
   if (bad_system(e, s)) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   return evaluate(e, s, forces, energies);
 }
 
 int mdb_potential(mdb_engine* e, int32_t s, const double* positions, double* forces, mdb_energies* energies) {
   if (bad_system(e, s) || !positions) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   // the positions wait in the volume moves' backup, free between barostat rounds
   const SysDev& S = e->sd[s];
   const size_t bytes = sizeof(long long) * size_t(S.n_atoms);
@@ -2011,6 +2041,7 @@ int mdb_get_neighbour_stats(mdb_engine* e, int32_t s, mdb_neighbour_stats* out) 
 
 int mdb_profile_step(mdb_engine* e, int32_t repeats, mdb_profile* out) {
   if (!e || !out || repeats <= 0) return MDB_ERR_INVALID_ARGUMENT;
+  const OnDevice on(e);
   std::memset(out, 0, sizeof(*out));
   const Dev& d = e->d;
   cudaStream_t st = e->s0;

@@ -132,3 +132,28 @@ def test_volume_moves(fake, surrogate_attempts):
         loop.run(1)
     assert np.abs(loop.box_vectors(0) / 3.0 - np.eye(3)).max() > 0.01
     loop.destroy()
+
+
+def test_engines_on_two_devices(fake):
+    """Every call reaches its engine's device whichever is current, and leaves the caller's."""
+    from mdb200 import steploop, synth
+
+    system, state = synth.water_box(n_waters=300, width=3.0, seed=1)
+    loops = [steploop.StepLoop.from_parsed(system, state, steploop.RunOptions(seed=1, device=k)) for k in (0, 1)]
+    for current in (1, 0):
+        fake.cudaSetDevice(current)
+        for loop in loops:
+            loop.positions(), loop.velocities()
+            loop.set_positions(state.positions)
+            loop.set_velocities(state.velocities)
+            loop.set_box(state.box)
+            loop.run(2)
+            loop.run_timed(1)
+            loop.evaluate(), loop.potential(state.positions)
+            loop.profile_step(1)
+            loop.advance_step_count(3)
+            now = C.c_int(-1)
+            fake.cudaGetDevice(C.byref(now))
+            assert now.value == current
+    for loop in loops:
+        loop.destroy()
