@@ -333,8 +333,9 @@ __device__ __forceinline__ int spline_axis(const SysDev& S, int axis, long long 
 // the grid: an eighth to a quarter of the global atomics of spreading each
 // atom's 125 points directly.  The patch holds the block's spline bases
 // (unwrapped around its first atom) plus the 5-point stencil; a block whose
-// patch would not fit (a cluster torn across a jump of the curve) or whose
-// slots reach into the next system spreads directly.  The grid is int64 fixed
+// patch would not fit (a cluster torn across a jump of the curve), whose slots
+// reach into the next system or that holds a charge of 1,000 e or more (the
+// sums' 32-bit halves) spreads directly.  The grid is int64 fixed
 // point and every contribution the same value either way, so the grid is the
 // same to the bit whatever the order and the route.  What bounds it is a
 // block's chain of loads, splines, shared atomics and grid atomics; hence
@@ -344,6 +345,7 @@ __device__ __forceinline__ int spline_axis(const SysDev& S, int axis, long long 
 // (128) 45.6 -> 40.7 us, 64-system ensemble (128) 248 -> 229 us; the
 // octahedron at 128 slots took 26.2 us.
 constexpr int kPatchPoints = 4096;  // 32 KB in two 32-bit halves
+constexpr float kPatchCharge = 1000.f;  // e; any charge there is
 
 // x 2^32 rounded to an integer, as hi 2^20 + lo, for |x| < 1024: both
 // roundings are f32 additions of 1.5 2^23 (whose low bits then hold the
@@ -362,14 +364,15 @@ template <int P>
 __global__ void __launch_bounds__(kThreads) k_spread(Dev d) {
   wait_for_predecessor();
   // the patch's sums in two 32-bit halves (hi 2^20 + lo), so the adds are
-  // 32-bit shared atomics: at most P atoms add to a point, which keeps both
-  // halves far from overflow
+  // 32-bit shared atomics: at most P = 128 atoms of less than kPatchCharge add
+  // to a point, weights below 1, so |hi| < 2^29 and |lo| <= 2^26
   __shared__ int patch_hi[kPatchPoints], patch_lo[kPatchPoints];
   __shared__ int base[P][3];
   __shared__ float th[P][3][5];
   __shared__ float qs[P];
   __shared__ int sysk[P];
   __shared__ int lo[3], hi[3];
+  __shared__ bool heavy;  // some charge is beyond what the halves hold
   const int t = threadIdx.x;
   const int first = blockIdx.x * P;
   if (first >= d.n_slots) return;
@@ -384,6 +387,7 @@ __global__ void __launch_bounds__(kThreads) k_spread(Dev d) {
   if (t < 3) {
     lo[t] = 1 << 30;
     hi[t] = -(1 << 30);
+    heavy = false;
   }
   __syncthreads();
   // splines, a thread per atom and axis (a warp's lanes share the axis)
@@ -393,7 +397,9 @@ __global__ void __launch_bounds__(kThreads) k_spread(Dev d) {
     const int st = gs <= last && !one_system ? d.slot_sys[gs] : s;
     const bool live = a >= 0 && sys_active(d, st);
     if (axis == 0) {
-      qs[k] = live ? d.prm_atom[a].w : 0.f;
+      const float q = live ? d.prm_atom[a].w : 0.f;
+      if (!(fabsf(q) < kPatchCharge)) heavy = true;
+      qs[k] = q;
       sysk[k] = st;
     }
     if (live) {
@@ -426,7 +432,7 @@ __global__ void __launch_bounds__(kThreads) k_spread(Dev d) {
     }
     __syncthreads();
   }
-  bool patch = one_system;
+  bool patch = one_system && !heavy;
   int points = 1, ext[3];
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
@@ -446,18 +452,10 @@ __global__ void __launch_bounds__(kThreads) k_spread(Dev d) {
       const int ix = r / kPmeOrder, iy = r - ix * kPmeOrder;
       const float wxy = q * th[k][0][ix] * th[k][1][iy];
       const int row = ((base[k][0] - lx + ix) * ey + (base[k][1] - ly + iy)) * ez + (base[k][2] - lz);
-      const bool small = fabsf(wxy) < 1000.f;  // any charge there is; the weights are below 1
 #pragma unroll
       for (int iz = 0; iz < kPmeOrder; ++iz) {
-        const float x = wxy * th[k][2][iz];
         int h, l;
-        if (small) {
-          split_fixed(x, h, l);
-        } else {
-          const long long v = to_fixed(x);
-          h = static_cast<int>(v >> 20);
-          l = static_cast<int>(v & 0xFFFFF);
-        }
+        split_fixed(wxy * th[k][2][iz], h, l);
         atomicAdd(&patch_hi[row + iz], h);
         atomicAdd(&patch_lo[row + iz], l);
       }

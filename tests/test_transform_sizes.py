@@ -1,7 +1,7 @@
 """The mesh transforms and the charge spread at the sizes where they can go
 wrong: axes of one, two and three stages, odd planes (whose last z line has no
 partner), planes that fit shared memory and planes that do not, charges past
-the range of the spread's f32 fixed-point split, and spread blocks that hold
+the range of the spread's sums in shared memory, and spread blocks that hold
 the end of one system and the start of the next.
 
 Bounds: reciprocal forces against the f64 oracle at the 1e-5 relative RMS the
@@ -53,8 +53,8 @@ def test_mesh_forces_and_energy(mesh):
 @pytest.mark.parametrize("mesh", [(21, 15, 25), (24, 120, 120)])
 @pytest.mark.parametrize("charge", [1.0, 1500.0])
 def test_engine_mesh_forces(mesh, charge):
-    """The engine's own passes, whole planes and strips, and charges beyond
-    1,000 e, which the spread converts the long way."""
+    """The engine's own passes, whole planes and strips, at ordinary charges and
+    beyond 1,000 e."""
     from mdb200 import steploop
     from oracle import oracle
 
@@ -82,3 +82,25 @@ def test_spread_blocks_across_systems(counts):
         assert np.array_equal(batch.positions(k), alone.positions()), k
         alone.destroy()
     batch.destroy()
+
+
+@pytest.mark.parametrize("charge", [1.0, 990.0, 1010.0, 1e5, 1e7])
+def test_large_charges_close_together(charge):
+    """Two clumps of 32 like charges, each a compact block of the spread: below 1,000 e their sums meet in shared
+    memory, 32 bits at a time, from there they go straight to the 64-bit grid.  The mesh energy against the oracle's."""
+    from mdb200 import steploop
+    from mdb200.system import State
+    from oracle import oracle
+
+    system, state, _ = separated_charges()
+    rng = np.random.default_rng(4)
+    corner = np.stack(np.meshgrid(range(4), range(4), range(2), indexing="ij"), -1).reshape(-1, 3) * 0.1
+    width = state.box[0][0]
+    pos = np.concatenate([corner + 0.2 * width, corner + 0.6 * width]) + rng.uniform(-0.02, 0.02, size=(64, 3))
+    system.nonbonded.charge = charge * np.repeat([1.0, -0.9], 32) * rng.uniform(0.99, 1.01, size=64)
+    state = State(positions=pos, box=state.box)
+    want, _ = oracle.potential(system, pos, grid=(40, 36, 42))
+    loop = steploop.StepLoop.from_parsed(system, state, steploop.RunOptions(mesh=(40, 36, 42)))
+    got, _ = loop.evaluate()
+    loop.destroy()
+    assert abs(got["reciprocal_mesh"] - want["reciprocal_mesh"]) < ENERGY_REL * abs(want["reciprocal_mesh"])
