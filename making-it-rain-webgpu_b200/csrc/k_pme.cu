@@ -464,16 +464,18 @@ __global__ void __launch_bounds__(kThreads) k_spread(Dev d) {
     const unsigned plane_magic = magic_for(unsigned(ey * ez)), row_magic = magic_for(unsigned(ez));
     const int Kx = S.grid[0], Ky = S.grid[1], Kz = S.grid[2];
     unsigned long long* grid = d.qgrid + S.grid_off;
+    // the patch's first point, turned into the mesh (its unwrapped base lies
+    // within half a mesh of one in it): no point is then a second turn away,
+    // however short the axis and whether or not the first atom has a charge
+    const int ox = lx + (lx < 0 ? Kx : (lx >= Kx ? -Kx : 0)), oy = ly + (ly < 0 ? Ky : (ly >= Ky ? -Ky : 0)),
+              oz = lz + (lz < 0 ? Kz : (lz >= Kz ? -Kz : 0));
     for (int i = t; i < points; i += blockDim.x) {
       const long long v = static_cast<long long>(patch_hi[i]) * (1ll << 20) + patch_lo[i];
       if (!v) continue;
       const int px = int(quotient(unsigned(i), plane_magic)), rem = i - px * ey * ez;
       const int py = int(quotient(unsigned(rem), row_magic)), pz = rem - py * ez;
-      // unwrapped bases lie within half a mesh of one in it: one turn at most
-      int gx = lx + px, gy = ly + py, gz = lz + pz;
-      gx += gx < 0 ? Kx : (gx >= Kx ? -Kx : 0);
-      gy += gy < 0 ? Ky : (gy >= Ky ? -Ky : 0);
-      gz += gz < 0 ? Kz : (gz >= Kz ? -Kz : 0);
+      const int gx = ox + px - (ox + px >= Kx ? Kx : 0), gy = oy + py - (oy + py >= Ky ? Ky : 0),
+                gz = oz + pz - (oz + pz >= Kz ? Kz : 0);
       add_fixed64(grid + (static_cast<long long>(gx) * Ky + gy) * Kz + gz, v);
     }
   } else {

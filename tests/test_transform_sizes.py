@@ -104,3 +104,38 @@ def test_large_charges_close_together(charge):
     got, _ = loop.evaluate()
     loop.destroy()
     assert abs(got["reciprocal_mesh"] - want["reciprocal_mesh"]) < ENERGY_REL * abs(want["reciprocal_mesh"])
+
+
+@pytest.mark.parametrize("short", [0, 1, 2])
+@pytest.mark.parametrize("corner", range(8))
+def test_spread_on_an_axis_of_five_points(short, corner):
+    """Uncharged atoms share a block with charged ones and come first in it for some corner: on an axis as short as
+    the stencil the charged ones' unwrapped points then start as much as six points from the mesh's first.  The mesh
+    energy against the oracle's."""
+    from mdb200 import steploop
+    from mdb200.system import Nonbonded, State, System
+    from oracle import oracle
+
+    rng = np.random.default_rng(6)
+    width, n, empty = 3.0, 32, np.zeros(0, dtype=np.int32)
+    mesh = [24, 27, 28]
+    mesh[short] = 5
+    place = np.array([(corner >> k) & 1 for k in range(3)]) * 0.9 + 0.05
+    pos = np.tile(place, (n, 1)) + rng.uniform(-0.03, 0.03, size=(n, 3))  # of the box
+    charge = rng.uniform(0.5, 1.0, size=n)
+    charge[: n // 2] = 0.0
+    pos[: n // 2, short] = rng.uniform(0.62, 0.78, size=n // 2)  # base 4 of the five
+    pos[n // 2 :, short] = rng.uniform(0.02, 0.18, size=n // 2)  # base 1
+    order = rng.permutation(n)
+    pos, charge = pos[order] * width, charge[order]
+    box = np.eye(3) * width
+    system = System(masses=np.full(n, 10.0), box=box,
+                    nonbonded=Nonbonded(cutoff=0.5, ewald_tolerance=5e-4, charge=charge, sigma=np.full(n, 0.3),
+                                        epsilon=np.zeros(n), exception_p1=empty, exception_p2=empty,
+                                        exception_charge_prod=np.zeros(0), exception_sigma=np.zeros(0),
+                                        exception_epsilon=np.zeros(0), use_dispersion_correction=False))
+    want, _ = oracle.potential(system, pos, grid=tuple(mesh))
+    loop = steploop.StepLoop.from_parsed(system, State(positions=pos, box=box), steploop.RunOptions(mesh=mesh))
+    got, _ = loop.evaluate()
+    loop.destroy()
+    assert abs(got["reciprocal_mesh"] - want["reciprocal_mesh"]) < ENERGY_REL * abs(want["reciprocal_mesh"])
