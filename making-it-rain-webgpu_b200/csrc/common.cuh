@@ -54,7 +54,7 @@ enum ErrorBit : int {
 };
 
 // kUnitStar: a SHAKE cluster whose constraints all join atom 0 to atoms
-// 1..nc (X-H_n, nc <= 3), solved with compile-time sizes.
+// 1..nc (X-H_n, nc <= 3; atoms 1..nc have mass), solved with compile-time sizes.
 enum UnitKind : int { kUnitFree = 0, kUnitSettle = 1, kUnitShake = 2, kUnitStar = 3 };
 
 // Integrate blocks: kIntegrateUnits units per block, their atoms staged in a

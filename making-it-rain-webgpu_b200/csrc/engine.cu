@@ -689,11 +689,17 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
         u.dist[k] = float(h.cdist[c]);
       }
       // An X-H_n star (one atom in every constraint, nc = na - 1 <= 3) is
-      // reordered to centre first and spoke c at position c + 1.
+      // reordered to centre first and spoke c at position c + 1.  Its direct
+      // solve needs every spoke to move, which keeps the system positive
+      // definite however they lie; with massless spokes in one plane it has no
+      // unique solution, and such a cluster takes the general sweeps.
       if (u.nc >= 1 && u.nc <= 3 && u.na == u.nc + 1) {
         for (int centre : {int(u.ci[0]), int(u.cj[0])}) {
           bool star = true;
-          for (int k = 0; k < u.nc; ++k) star &= u.ci[k] == centre || u.cj[k] == centre;
+          for (int k = 0; k < u.nc; ++k) {
+            star &= u.ci[k] == centre || u.cj[k] == centre;
+            star &= h.mass[cl.atoms[u.ci[k] == centre ? u.cj[k] : u.ci[k]]] > 0;
+          }
           if (!star) continue;
           int atom[kMaxClusterAtoms];
           atom[0] = u.atom[centre];

@@ -247,9 +247,11 @@ __device__ __forceinline__ long long displace(float wanted, float& left_over) {
 // CH3: the velocities exactly, the positions by Newton's method (three
 // rounds) on the same equations, to the same convergence window.
 
-// x of A x = b (n = 1 to 3, A row-major) by elimination without pivoting: the
-// stars' matrices are dominated by the spokes' own terms.  A zero row (both
-// atoms massless) gives zero.
+// x of A x = b (n = 1 to 3, A row-major) by elimination without pivoting.  A
+// star's velocity matrix is (inverse centre mass) x (Gram matrix of the bonds)
+// plus each spoke's own inverse mass x squared length on the diagonal: spokes
+// that move (every star's do) make it positive definite however they lie.  A
+// zero row (a bond of no length) gives zero, as the sweeps do.
 template <int N>
 __device__ __forceinline__ void solve_small(double (*A)[N], double* b) {
 #pragma unroll

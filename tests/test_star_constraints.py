@@ -63,3 +63,30 @@ def test_star_step_meets_its_constraints(spokes, temperature):
     length = np.linalg.norm(x[system.constraint_p1] - x[system.constraint_p2], axis=1)
     assert np.abs(length / 0.109 - 1).max() < 2e-6
     loop.destroy()
+
+
+def test_massless_spokes_in_one_plane():
+    """Three fixed atoms around a moving one, in a plane with it: the velocity equations have no unique solution and
+    Jacobi's sweeps leave the motion out of the plane alone, which nothing constrains.  One slow step (lengths stay
+    inside the solver's window) against the oracle; the step moves an atom about 4e-5 nm."""
+    from mdb200 import steploop
+    from mdb200.system import State
+    from oracle import oracle
+
+    system, state = stars(3, 300.0)
+    rng = np.random.default_rng(5)
+    pos, vel = state.positions.copy(), np.zeros_like(state.positions)
+    for base in range(0, len(pos), 4):
+        u, v, w = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+        for k in range(3):
+            angle = 2 * np.pi * k / 3
+            pos[base + 1 + k] = pos[base] + 0.109 * (np.cos(angle) * u + np.sin(angle) * v)
+        vel[base] = 0.02 * (w + 0.3 * rng.normal(size=3))
+        system.masses[base + 1 : base + 4] = 0.0
+    state = State(positions=pos, box=state.box, velocities=vel)
+    loop = steploop.StepLoop.from_parsed(system, state, steploop.RunOptions(friction=0.0, seed=2))
+    loop.run(1)
+    want, _, _ = oracle.run(system, state, 1, friction=0.0, seed=2)
+    assert np.abs(want[::4] - pos[::4]).max() > 2e-5
+    assert np.abs(loop.positions() - want).max() < 4e-7
+    loop.destroy()
