@@ -21,14 +21,18 @@ int pme_minimum_grid(double alpha, double length, double tol) {
   return std::max(6, int(std::ceil(2 * alpha * length / (3 * std::pow(tol, 0.2)))));
 }
 
+bool is_smooth(int n) {
+  if (n < 1) return false;
+  for (int p : {2, 3, 5, 7})
+    while (n % p == 0) n /= p;
+  return n == 1;
+}
+
 // units.ts:78 -- the next 2/3/5/7-smooth size
 int smooth_size(int minimum) {
-  for (int n = std::max(1, minimum);; ++n) {
-    int r = n;
-    for (int p : {2, 3, 5, 7})
-      while (r % p == 0) r /= p;
-    if (r == 1) return n;
-  }
+  int n = std::max(1, minimum);
+  while (!is_smooth(n)) ++n;
+  return n;
 }
 
 template <typename T>
@@ -114,11 +118,11 @@ std::vector<double> bspline_moduli(int n) {
   return mod;
 }
 
-// Stages for the shared-memory Stockham FFT: radix 4 where it divides, then
-// 7, 5, 3, 2.  False for a length that is not 2/3/5/7-smooth.
+// Stages for the shared-memory Stockham FFT: the fewest (a stage is a pass
+// through shared memory and a barrier), and among those the smallest largest
+// radix; four at most up to 512 points (375 = 3 5 5 5).  False for a length
+// that is not 2/3/5/7-smooth.
 bool plan_radices(int n, unsigned* plan) {
-  // the fewest stages (a stage is a pass through shared memory and a barrier),
-  // and among those the smallest largest radix: n <= 10^8 in eight of them
   *plan = 0;
   unsigned best[9];
   int count = 0;
@@ -142,11 +146,10 @@ bool plan_radices(int n, unsigned* plan) {
         self(self, rest / int(r), depth + 1, r);
       }
   };
-  if (n < 1) return false;
-  if (n == 1) return true;
+  if (!is_smooth(n)) return false;
   search(search, n, 0, 2);
   for (int k = 0; k < count; ++k) *plan |= best[k] << (4 * k);
-  return count > 0;
+  return true;
 }
 
 // nonbonded.ts:107 (dispersion, grouped by class), :594 (net charge), :610 (self)
@@ -242,8 +245,7 @@ int prepare_system(const mdb_system_desc& in, const mdb_state_desc& state, const
     int g = opt.mesh[k] > 0 ? opt.mesh[k] : in.grid[k];
     // potential.ts:79 -- the mesh from the box *diagonal*
     if (g <= 0) g = smooth_size(pme_minimum_grid(h.alpha, h.box[k * 4], h.tolerance));
-    unsigned plan = 0;
-    if (!plan_radices(g, &plan)) {
+    if (!is_smooth(g)) {
       msg << "mesh size " << g << " is not 2/3/5/7-smooth, so the transform cannot do it";
       error = msg.str();
       return MDB_ERR_NOT_SMOOTH;

@@ -63,8 +63,9 @@ void perpendicular_widths(const double* box, double* out);
 double box_volume(const double* box);
 void inverse_box(const double* box, double* m);  // f = r . M, M[v*3+u]
 std::vector<double> bspline_moduli(int n);
-// The radices (2 to 10) of an n-point transform, four bits each from the first
-// stage up; false if n has a prime factor above 7.  As few stages as possible.
+// The radices (2 to 10) of an n-point transform (512 points at most), four bits
+// each from the first stage up; false if n has a prime factor above 7.  As few
+// stages as possible.
 bool plan_radices(int n, unsigned* plan);
 
 }  // namespace mdb

@@ -292,3 +292,14 @@ def test_mesh_axes_shorter_than_the_spline_are_refused_before_device_work(lib):
         status = lib.mdb_reciprocal_noalloc(1, dummy, dummy, box.ctypes.data_as(C.POINTER(C.c_double)), 3.0, mesh,
                                             dummy, dummy, None)
         assert status == abi.ERR_INVALID_ARGUMENT, (axes, status)
+
+
+@pytest.mark.parametrize("axis", [525, 1024, 5**9, 7**9, 2**30])
+def test_long_smooth_mesh_axes_are_refused_as_too_long(axis):
+    """Smooth axes above 512 points are too long, however many stages they would take, and not unsmooth."""
+    from mdb200 import steploop, synth
+
+    system, state = synth.water_box(n_waters=300, width=2.1, seed=5)
+    with pytest.raises(steploop.EngineError, match="exceeds the 512 points") as caught:
+        steploop.StepLoop.from_parsed(system, state, steploop.RunOptions(mesh=(24, axis, 24)))
+    assert not isinstance(caught.value, steploop.NotSmooth)
