@@ -131,30 +131,59 @@ def test_batch_equals_single(mdb, water):
     batch.destroy()
 
 
-def test_slot_ordered_spread_equals_atom_ordered_spread(mdb):
-    """An engine of 80k atoms spreads PME charges by slot through shared-memory
-    mesh patches, a single 10k-atom system by atom straight into the grid: the
-    same fixed-point sums, so eight systems batched advance exactly as each
-    does alone -- through steps that rebuild the list, whose snapshot of the
-    slot order the spread reads."""
+def test_spread_blocks_of_every_size_agree(mdb):
+    """The charge spread's blocks hold 32 slots in a 10k-atom engine, 64 from
+    296 blocks of them (18,881 slots) and 128 from 37,761: the same fixed-point
+    sums, so systems batched by two and by eight advance exactly as each does
+    alone -- through steps that rebuild the list, whose snapshot of the slot
+    order the spread reads."""
     from mdb200 import synth
 
     members = [synth.water_box(width=4.6, seed=20 + k) for k in range(8)]
-    assert sum(m[0].particle_count for m in members) >= 148 * 128  # the slot-ordered spread's threshold
-    assert members[0][0].particle_count < 148 * 128 - 128  # alone, each spreads by atom
+    slots = [-(-m[0].particle_count // 32) * 32 for m in members]
+    assert slots[0] < 295 * 64 and 295 * 64 < sum(slots[:2]) < 295 * 128 < sum(slots)
     single = []
     for system, state in members:
         loop = make_loop(mdb, system, state, seed=6)
         loop.run(30)
         single.append(loop.positions())
         loop.destroy()
-    batch = mdb.StepLoop.batch([m[0] for m in members], [m[1] for m in members], mdb.RunOptions(seed=6))
-    batch.run(30)
-    rebuilds = [batch.verlet_flags(k)["rebuilds"] for k in range(len(members))]
-    print("rebuilds per system", rebuilds)
-    for k in range(len(members)):
-        assert np.array_equal(batch.positions(k), single[k]), k
-    batch.destroy()
+    for count in (2, 8):
+        batch = mdb.StepLoop.batch([m[0] for m in members[:count]], [m[1] for m in members[:count]],
+                                   mdb.RunOptions(seed=6))
+        batch.run(30)
+        assert all(batch.verlet_flags(k)["rebuilds"] > 1 for k in range(count))
+        for k in range(count):
+            assert np.array_equal(batch.positions(k), single[k]), (count, k)
+        batch.destroy()
+
+
+@pytest.mark.parametrize("copies", [1, 2, 4])
+def test_spread_by_slot_against_spread_by_atom(mdb, copies):
+    """A dense system, whose blocks sum in shared memory at each block size,
+    against the allocation-free call, which adds atom by atom: the grids are
+    the same integers, so the mesh energies differ by the f32 tables alone (a
+    few 2^-24; one atom's charge lost or doubled shifts them by about 1e-4)."""
+    import ctypes as C
+
+    import torch
+    from mdb200 import abi, synth
+
+    system, state = synth.water_box(width=4.6, seed=20)
+    loop = mdb.StepLoop.batch([system] * copies, [state] * copies, mdb.RunOptions(seed=6))
+    n, mesh = system.particle_count, loop.mesh()
+    pos, q = torch.from_numpy(state.positions).cuda(), torch.from_numpy(system.nonbonded.charge).cuda()
+    forces = torch.empty((n, 3), dtype=torch.float64, device="cuda")
+    energy = torch.empty(1, dtype=torch.float64, device="cuda")
+    alpha = np.sqrt(-np.log(2 * system.nonbonded.ewald_tolerance)) / system.nonbonded.cutoff
+    status = abi.load().mdb_reciprocal_noalloc(
+        n, pos.data_ptr(), q.data_ptr(), (C.c_double * 9)(*np.asarray(state.box).reshape(9)), alpha,
+        (C.c_int32 * 3)(*mesh), forces.data_ptr(), energy.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert status == abi.OK
+    for k in range(copies):
+        got = loop.evaluate(k)[0]["reciprocal_mesh"]
+        assert abs(got - energy.item()) < 1e-6 * abs(got)
+    loop.destroy()
 
 
 def test_set_box_equals_an_engine_created_at_that_box(mdb):

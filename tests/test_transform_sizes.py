@@ -1,5 +1,5 @@
 """The mesh transforms and the charge spread at the sizes where they can go
-wrong: axes of one, two and three stages, odd planes (whose last z line has no
+wrong: axes of one to four stages, odd planes (whose last z line has no
 partner), planes that fit shared memory and planes that do not, charges past
 the range of the spread's sums in shared memory, and spread blocks that hold
 the end of one system and the start of the next.
@@ -21,9 +21,10 @@ from test_zz_no_alloc import ENERGY_REL, RECIPROCAL_FORCE_REL_RMS, separated_cha
 
 pytestmark = pytest.mark.gpu
 
-# one stage; odd; three stages (7^3 is past 128, 98 = 2 7^2 is three); both
-# sides of the plane kernels' shared memory; the largest
-MESHES = [(10, 9, 8), (21, 15, 25), (35, 27, 49), (98, 27, 14), (20, 100, 128), (18, 125, 63), (64, 64, 64)]
+# one stage; odd; three stages on x, on y and z of whole planes (75, 98, 112; 75 is odd) and in strips; both sides
+# of the plane kernels' shared memory; the largest
+MESHES = [(10, 9, 8), (21, 15, 25), (35, 27, 49), (98, 27, 14), (12, 75, 75), (9, 98, 50), (9, 30, 112), (20, 100, 128),
+          (18, 125, 63), (64, 64, 64)]
 
 
 @pytest.mark.parametrize("mesh", MESHES)
@@ -50,11 +51,12 @@ def test_mesh_forces_and_energy(mesh):
         assert abs(energy.item() - want["reciprocal_mesh"]) < ENERGY_REL * abs(want["reciprocal_mesh"])
 
 
-@pytest.mark.parametrize("mesh", [(21, 15, 25), (24, 120, 120)])
+@pytest.mark.parametrize("mesh", [(21, 15, 25), (75, 84, 96), (96, 98, 75), (25, 105, 112), (24, 30, 375),
+                                  (375, 24, 27), (24, 120, 120)])
 @pytest.mark.parametrize("charge", [1.0, 1500.0])
 def test_engine_mesh_forces(mesh, charge):
-    """The engine's own passes, whole planes and strips, at ordinary charges and
-    beyond 1,000 e."""
+    """The engine's own passes, at ordinary charges and beyond 1,000 e: whole planes of two-stage and of three-stage
+    axes, four stages, and strips."""
     from mdb200 import steploop
     from oracle import oracle
 
@@ -64,7 +66,10 @@ def test_engine_mesh_forces(mesh, charge):
     loop = steploop.StepLoop.from_parsed(system, state, steploop.RunOptions(mesh=mesh))
     _, got = loop.evaluate()
     loop.destroy()
-    assert np.sqrt(((got - want) ** 2).sum() / (want**2).sum()) < RECIPROCAL_FORCE_REL_RMS
+    # a force is the difference of neighbouring points' f32 potentials over their distance: past 100 points on these
+    # 3 nm the potentials' rounding grows with the points (radix-4 transforms of 375 points: 3.8e-5)
+    bound = RECIPROCAL_FORCE_REL_RMS * max(1.0, max(mesh) / 100)
+    assert np.sqrt(((got - want) ** 2).sum() / (want**2).sum()) < bound
 
 
 @pytest.mark.parametrize("counts", [(672, 700), (672, 683, 691, 705, 672, 690, 750)])
