@@ -198,9 +198,8 @@ void release(mdb_engine* e, void* ptr) {
 }
 
 // The tile-list arrays, sized by the systems' tile capacities (tile_cap):
-// tiles, their interaction-mask words (C * C / 32 a tile), shifts and
-// survival flags for the fill pass's raw list and for the list the pair
-// kernel reads, and the inner list's copies.
+// tiles, their interaction-mask words (C * C / 32 a tile) and shifts, and the
+// inner list's copies.
 int alloc_tile_list(mdb_engine* e) {
   Dev& d = e->d;
   const size_t n = size_t(d.tile_cap_total), words = size_t(e->cluster * e->cluster / 32);
@@ -1057,7 +1056,7 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
     if (!halted || attempt == 4) break;
     if (const int st = grow_tile_list(e)) return st;
   }
-  // the slot-ordered spread's copy of the order, until the first step writes it
+  // the spread's copy of the order, until the first step writes it
   if (e->d.n_slots)
     CUDA_TRY(e, cudaMemcpyAsync(e->d.spread_atom, e->d.order, sizeof(int) * size_t(e->d.n_slots),
                                 cudaMemcpyDeviceToDevice, e->s0));
@@ -1085,9 +1084,14 @@ int build_engine(mdb_engine* e, int n, const mdb_system_desc* systems, const mdb
   if (e->opt.flags & MDB_FLAG_PHASE_LAUNCHES) e->coop_list = false;
   // A large batch rebuilds some system's list nearly every step; its search
   // phases then want the full grids of separate launches more than the
-  // cooperative kernel's two blocks per SM (64-system ensemble, 627k atoms:
-  // 3.51 against 3.56 ms per step), and a step of milliseconds hides the
-  // thirteen launches.  Single systems and small batches keep the one launch.
+  // cooperative kernel's two blocks per SM, and a step of milliseconds hides
+  // the eight launches.  Single systems and small batches keep the one launch.
+  // A step in one launch and in separate ones, us, with an inner list (skin
+  // 0.4) and with default lists: 4 systems, 29k atoms 137, 140 and 183, 158; 8,
+  // 67k 312, 300 and 429, 329; 16, 177k 701, 690 and 908, 754; 24, 378k 1322,
+  // 1297 and 1556, 1397; 40, 602k 2069, 2025 and 2366, 2140.  The line is on
+  // the safe side: separate launches win from about 67k atoms on, and with
+  // default lists from 29k.
   if (d.S > 1 && d.n_slots >= (1 << 18)) e->coop_list = false;
   return MDB_OK;
 }
@@ -2122,10 +2126,6 @@ int mdb_profile_step(mdb_engine* e, int32_t repeats, mdb_profile* out) {
   CUDA_TRY(e, cudaMemsetAsync(d.fy, 0, sizeof(long long) * d.n_slots, st));
   CUDA_TRY(e, cudaMemsetAsync(d.fz, 0, sizeof(long long) * d.n_slots, st));
   out->ms_integrate = time([&] { launch_integrate(d, st); });
-  // per step: the list kernels (one cooperative launch, or 5 sort + 1 wrap +
-  // 6 tile-list kernels, 3 more when rebuilds prune), the inner-list kernel,
-  // PME (spread, 3 transform passes or 5 without the plane kernels, gather),
-  // listed, nonbonded, integrator
   out->launches_per_step = launches_per_step(e);
   CUDA_TRY(e, cudaMemsetAsync(d.fx, 0, sizeof(long long) * d.n_slots, st));
   CUDA_TRY(e, cudaMemsetAsync(d.fy, 0, sizeof(long long) * d.n_slots, st));

@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(kThreads) k_exclusions(Dev d) {
   if (*d.any_rebuild) phase_exclusions_finish<C>(d);
 }
 // The inner list, its own launch after the list kernels (a full grid, where
-// the cooperative list kernel has two blocks per SM): nothing to do unless a
+// the cooperative list kernel has one or two blocks per SM): nothing to do unless a
 // system rebuilt or is due a prune.  The last block to finish writes the
 // offsets and clears the requests; every block has read them by then, since
 // each reads them before taking its ticket.
@@ -1075,9 +1075,13 @@ bool launch_list(const Dev& d, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   // Two blocks per SM, or one where an inner list makes rebuilds rare and the
   // system is small: most launches then find nothing to do, and the fewer
-  // blocks cost the spread beside them less (27k-atom octahedron: step 117 us
-  // with one, 123 with two, though its rebuild takes 267 instead of 219 us; 100k
-  // atoms: 400 and 392 us, rebuild 566 and 414).  Rebuilds before the phases
+  // blocks cost the spread beside them less.  A step with one and with two, us
+  // (skin 0.5, inner skin 0.1, TIP3P cubes): 2.7k atoms 45.6, 45.7; 9.8k 59.2,
+  // 58.7; 27k 103.1, 109.6; 55k 196.5, 201.4; 64k 233, 237; from 2^16 slots the
+  // rebuild outweighs it (100k 400, 392).  An evaluation at new positions
+  // always rebuilds and would take two: 340, 317; 600, 559; 993, 901; 1161,
+  // 1042 for 9.8k, 27k, 55k and 64k (rebuild alone 108, 90; 186, 144; 325, 238;
+  // 410, 291).  Rebuilds before the phases
   // were joined and the rows searched once: 2,652 atoms (defaults) 111 -> 72
   // us, 12k 163 -> 146, 27k 305 -> 267, 100k 694 -> 414, the 64-system ensemble
   // (all systems, separate launches) 2.58 -> 1.73 ms.

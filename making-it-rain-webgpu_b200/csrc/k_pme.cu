@@ -38,8 +38,9 @@ namespace {
 constexpr int kThreads = 256;
 
 // ------------------------------------------------------------ transforms --
-// Discrete transforms of R values in registers, R = 2 .. 10, so that a mesh
-// axis of up to 100 points takes two passes through shared memory.  SIGN is
+// Discrete transforms of R values in registers, R = 2 .. 10, so that most mesh
+// axes of up to 100 points take two passes through shared memory (75, 84, 96
+// and 98 take three).  SIGN is
 // the exponent's (-1 forward, +1 inverse).  Products that feed a sum are
 // written as fused steps, so every kernel that runs a line gives the same bits.
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
@@ -605,7 +606,7 @@ __device__ __forceinline__ void store_potential(float* out, int lines, int Kz, i
 // direction is two launches (with the x pass) and each has a plane of work.
 // What bounds them is the chain of one CTA (a load, four stages, four
 // barriers, a store), not bandwidth: 50^3 moves 2 MB.  Two real lines to a
-// complex one halve the z stages; radices up to 10 make an axis two stages;
+// complex one halve the z stages; radices up to 10 make most axes two stages;
 // the y transform's first stage separates the pairs as it loads and its last
 // stores to global memory, so nothing is copied between.  Measured with the x
 // pass against radices up to 5, lines one at a time and copies between the
@@ -1202,8 +1203,9 @@ __global__ void __launch_bounds__(kThreads) k_na_setup(SysDev S, NaPtrs p) {
       mod[m] = float(re * re + im * im);
     }
     __syncthreads();
-    // bspline.ts:126 -- replace a vanishing modulus by its neighbours' mean,
-    // from the first point up (a replaced neighbour counts as replaced)
+    // bspline.ts:126 -- replace a vanishing modulus by its neighbours' mean.
+    // Of an order-5 spline's only the one at n/2 of an even axis vanishes, so
+    // no neighbour is itself one to be replaced.
     for (int m = threadIdx.x; m < n; m += blockDim.x) {
       float* out = p.moduli + axis * kNoAllocMaxAxis;
       const float before = mod[(m - 1 + n) % n], after = mod[(m + 1) % n];
